@@ -1,4 +1,4 @@
-// dist.cu - distance (non-equi) nested-loop join over all |R| x |S| point pairs.
+// dist.cu - distance (non-equi) join: all pairs of R and S points within a radius.
 //
 // Reference: the 2-D GPU join joins/blockJoin_gpu/complex_block/dire_join
 // (eval, count and join kernels, join_gpu.cu:12-130; VAL_NUM 2, tuple.h:18-30)
@@ -9,39 +9,43 @@
 //   temp = 0; for each dimension i: t = r.val[i] - l.val[i]; temp += t * t;
 //   temp < radius * radius                   (radius = DISTANCE = 1 there).
 //
-// Screen.  Every point p carries x = p.val[0] rounded to nearest float
-// (+-inf beyond float range, NaN for NaN).  A CTA compares its R points with
-// one tile of S points at a time and rejects a pair when
-//   |round(x_s - x_r)| > W,   W = (|radius| + 2^-24 (M_S + M_R) + 2^-148)(1 + 2^-23),
-// everything rounded up, with M_S and M_R the largest |x| of the S tile and
-// of the CTA's R points.  Rounding a double to float moves it by at most
-// 2^-24 |x| + 2^-149 and the float subtraction by a factor 1 + 2^-24, so a
-// rejected pair has |r.val[0] - l.val[0]| >= |radius| in exact arithmetic;
-// its rounded difference and square are then at least |radius| and radius^2
-// (rounding is monotone), the other dimensions' squares only add, and the
-// pair cannot match.  A NaN difference is rejected too: its double difference
-// is NaN (or inf - inf) and never matches.  Points beyond float range make
-// M infinite and W infinite (their x is clamped to +-FLT_MAX in the loop), a
-// NaN radius makes W NaN and rejects everything, as radius^2 = NaN matches
-// nothing.  Pairs that pass get the exact predicate (__dsub_rn, __dmul_rn,
-// __dadd_rn in the reference's order: no fused multiply-add), so the matches
-// are the reference's, bit for bit.
+// Grid.  A match has |r.val[i] - l.val[i]| < rho = |radius| in exact arithmetic
+// in every dimension: rounding is monotone, so a difference of rho or more
+// rounds to rho or more, its square to radius^2 or more, and the other squares
+// only add.  So R is grouped by cells of width 2 rho (hashed over all
+// dimensions into 2 to 4 buckets per point) and an S point looks only at the
+// cells that hold [l - rho, l + rho], two per dimension on average: a few
+// lookups and a few candidates per S point instead of |R| compares.  The cell
+// number is a monotone function of the coordinate (dist_cell), so the cells
+// from that of l - rho (rounded down) to that of l + rho (rounded up) hold
+// every match whatever the rounding; a width fixed by the radius keeps the
+// cells small when a few points lie far out.  Points with a NaN or an infinite
+// coordinate match nothing (NaN and inf - inf differences are NaN, the others
+// infinite, and neither is below any radius^2) and are left out; radius^2 of
+// zero or NaN matches nothing at all.
 //
-// Layout: each CTA holds x of 16384 R points in registers (64 per thread,
-// packed in pairs; 160 registers, one CTA per SM, which the pure arithmetic
-// loop needs no more than); the x of S stream through shared memory in
-// 4096-point tiles.  Per S point a
-// thread takes the smallest (x_s - x_r)^2 over its 16 R points with packed
-// two-lane subtractions and products and three-input minima (three
-// instructions per two pairs) and compares it with W^2 once; only then are
-// the slots tested one by one.  Matches take an output slot from an atomic cursor (the row order is
-// not deterministic, the row multiset is); count-only mode sums per-thread
-// counters.
+// Candidates.  The grouped R keeps one 16-byte entry per point, its
+// coordinates rounded to float and its row.  A candidate is dropped when its
+// float distance is past a bound that no match reaches (dist_screen_bound);
+// the others get the reference's predicate on the doubles (__dsub_rn,
+// __dmul_rn, __dadd_rn in its order: no fused multiply-add), so the matches
+// are the reference's, bit for bit.  FP64 runs at 1/64 of the FP32 rate here,
+// so the screen is what keeps a dense grid off the FP64 pipe.  Two cells may
+// share a bucket: a matching candidate counts only when the cell being looked
+// at is its own, so no pair comes twice.
+//
+// Launches: cells (histogram with the points' ranks in their buckets), scan,
+// placement, probe.  A probe warp takes 32 S points, walks their cells
+// together and collects the matching pairs in shared memory; full buffers
+// become rows with one atomic add on the cursor and coalesced 8-byte stores
+// (the row order is not deterministic, the row multiset is).  Count-only mode
+// sums per-thread counters.  Both calls of a join (count, then rows), by all
+// pairs and here: 2^19 x 2^19 2-D points far apart 37.7 -> 0.356 ms; 100 003 x
+// 150 001 points of a 3-D box with about three matches each 77.7 -> 1.04 ms.
 #include <float.h>
 #include <math.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "ej_device.cuh"
 #include "ej_entry.h"
@@ -49,9 +53,12 @@
 namespace {
 
 constexpr int DJ_THREADS = 256;
-constexpr int DJ_RK = 64;                      // R points per thread
-constexpr int DJ_RCHUNK = DJ_THREADS * DJ_RK;  // R points per CTA
-constexpr int DJ_STILE = 4096;                 // S screen values per shared-memory tile (16 KB)
+constexpr int DJ_WARPS = DJ_THREADS / 32;
+constexpr int DJ_BUF = 160;  // pairs a warp collects before it writes rows (room for 32 more at 128)
+// points per launch sequence: 32-bit rows in the grid's entries, and a grid of
+// at most 2 GB of scratch; larger relations go in pieces
+constexpr uint64_t DJ_RPIECE = 1ull << 26;
+constexpr uint64_t DJ_SPIECE = 1ull << 31;
 
 template <int D>
 struct Point {
@@ -60,54 +67,47 @@ struct Point {
 };
 static_assert(sizeof(Point<2>) == sizeof(ej_point2) && sizeof(Point<3>) == sizeof(ej_point3), "point layouts");
 
-// dimension 0 of every point rounded to nearest float
+// the radius as the kernels use it
+struct DistRadius {
+  double rho;    // |radius|
+  double inv_w;  // 1 / (2 rho): cells of width 2 rho; 0 (one cell) when that is infinite
+  double r2;     // radius^2, rounded as the reference's
+  float rho_up;  // rho rounded up to float
+};
+
 template <int D>
-__global__ void dist_screen_kernel(const Point<D>* __restrict__ P, uint64_t n, float* __restrict__ x) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    x[i] = __double2float_rn(P[i].val[0]);
-}
-
-// the loop's operand: +-inf clamped to +-FLT_MAX (their tiles have W = inf), NaN kept
-__device__ __forceinline__ float dist_clamp(float x) {
-  return fabsf(x) == INFINITY ? copysignf(FLT_MAX, x) : x;
-}
-
-// the screening bound W of the header comment, rounded up
-__device__ __forceinline__ float dist_bound(float rad_up, float m_s, float m_r) {
-  const float err = __fmul_ru(0x1p-24f, __fadd_ru(m_s, m_r));
-  return __fmul_ru(__fadd_ru(__fadd_ru(rad_up, err), 0x1p-148f), 1.0f + 0x1p-23f);
-}
-
-// two float differences in one instruction (Blackwell packed f32x2):
-// (x - lo(r), x - hi(r)) for x2 = (x, x), each rounded to nearest like __fsub_rn
-__device__ __forceinline__ unsigned long long dist_sub2(unsigned long long x2, unsigned long long r) {
-  unsigned long long d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x2), "l"(r));
-  return d;
-}
-
-// minimum of three floats in one instruction; NaN operands are ignored
-__device__ __forceinline__ float dist_min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-
-__device__ __forceinline__ unsigned long long dist_pack(float lo, float hi) {
-  return (unsigned long long)__float_as_uint(hi) << 32 | __float_as_uint(lo);
-}
-
-// block-wide maximum (NaN inputs ignored); every thread gets it
-__device__ __forceinline__ float dist_block_max(float v, float* red) {
+__device__ __forceinline__ bool dist_finite(const Point<D>& p) {
+  bool ok = true;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float m = red[0];
+  for (int i = 0; i < D; i++) ok = ok && isfinite(p.val[i]);
+  return ok;
+}
+
+// The cell number of a finite coordinate: floor(x inv_w) up to 2^50 cells from
+// the origin; past that, where neighbouring doubles are rho / 4 or more
+// apart, every representable x inv_w is a cell of its own, numbered on by its
+// bit pattern.  Monotone in x throughout (the product is rounded monotonely),
+// and [l - rho, l + rho] spans at most 3 cells in the first range, 12 in the
+// second.
+__device__ __forceinline__ long long dist_cell(double x, double inv_w) {
+  const double t = inv_w == 0.0 ? 0.0 : __dmul_rn(x, inv_w);
+  if (fabs(t) < 0x1p50) return __double2ll_rd(t);
+  const long long c = (1ll << 50) + (__double_as_longlong(fabs(t)) - __double_as_longlong(0x1p50));
+  return t < 0.0 ? -c : c;
+}
+
+// the bucket of a cell: top `bits` bits of a multiplicative hash of its numbers
+template <int D>
+__device__ __forceinline__ uint32_t dist_bucket(const long long (&c)[D], uint32_t bits) {
+  unsigned long long x = (unsigned long long)c[0] * 0x9E3779B97F4A7C15ull;
 #pragma unroll
-  for (int w = 1; w < DJ_THREADS / 32; w++) m = fmaxf(m, red[w]);
-  __syncthreads();
-  return m;
+  for (int i = 1; i < D; i++) {
+    x ^= x >> 32;
+    x = (x + (unsigned long long)c[i]) * 0xD1342543DE82EF95ull;
+  }
+  x ^= x >> 32;
+  x *= 0x9E3779B97F4A7C15ull;
+  return (uint32_t)(x >> (64u - bits));
 }
 
 // the reference's predicate, operation by operation
@@ -122,27 +122,20 @@ __device__ __forceinline__ bool dist_match(const Point<D>& r, const Point<D>& l,
   return temp < r2;
 }
 
-// result rows as the reference lays them out, written as whole 8-byte words
-// (padding zero): dims 2 {lid, lval[2], rid, rval[2]}, dims 3 {lval[3], rval[3], lid, rid}
-__device__ __forceinline__ void dist_store(ej_point_result2* out, uint64_t pos, const Point<2>& l,
-                                           const Point<2>& r) {
-  unsigned long long* w = reinterpret_cast<unsigned long long*>(out + pos);
-  w[0] = (uint32_t)l.id;
-  w[1] = __double_as_longlong(l.val[0]);
-  w[2] = __double_as_longlong(l.val[1]);
-  w[3] = (uint32_t)r.id;
-  w[4] = __double_as_longlong(r.val[0]);
-  w[5] = __double_as_longlong(r.val[1]);
-}
-__device__ __forceinline__ void dist_store(ej_point_result3* out, uint64_t pos, const Point<3>& l,
-                                           const Point<3>& r) {
-  unsigned long long* w = reinterpret_cast<unsigned long long*>(out + pos);
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    w[i] = __double_as_longlong(l.val[i]);
-    w[3 + i] = __double_as_longlong(r.val[i]);
-  }
-  w[6] = (unsigned long long)(uint32_t)l.id | (unsigned long long)(uint32_t)r.id << 32;
+// Bound of the float screen: a pair whose float squared distance is above it
+// is no match.  For a match, with l at most m away from the origin in every
+// dimension and rho the radius, r in a looked-at cell is at most m + 4 rho away;
+// rounding both to float moves each difference by at most
+// e = 2^-24 (2 m + 4 rho) (and 2^-149 twice below the normal range), so the
+// float distance is at most (rho + sqrt(3) e) times 1 + 2^-18, which also
+// covers the rounding of the float operations, the squares' underflow
+// (2^-140) and the predicate's own rounding.  Past 10^18 the squares could
+// overflow: no screen (infinity; NaN distances pass it too).
+__device__ __forceinline__ float dist_screen_bound(float rho_up, float m) {
+  if (!(m < 1e18f) || !(rho_up < 1e18f)) return INFINITY;
+  const float e = __fadd_ru(__fmul_ru(0x1p-24f, __fadd_ru(__fmul_ru(2.0f, m), __fmul_ru(4.0f, rho_up))), 0x1p-140f);
+  const float b = __fmul_ru(__fadd_ru(rho_up, __fmul_ru(1.7320509f, e)), 1.0f + 0x1p-18f);
+  return __fadd_ru(__fmul_ru(__fmul_ru(b, b), 1.0f + 0x1p-18f), 0x1p-140f);
 }
 
 template <int D>
@@ -156,83 +149,160 @@ struct RowOf<3> {
   using type = ej_point_result3;
 };
 
+// A warp's lanes whose bucket is the same take consecutive ranks with one
+// atomic: a bucket that holds most of R costs 1/32 of the atomics.
+template <int D>
+__global__ void __launch_bounds__(256)
+dist_cell_kernel(const Point<D>* __restrict__ R, uint32_t nR, DistRadius rad, uint32_t bits,
+                 uint32_t* __restrict__ count, uint2* __restrict__ place) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; w < nR;
+       w += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = w + lane;
+    uint32_t b = 0xFFFFFFFFu;  // past nR, or a point that matches nothing
+    if (i < nR) {
+      const Point<D> p = R[i];
+      if (dist_finite<D>(p)) {
+        long long c[D];
+#pragma unroll
+        for (int d = 0; d < D; d++) c[d] = dist_cell(p.val[d], rad.inv_w);
+        b = dist_bucket<D>(c, bits);
+      }
+    }
+    const unsigned peers = __match_any_sync(EJ_FULL_MASK, b);
+    const int leader = __ffs(peers) - 1;
+    uint32_t first = 0;
+    if ((int)lane == leader && b != 0xFFFFFFFFu) first = atomicAdd(count + b, (uint32_t)__popc(peers));
+    first = __shfl_sync(EJ_FULL_MASK, first, leader);
+    if (i < nR) place[i] = make_uint2(b, first + __popc(peers & ej_lanemask_lt()));
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256)
+dist_place_kernel(const Point<D>* __restrict__ R, uint32_t nR, const uint2* __restrict__ place,
+                  const uint32_t* __restrict__ start, float4* __restrict__ grid) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint2 pl = place[i];
+    if (pl.x == 0xFFFFFFFFu) continue;
+    const Point<D> p = R[i];
+    float4 e;
+    e.x = __double2float_rn(p.val[0]);
+    e.y = __double2float_rn(p.val[1]);
+    e.z = D == 3 ? __double2float_rn(p.val[D - 1]) : 0.0f;
+    e.w = __uint_as_float((uint32_t)i);
+    grid[start[pl.x] + pl.y] = e;
+  }
+}
+
+// the first n pairs {S row, R row} of a warp's buffer as result rows, laid out
+// as the reference's (padding zero): dims 2 {lid, lval[2], rid, rval[2]},
+// dims 3 {lval[3], rval[3], lid, rid}; consecutive lanes write consecutive
+// 8-byte words
+template <int D>
+__device__ __forceinline__ void dist_flush(const uint2* buf, uint32_t n, const Point<D>* __restrict__ R,
+                                           const Point<D>* __restrict__ S, typename RowOf<D>::type* __restrict__ out,
+                                           uint64_t cap, unsigned long long* cursor) {
+  constexpr uint32_t WORDS = sizeof(typename RowOf<D>::type) / 8;
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();
+  unsigned long long off = 0;
+  if (lane == 0) off = atomicAdd(cursor, (unsigned long long)n);
+  off = __shfl_sync(EJ_FULL_MASK, off, 0);
+  for (uint32_t k = lane; k < n * WORDS; k += 32) {
+    const uint32_t row = k / WORDS, word = k - row * WORDS;
+    if (off + row >= cap) break;
+    const uint2 pr = buf[row];
+    const Point<D>& l = S[pr.x];
+    const Point<D>& r = R[pr.y];
+    unsigned long long v;
+    if (D == 2) {
+      const Point<D>& p = word < 3 ? l : r;
+      const uint32_t q = word < 3 ? word : word - 3;
+      v = q == 0 ? (unsigned long long)(uint32_t)p.id : (unsigned long long)__double_as_longlong(p.val[q - 1]);
+    } else {
+      v = word == 6 ? (unsigned long long)(uint32_t)l.id | (unsigned long long)(uint32_t)r.id << 32
+                    : (unsigned long long)__double_as_longlong(word < 3 ? l.val[word] : r.val[word - 3]);
+    }
+    reinterpret_cast<unsigned long long*>(out + off)[k] = v;
+  }
+  __syncwarp();
+}
+
 template <int D, bool COUNT_ONLY>
 __global__ void __launch_bounds__(DJ_THREADS)
-dist_kernel(const Point<D>* __restrict__ R, const float* __restrict__ rx_all, uint64_t nR,
-            const Point<D>* __restrict__ S, const float* __restrict__ sx_all, uint64_t nS, uint64_t s_per_cta,
-            float rad_up, double r2, typename RowOf<D>::type* __restrict__ out, uint64_t cap,
-            unsigned long long* cursor) {
-  __shared__ float tile[DJ_STILE];
-  __shared__ float red[DJ_THREADS / 32];
-  __shared__ unsigned long long warp_tmp[DJ_THREADS / 32 + 1];
-  const uint64_t rbase = (uint64_t)blockIdx.x * DJ_RCHUNK;
-  // the thread's R screen values in pairs, for the packed subtraction
-  unsigned long long rx2[DJ_RK / 2];
-  using Mask = typename std::conditional<(DJ_RK > 32), unsigned long long, uint32_t>::type;
-  Mask valid = 0;
-  float m = 0.0f;
-#pragma unroll
-  for (int k = 0; k < DJ_RK; k += 2) {
-    float x[2];
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const uint64_t ri = rbase + (uint64_t)(k + e) * DJ_THREADS + threadIdx.x;
-      x[e] = __int_as_float(0x7fc00000);  // slots past nR: NaN, never a candidate
-      if (ri < nR) {
-        x[e] = __ldg(rx_all + ri);
-        valid |= (Mask)1 << (k + e);
-      }
-      m = fmaxf(m, fabsf(x[e]));
-    }
-    rx2[k / 2] = dist_pack(dist_clamp(x[0]), dist_clamp(x[1]));
-  }
-  const float m_r = dist_block_max(m, red);
-  const uint64_t s_begin = (uint64_t)blockIdx.y * s_per_cta;
-  const uint64_t s_end = min(nS, s_begin + s_per_cta);
+dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S, uint32_t nS,
+                  const uint32_t* __restrict__ start, const float4* __restrict__ grid, uint32_t bits, DistRadius rad,
+                  typename RowOf<D>::type* __restrict__ out, uint64_t cap, unsigned long long* cursor) {
+  __shared__ uint2 bufs[DJ_WARPS][DJ_BUF];
+  __shared__ unsigned long long warp_tmp[DJ_WARPS + 1];
+  const uint32_t lane = threadIdx.x & 31u;
+  uint2* buf = bufs[threadIdx.x >> 5];
+  uint32_t held = 0;  // pairs in the warp's buffer
   unsigned long long local = 0;
-  for (uint64_t t0 = s_begin; t0 < s_end; t0 += DJ_STILE) {
-    const uint32_t n = (uint32_t)min((uint64_t)DJ_STILE, s_end - t0);
-    __syncthreads();  // the previous tile is no longer read
-    float ms = 0.0f;
-    for (uint32_t k = threadIdx.x; k < n; k += DJ_THREADS) {
-      const float x = __ldcs(sx_all + t0 + k);
-      ms = fmaxf(ms, fabsf(x));
-      tile[k] = dist_clamp(x);
+  for (uint64_t w = ((uint64_t)blockIdx.x * DJ_THREADS + threadIdx.x) & ~31ull; w < nS;
+       w += (uint64_t)gridDim.x * DJ_THREADS) {
+    const uint64_t si = w + lane;
+    Point<D> l;
+    bool ok = si < nS;
+    if (ok) {
+      l = S[si];
+      ok = dist_finite<D>(l);
     }
-    const float W = dist_bound(rad_up, dist_block_max(ms, red), m_r);  // its barriers publish the tile
-    if (!valid) continue;
-    for (uint32_t k = 0; k < n; k++) {
-      const float xs = tile[k];
-      // the smallest |xs - x_r| over the thread's R points (NaN differences
-      // ignored): two differences per instruction, two minima per instruction
-      const unsigned long long xs2 = dist_pack(xs, xs);
-      float dmin = INFINITY;
+    // the cells that hold [l - rho, l + rho], dimension by dimension
+    long long lo[D], cur[D];
+    int span[D], cells = ok ? 1 : 0;
+    float x[3] = {0.0f, 0.0f, 0.0f}, m = 0.0f;
 #pragma unroll
-      for (int j = 0; j < DJ_RK / 2; j++) {
-        const unsigned long long d = dist_sub2(xs2, rx2[j]);
-        dmin = dist_min3(dmin, fabsf(__uint_as_float((uint32_t)d)), fabsf(__uint_as_float((uint32_t)(d >> 32))));
+    for (int d = 0; d < D; d++) {
+      const double v = ok ? l.val[d] : 0.0;
+      lo[d] = cur[d] = dist_cell(fmax(__dsub_rd(v, rad.rho), -DBL_MAX), rad.inv_w);
+      span[d] = (int)(dist_cell(fmin(__dadd_ru(v, rad.rho), DBL_MAX), rad.inv_w) - lo[d]) + 1;
+      cells *= span[d];
+      x[d] = __double2float_rn(v);
+      m = fmaxf(m, __double2float_ru(fabs(v)));
+    }
+    const float bound = dist_screen_bound(rad.rho_up, m);
+    for (int k = 0; __any_sync(EJ_FULL_MASK, k < cells); k++) {
+      uint32_t p = 0, end = 0;
+      if (k < cells) {
+        const uint32_t b = dist_bucket<D>(cur, bits);
+        p = __ldg(start + b);
+        end = __ldg(start + b + 1);
       }
-      if (!(dmin <= W)) continue;
-      // the rare path: candidate slots as a bit mask (static indices keep rx2 in registers)
-      Mask mask = 0;
+      while (__any_sync(EJ_FULL_MASK, p < end)) {
+        bool hit = false;
+        uint32_t ri = 0;
+        if (p < end) {
+          const float4 e = __ldg(grid + p);
+          const float dx = e.x - x[0], dy = e.y - x[1], dz = e.z - x[2];
+          p++;
+          if (!(fmaf(dx, dx, fmaf(dy, dy, D == 3 ? dz * dz : 0.0f)) > bound)) {
+            ri = __float_as_uint(e.w);
+            const Point<D> r = R[ri];
+            hit = dist_match<D>(r, l, rad.r2);
 #pragma unroll
-      for (int j = 0; j < DJ_RK / 2; j++) {
-        const unsigned long long d = dist_sub2(xs2, rx2[j]);
-        mask |= (Mask)(fabsf(__uint_as_float((uint32_t)d)) <= W) << (2 * j);
-        mask |= (Mask)(fabsf(__uint_as_float((uint32_t)(d >> 32))) <= W) << (2 * j + 1);
-      }
-      mask &= valid;
-      const Point<D> l = S[t0 + k];
-      for (; mask; mask &= mask - 1) {
-        const int j = DJ_RK > 32 ? __ffsll((long long)mask) - 1 : __ffs((int)mask) - 1;
-        const Point<D> r = R[rbase + (uint64_t)j * DJ_THREADS + threadIdx.x];
-        if (!dist_match<D>(r, l, r2)) continue;
+            for (int d = 0; d < D; d++) hit = hit && dist_cell(r.val[d], rad.inv_w) == cur[d];
+          }
+        }
         if (COUNT_ONLY) {
-          local++;
+          local += hit ? 1u : 0u;
           continue;
         }
-        const unsigned long long pos = atomicAdd(cursor, 1ull);
-        if (pos < cap) dist_store(out, pos, l, r);
+        const unsigned hits = __ballot_sync(EJ_FULL_MASK, hit);
+        if (hits == 0) continue;
+        if (hit) buf[held + __popc(hits & ej_lanemask_lt())] = make_uint2((uint32_t)si, ri);
+        held += __popc(hits);
+        if (held > DJ_BUF - 32) {
+          dist_flush<D>(buf, held, R, S, out, cap, cursor);
+          held = 0;
+        }
+      }
+      // the next cell, dimension 0 fastest
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        if (++cur[d] < lo[d] + span[d]) break;
+        cur[d] = lo[d];
       }
     }
   }
@@ -240,18 +310,28 @@ dist_kernel(const Point<D>* __restrict__ R, const float* __restrict__ rx_all, ui
     unsigned long long total;
     ej_block_exclusive_sum<DJ_THREADS, unsigned long long>(local, warp_tmp, &total);
     if (threadIdx.x == 0 && total) atomicAdd(cursor, total);
+  } else if (held) {
+    dist_flush<D>(buf, held, R, S, out, cap, cursor);
   }
 }
 
-// |radius| rounded up to float (infinite beyond float range, NaN for NaN)
-float dist_radius_up(double radius) {
-  const double a = fabs(radius);
-  if (a != a) return NAN;
-  if (a > (double)FLT_MAX) return INFINITY;
-  float f = (float)a;
-  if ((double)f < a) f = nextafterf(f, INFINITY);
-  return f;
+DistRadius dist_radius(double radius) {
+  DistRadius r;
+  r.rho = fabs(radius);
+  const double w = 2.0 * r.rho;
+  r.inv_w = w > 0.0 && w <= DBL_MAX ? 1.0 / w : 0.0;
+  r.r2 = radius * radius;
+  if (r.rho > (double)FLT_MAX) {
+    r.rho_up = INFINITY;
+  } else {
+    r.rho_up = (float)r.rho;
+    if ((double)r.rho_up < r.rho) r.rho_up = nextafterf(r.rho_up, INFINITY);
+  }
+  return r;
 }
+
+// buckets of a grid of n points: 2^bits, two to four per point
+uint32_t dist_bits(uint64_t n) { return std::max(8u, ej_ceil_log2(n) + 1u); }
 
 template <int D>
 ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, uint64_t nS, double radius, void* outv,
@@ -259,40 +339,47 @@ ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, ui
   const Point<D>* R = static_cast<const Point<D>*>(Rv);
   const Point<D>* S = static_cast<const Point<D>*>(Sv);
   EJ_CUDA(h, cudaMemsetAsync(h->d_words, 0, sizeof(unsigned long long), h->stream));
-  if (nR == 0 || nS == 0) return EJ_OK;
-  const uint64_t rchunks = (nR + DJ_RCHUNK - 1) / DJ_RCHUNK;
-  if (rchunks > 0x7FFFFFFFull) return ej_fail(h, EJ_ERR_TOO_LARGE, "R too large for the nested loop");
+  const DistRadius rad = dist_radius(radius);
+  if (nR == 0 || nS == 0 || !(rad.r2 > 0.0)) return EJ_OK;
+  const uint64_t piece = std::min(nR, DJ_RPIECE);
+  const uint64_t nb = 1ull << dist_bits(piece);
   ej_plan_bytes p;
-  const size_t roff = p.add(nR * sizeof(float)), soff = p.add(nS * sizeof(float));
+  const size_t coff = p.add(nb * sizeof(uint32_t)), soff = p.add((nb + 1) * sizeof(uint32_t)),
+               scan_off = p.add(ej_scan_scratch_bytes(nb)), poff = p.add(piece * sizeof(uint2)),
+               goff = p.add(piece * sizeof(float4));
   EJ_TRY(ej_arena_reserve(h, p.bytes));
-  float* rx = reinterpret_cast<float*>(ej_arena_at(h, roff));
-  float* sx = reinterpret_cast<float*>(ej_arena_at(h, soff));
-  ej_phase_begin(h);
-  const unsigned blocks = (unsigned)std::min<uint64_t>((std::max(nR, nS) + 255) / 256, (uint64_t)h->num_sms * 8);
-  dist_screen_kernel<D><<<blocks, 256, 0, h->stream>>>(R, nR, rx);
-  EJ_TRY(ej_check_launch(h, "dist_screen_kernel"));
-  dist_screen_kernel<D><<<blocks, 256, 0, h->stream>>>(S, nS, sx);
-  EJ_TRY(ej_check_launch(h, "dist_screen_kernel"));
-  // the screen values are the build phase; the nested loop is recorded as the write phase
-  for (int k = 1; k < EJ_PHASES; k++) ej_phase_mark(h, k);
-  // about four CTAs per SM; each CTA's S range a whole number of tiles
-  const uint64_t want = (uint64_t)h->num_sms * 4;
-  const uint64_t stiles = (nS + DJ_STILE - 1) / DJ_STILE;
-  uint64_t splits = (want + rchunks - 1) / rchunks;
-  splits = std::max<uint64_t>(1, std::min<uint64_t>(std::min<uint64_t>(splits, stiles), 65535));
-  const uint64_t s_per_cta = ((stiles + splits - 1) / splits) * DJ_STILE;
-  splits = (nS + s_per_cta - 1) / s_per_cta;
-  const dim3 grid((unsigned)rchunks, (unsigned)splits);
-  const float rad_up = dist_radius_up(radius);
-  const double r2 = radius * radius;
+  uint32_t* count = reinterpret_cast<uint32_t*>(ej_arena_at(h, coff));
+  uint32_t* start = reinterpret_cast<uint32_t*>(ej_arena_at(h, soff));
+  uint2* place = reinterpret_cast<uint2*>(ej_arena_at(h, poff));
+  float4* grid = reinterpret_cast<float4*>(ej_arena_at(h, goff));
   using Row = typename RowOf<D>::type;
-  if (count_only)
-    dist_kernel<D, true><<<grid, DJ_THREADS, 0, h->stream>>>(R, rx, nR, S, sx, nS, s_per_cta, rad_up, r2, nullptr,
-                                                             0, h->d_words);
-  else
-    dist_kernel<D, false><<<grid, DJ_THREADS, 0, h->stream>>>(R, rx, nR, S, sx, nS, s_per_cta, rad_up, r2,
-                                                              static_cast<Row*>(outv), cap, h->d_words);
-  EJ_TRY(ej_check_launch(h, "dist_kernel"));
+  // the first piece's grid is the build phase; the probe (and any further pieces) the write phase
+  ej_phase_begin(h);
+  for (uint64_t r0 = 0; r0 < nR; r0 += DJ_RPIECE) {
+    const uint32_t n = (uint32_t)std::min<uint64_t>(DJ_RPIECE, nR - r0);
+    const uint32_t bits = dist_bits(n);
+    const unsigned rblocks = (unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, (uint64_t)h->num_sms * 8);
+    EJ_CUDA(h, cudaMemsetAsync(count, 0, sizeof(uint32_t) << bits, h->stream));
+    dist_cell_kernel<D><<<rblocks, 256, 0, h->stream>>>(R + r0, n, rad, bits, count, place);
+    EJ_TRY(ej_check_launch(h, "dist_cell_kernel"));
+    EJ_TRY(ej_scan_u32_u32(h, count, 1ull << bits, start, ej_arena_at(h, scan_off)));
+    dist_place_kernel<D><<<rblocks, 256, 0, h->stream>>>(R + r0, n, place, start, grid);
+    EJ_TRY(ej_check_launch(h, "dist_place_kernel"));
+    if (r0 == 0)
+      for (int k = 1; k < EJ_PHASES; k++) ej_phase_mark(h, k);
+    for (uint64_t s0 = 0; s0 < nS; s0 += DJ_SPIECE) {
+      const uint32_t ns = (uint32_t)std::min<uint64_t>(DJ_SPIECE, nS - s0);
+      const unsigned sblocks =
+          (unsigned)std::min<uint64_t>(((uint64_t)ns + DJ_THREADS - 1) / DJ_THREADS, (uint64_t)h->num_sms * 8);
+      if (count_only)
+        dist_probe_kernel<D, true><<<sblocks, DJ_THREADS, 0, h->stream>>>(R + r0, S + s0, ns, start, grid, bits, rad,
+                                                                          nullptr, 0, h->d_words);
+      else
+        dist_probe_kernel<D, false><<<sblocks, DJ_THREADS, 0, h->stream>>>(R + r0, S + s0, ns, start, grid, bits, rad,
+                                                                           static_cast<Row*>(outv), cap, h->d_words);
+      EJ_TRY(ej_check_launch(h, "dist_probe_kernel"));
+    }
+  }
   ej_phase_mark(h, EJ_PHASES);
   return EJ_OK;
 }
