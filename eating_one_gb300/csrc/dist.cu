@@ -29,19 +29,27 @@
 // float distance is past a bound that no match reaches (dist_screen_bound);
 // the others get the reference's predicate on the doubles (__dsub_rn,
 // __dmul_rn, __dadd_rn in its order: no fused multiply-add), so the matches
-// are the reference's, bit for bit.  FP64 runs at 1/64 of the FP32 rate here,
-// so the screen is what keeps a dense grid off the FP64 pipe.  Two cells may
-// share a bucket: a matching candidate counts only when the cell being looked
-// at is its own, so no pair comes twice.
+// are the reference's, bit for bit.  FP64 runs at 1/64 of the FP32 rate here
+// (a warp instruction takes 16 cycles, however few lanes are active), so the
+// candidates that pass the screen are collected and tested by full warps: at
+// once, most steps of a probe warp would take the double path for one or two
+// lanes.  Two of an S point's cells may share a bucket, which is then looked
+// at once: every R point lies in one bucket, so no pair comes twice.
 //
 // Launches: cells (histogram with the points' ranks in their buckets), scan,
-// placement, probe.  A probe warp takes 32 S points, walks their cells
-// together and collects the matching pairs in shared memory; full buffers
-// become rows with one atomic add on the cursor and coalesced 8-byte stores
-// (the row order is not deterministic, the row multiset is).  Count-only mode
-// sums per-thread counters.  Both calls of a join (count, then rows), by all
-// pairs and here: 2^19 x 2^19 2-D points far apart 37.7 -> 0.356 ms; 100 003 x
-// 150 001 points of a 3-D box with about three matches each 77.7 -> 1.04 ms.
+// placement, probe.  A probe warp takes 32 S points: each lane finds its point's
+// cells, then groups of 4 (2-D) or 8 (3-D) lanes share a point, a lane per cell,
+// and walk the buckets together, two candidates a step; the pairs that pass
+// the screen collect in shared memory, and full buffers are tested and become
+// rows with one atomic add on the cursor and coalesced 8-byte stores (the row
+// order is not deterministic, the row multiset is).  Count-only mode sums
+// per-thread counters.
+// Both calls of a join (count, then rows): 2^19 x 2^19 2-D points far apart by
+// all pairs 37.7 ms, by the grid with a lane per S point and the predicate in
+// the step 0.356 ms, here 0.249 (the
+// probe 87 -> 49 us); 100 003 x 150 001 points of a 3-D box with
+// about three matches each 77.7, 1.04 and 0.242 ms (the probe
+// 430 -> 55 us).
 #include <float.h>
 #include <math.h>
 
@@ -54,7 +62,7 @@ namespace {
 
 constexpr int DJ_THREADS = 256;
 constexpr int DJ_WARPS = DJ_THREADS / 32;
-constexpr int DJ_BUF = 160;  // pairs a warp collects before it writes rows (room for 32 more at 128)
+constexpr int DJ_BUF = 192;  // candidate pairs a warp collects (tested past 128; a step adds at most 64)
 // points per launch sequence: 32-bit rows in the grid's entries, and a grid of
 // at most 2 GB of scratch; larger relations go in pieces
 constexpr uint64_t DJ_RPIECE = 1ull << 26;
@@ -79,7 +87,8 @@ template <int D>
 __device__ __forceinline__ bool dist_finite(const Point<D>& p) {
   bool ok = true;
 #pragma unroll
-  for (int i = 0; i < D; i++) ok = ok && isfinite(p.val[i]);
+  for (int i = 0; i < D; i++)
+    ok = ok && ((unsigned long long)__double_as_longlong(p.val[i]) & 0x7FF0000000000000ull) != 0x7FF0000000000000ull;
   return ok;
 }
 
@@ -89,11 +98,20 @@ __device__ __forceinline__ bool dist_finite(const Point<D>& p) {
 // bit pattern.  Monotone in x throughout (the product is rounded monotonely),
 // and [l - rho, l + rho] spans at most 3 cells in the first range, 12 in the
 // second.
+// (The magnitude test is on the exponent bits, off the FP64 pipe.)
 __device__ __forceinline__ long long dist_cell(double x, double inv_w) {
-  const double t = inv_w == 0.0 ? 0.0 : __dmul_rn(x, inv_w);
-  if (fabs(t) < 0x1p50) return __double2ll_rd(t);
-  const long long c = (1ll << 50) + (__double_as_longlong(fabs(t)) - __double_as_longlong(0x1p50));
-  return t < 0.0 ? -c : c;
+  const double t = __dmul_rn(x, inv_w);  // x finite: inv_w = 0 gives 0
+  const unsigned long long mag = (unsigned long long)__double_as_longlong(t) & 0x7FFFFFFFFFFFFFFFull;
+  constexpr unsigned long long FAR = 0x4310000000000000ull;  // the bits of 2^50
+  if (mag < FAR) return __double2ll_rd(t);
+  const long long c = (long long)((1ull << 50) + (mag - FAR));
+  return __double_as_longlong(t) < 0 ? -c : c;
+}
+
+// a bound of [l - rho, l + rho] kept finite (R's points are)
+__device__ __forceinline__ double dist_clamp(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (b & 0x7FFFFFFFFFFFFFFFull) == 0x7FF0000000000000ull ? __longlong_as_double((long long)(b - 1)) : x;
 }
 
 // the bucket of a cell: top `bits` bits of a multiplicative hash of its numbers
@@ -195,21 +213,42 @@ dist_place_kernel(const Point<D>* __restrict__ R, uint32_t nR, const uint2* __re
   }
 }
 
-// the first n pairs {S row, R row} of a warp's buffer as result rows, laid out
-// as the reference's (padding zero): dims 2 {lid, lval[2], rid, rval[2]},
-// dims 3 {lval[3], rval[3], lid, rid}; consecutive lanes write consecutive
-// 8-byte words
-template <int D>
-__device__ __forceinline__ void dist_flush(const uint2* buf, uint32_t n, const Point<D>* __restrict__ R,
-                                           const Point<D>* __restrict__ S, typename RowOf<D>::type* __restrict__ out,
-                                           uint64_t cap, unsigned long long* cursor) {
+// Tests the n candidate pairs {S row, R row} of a warp's buffer and writes the
+// matches as result rows, laid out as the reference's (padding zero): dims 2
+// {lid, lval[2], rid, rval[2]}, dims 3 {lval[3], rval[3], lid, rid}; consecutive
+// lanes write consecutive 8-byte words.  Count-only: returns the lane's matches.
+template <int D, bool COUNT_ONLY>
+__device__ __forceinline__ uint32_t dist_flush(uint2* buf, uint32_t n, const Point<D>* __restrict__ R,
+                                               const Point<D>* __restrict__ S, double r2,
+                                               typename RowOf<D>::type* __restrict__ out, uint64_t cap,
+                                               unsigned long long* cursor) {
   constexpr uint32_t WORDS = sizeof(typename RowOf<D>::type) / 8;
   const uint32_t lane = threadIdx.x & 31u;
+  uint32_t rows = 0;
   __syncwarp();
+  for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+    uint2 pr = make_uint2(0u, 0u);
+    bool hit = false;
+    if (k0 + lane < n) {
+      pr = buf[k0 + lane];
+      hit = dist_match<D>(R[pr.y], S[pr.x], r2);
+    }
+    if (COUNT_ONLY) {
+      rows += hit ? 1u : 0u;
+      continue;
+    }
+    // the matches move to the front, behind those of the steps before (all
+    // lanes have read their pairs of this step)
+    const unsigned hits = __ballot_sync(EJ_FULL_MASK, hit);
+    if (hit) buf[rows + __popc(hits & ej_lanemask_lt())] = pr;
+    rows += __popc(hits);
+    __syncwarp();
+  }
+  if (COUNT_ONLY || rows == 0) return rows;
   unsigned long long off = 0;
-  if (lane == 0) off = atomicAdd(cursor, (unsigned long long)n);
+  if (lane == 0) off = atomicAdd(cursor, (unsigned long long)rows);
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
-  for (uint32_t k = lane; k < n * WORDS; k += 32) {
+  for (uint32_t k = lane; k < rows * WORDS; k += 32) {
     const uint32_t row = k / WORDS, word = k - row * WORDS;
     if (off + row >= cap) break;
     const uint2 pr = buf[row];
@@ -227,6 +266,7 @@ __device__ __forceinline__ void dist_flush(const uint2* buf, uint32_t n, const P
     reinterpret_cast<unsigned long long*>(out + off)[k] = v;
   }
   __syncwarp();
+  return rows;
 }
 
 template <int D, bool COUNT_ONLY>
@@ -234,84 +274,121 @@ __global__ void __launch_bounds__(DJ_THREADS)
 dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S, uint32_t nS,
                   const uint32_t* __restrict__ start, const float4* __restrict__ grid, uint32_t bits, DistRadius rad,
                   typename RowOf<D>::type* __restrict__ out, uint64_t cap, unsigned long long* cursor) {
+  constexpr int G = D == 2 ? 4 : 8;  // lanes of an S point: its cells, when no dimension has three
   __shared__ uint2 bufs[DJ_WARPS][DJ_BUF];
   __shared__ unsigned long long warp_tmp[DJ_WARPS + 1];
-  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lane = threadIdx.x & 31u, g = lane % G;
+  const unsigned group = (D == 2 ? 0xFu : 0xFFu) << (lane - g);  // the lanes of this lane's S point
   uint2* buf = bufs[threadIdx.x >> 5];
   uint32_t held = 0;  // pairs in the warp's buffer
   unsigned long long local = 0;
   for (uint64_t w = ((uint64_t)blockIdx.x * DJ_THREADS + threadIdx.x) & ~31ull; w < nS;
        w += (uint64_t)gridDim.x * DJ_THREADS) {
-    const uint64_t si = w + lane;
-    Point<D> l;
-    bool ok = si < nS;
-    if (ok) {
-      l = S[si];
-      ok = dist_finite<D>(l);
-    }
-    // the cells that hold [l - rho, l + rho], dimension by dimension
-    long long lo[D], cur[D];
-    int span[D], cells = ok ? 1 : 0;
-    float x[3] = {0.0f, 0.0f, 0.0f}, m = 0.0f;
-#pragma unroll
-    for (int d = 0; d < D; d++) {
-      const double v = ok ? l.val[d] : 0.0;
-      lo[d] = cur[d] = dist_cell(fmax(__dsub_rd(v, rad.rho), -DBL_MAX), rad.inv_w);
-      span[d] = (int)(dist_cell(fmin(__dadd_ru(v, rad.rho), DBL_MAX), rad.inv_w) - lo[d]) + 1;
-      cells *= span[d];
-      x[d] = __double2float_rn(v);
-      m = fmaxf(m, __double2float_ru(fabs(v)));
-    }
-    const float bound = dist_screen_bound(rad.rho_up, m);
-    for (int k = 0; __any_sync(EJ_FULL_MASK, k < cells); k++) {
-      uint32_t p = 0, end = 0;
-      if (k < cells) {
-        const uint32_t b = dist_bucket<D>(cur, bits);
-        p = __ldg(start + b);
-        end = __ldg(start + b + 1);
+    // the lane's own S point: the first of the cells that hold [l - rho, l +
+    // rho] and their number in every dimension (at most 12)
+    long long lo[D];
+    uint32_t spans = 0;  // 8 bits per dimension; 0: no point
+    float x[D], bound;
+    {
+      const uint64_t si = w + lane;
+      Point<D> l;
+      bool ok = si < nS;
+      if (ok) {
+        l = S[si];
+        ok = dist_finite<D>(l);
       }
-      while (__any_sync(EJ_FULL_MASK, p < end)) {
-        bool hit = false;
-        uint32_t ri = 0;
-        if (p < end) {
-          const float4 e = __ldg(grid + p);
-          const float dx = e.x - x[0], dy = e.y - x[1], dz = e.z - x[2];
-          p++;
-          if (!(fmaf(dx, dx, fmaf(dy, dy, D == 3 ? dz * dz : 0.0f)) > bound)) {
-            ri = __float_as_uint(e.w);
-            const Point<D> r = R[ri];
-            hit = dist_match<D>(r, l, rad.r2);
-#pragma unroll
-            for (int d = 0; d < D; d++) hit = hit && dist_cell(r.val[d], rad.inv_w) == cur[d];
-          }
-        }
-        if (COUNT_ONLY) {
-          local += hit ? 1u : 0u;
-          continue;
-        }
-        const unsigned hits = __ballot_sync(EJ_FULL_MASK, hit);
-        if (hits == 0) continue;
-        if (hit) buf[held + __popc(hits & ej_lanemask_lt())] = make_uint2((uint32_t)si, ri);
-        held += __popc(hits);
-        if (held > DJ_BUF - 32) {
-          dist_flush<D>(buf, held, R, S, out, cap, cursor);
-          held = 0;
-        }
-      }
-      // the next cell, dimension 0 fastest
+      float m = 0.0f;
 #pragma unroll
       for (int d = 0; d < D; d++) {
-        if (++cur[d] < lo[d] + span[d]) break;
-        cur[d] = lo[d];
+        const double v = ok ? l.val[d] : 0.0;
+        lo[d] = dist_cell(dist_clamp(__dsub_rd(v, rad.rho)), rad.inv_w);
+        const uint32_t span = (uint32_t)(dist_cell(dist_clamp(__dadd_ru(v, rad.rho)), rad.inv_w) - lo[d]) + 1u;
+        spans |= (ok ? span : 0u) << (8 * d);
+        x[d] = __double2float_rn(v);
+        m = fmaxf(m, __fmul_ru(fabsf(x[d]), 1.0f + 0x1p-23f));
+      }
+      bound = dist_screen_bound(rad.rho_up, m);
+    }
+    // 32 / G of the warp's S points at a time, G lanes each
+    for (int t = 0; t < G; t++) {
+      const int owner = t * (32 / G) + (int)(lane / G);
+      long long c0[D];
+      float xs[D];
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        c0[d] = __shfl_sync(EJ_FULL_MASK, lo[d], owner);
+        xs[d] = __shfl_sync(EJ_FULL_MASK, x[d], owner);
+      }
+      const uint32_t sp = __shfl_sync(EJ_FULL_MASK, spans, owner);
+      const float bd = __shfl_sync(EJ_FULL_MASK, bound, owner);
+      const uint32_t n0 = sp & 0xFFu, n1 = sp >> 8 & 0xFFu, n2 = D == 3 ? sp >> 16 : 1u;
+      const uint32_t cells = n0 * n1 * n2;
+      for (uint32_t first = 0; __any_sync(EJ_FULL_MASK, first < cells); first += G) {
+        const uint32_t k = first + g;
+        uint32_t p = 0, end = 0, b = 0xFFFFFFFFu;
+        if (k < cells) {
+          const uint32_t k1 = k / n0;
+          long long c[D];
+          c[0] = c0[0] + (k - k1 * n0);
+          const uint32_t k2 = k1 / n1;
+          c[1] = c0[1] + (k1 - k2 * n1);
+          if (D == 3) c[D - 1] = c0[D - 1] + k2;
+          b = dist_bucket<D>(c, bits);
+          // the point's earlier cells in this bucket: in this round of G
+          // cells (below), and in the rounds before, which only points whose
+          // reach spans three cells or more somewhere have
+          for (uint32_t e = 0; e < first; e++) {
+            const uint32_t e1 = e / n0, e2 = e1 / n1;
+            long long f[D];
+            f[0] = c0[0] + (e - e1 * n0);
+            f[1] = c0[1] + (e1 - e2 * n1);
+            if (D == 3) f[D - 1] = c0[D - 1] + e2;
+            if (dist_bucket<D>(f, bits) == b) b = 0xFFFFFFFFu;
+          }
+        }
+        const unsigned same = __match_any_sync(EJ_FULL_MASK, b) & group & ej_lanemask_lt();
+        if (b != 0xFFFFFFFFu && same == 0) {
+          p = __ldg(start + b);
+          end = __ldg(start + b + 1);
+        }
+        while (__any_sync(EJ_FULL_MASK, p < end)) {
+          bool pass[2];
+          uint32_t ri[2];
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            pass[u] = p + u < end;
+            ri[u] = 0;
+            if (pass[u]) {
+              const float4 e = __ldg(grid + p + u);
+              const float dx = e.x - xs[0], dy = e.y - xs[1], dz = D == 3 ? e.z - xs[D - 1] : 0.0f;
+              ri[u] = __float_as_uint(e.w);
+              pass[u] = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > bd);
+            }
+          }
+          p += 2;
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const unsigned some = __ballot_sync(EJ_FULL_MASK, pass[u]);
+            if (pass[u]) buf[held + __popc(some & ej_lanemask_lt())] = make_uint2((uint32_t)w + owner, ri[u]);
+            held += __popc(some);
+          }
+          if (held > DJ_BUF - 64) {
+            const uint32_t rows = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+            if (COUNT_ONLY) local += rows;
+            held = 0;
+          }
+        }
       }
     }
+  }
+  if (held) {
+    const uint32_t rows = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+    if (COUNT_ONLY) local += rows;
   }
   if (COUNT_ONLY) {
     unsigned long long total;
     ej_block_exclusive_sum<DJ_THREADS, unsigned long long>(local, warp_tmp, &total);
     if (threadIdx.x == 0 && total) atomicAdd(cursor, total);
-  } else if (held) {
-    dist_flush<D>(buf, held, R, S, out, cap, cursor);
   }
 }
 
