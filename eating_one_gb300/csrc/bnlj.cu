@@ -11,18 +11,20 @@
 // in-memory hash table instead of being compared one by one):
 //   - each CTA takes one block of up to 16384 R rows and builds its table in
 //     shared memory: rows grouped by bucket (top hash bits, about one row a
-//     bucket) by a counting sort, each bucket one 4-byte {start, count} word;
+//     bucket) by a counting sort, with 2-byte bucket starts;
 //   - S is streamed through two 16 KB shared-memory buffers filled by 1-D TMA
 //     bulk copies (cp.async.bulk + mbarrier complete_tx), so the next S tile
-//     lands while the current one is probed, four S tuples per thread and tile;
-//   - a warp counts the matches of its 128 S tuples, takes their output rows
-//     with one atomic add on the cursor and writes them, consecutive lanes to
-//     consecutive rows (count-only mode sums per-thread counters instead).
-//     Result order is not deterministic; the result multiset is.
+//     lands while the current one is probed, two S tuples per thread and tile;
+//   - a warp collects its matches {S key, R position} in a shared-memory
+//     buffer and turns 64 to 128 of them into rows at a time, with one atomic
+//     add on the cursor and coalesced stores (count-only mode sums per-thread
+//     counters).  Result order is not deterministic; the result multiset is.
 // Work is |S| bucket lookups per 16384 R rows instead of |S| x 16384
-// compares, and what bounds it is the shared-memory pipe (scattered 4-byte
-// reads) and one cursor atomic per 128 S tuples.  2^16 x 2^20 rows over 2^16 keys,
-// the call measured: 4.81 ms by compares (14.4 T/s), 0.112 ms here.
+// compares.  2^16 x 2^20 rows over 2^16 keys, the whole call: by compares 4.81
+// ms (14.4 T/s); 16 warps of four tuples a lane, one cursor atomic per 128 S
+// tuples 0.112 ms (kernel 72 us); 32 warps of two, matches buffered 0.091 ms
+// (kernel 51 us, 33 of them building and counting alone).  What bounds it is
+// the latency of the lookups' dependent shared-memory reads at 32 warps.
 // Waits on the mbarrier are bounded by the handle's wait limit and report
 // EJ_ERR_TIMEOUT instead of hanging; a CTA that gave up still waits (bounded
 // by EJ_DEFAULT_WAIT_LIMIT_NS) for its own copies in flight before it exits.
@@ -33,18 +35,27 @@
 
 namespace {
 
-constexpr int BN_THREADS = 512;
+constexpr int BN_THREADS = 1024;
 constexpr int BN_WARPS = BN_THREADS / 32;
 constexpr int BN_RBLOCK = 16384;   // most R rows per CTA: 128 KB of columns, 64 KB of buckets
-constexpr int BN_MIN_BUCKETS = BN_THREADS * 2;
-constexpr int BN_ITEMS = 4;                      // S tuples per thread and tile
+constexpr int BN_MIN_BUCKETS = 1024;
+constexpr int BN_ITEMS = 2;                      // S tuples per thread and tile
 constexpr int BN_STILE = BN_THREADS * BN_ITEMS;  // S tuples per shared-memory tile (16 KB)
 
-struct BnSmem {
+constexpr int BN_BUF = 128;                      // matches a warp collects
+
+struct BnStream {
   int4 tile[2][BN_STILE / 2];  // two S tuples per int4
-  int32_t rval[BN_RBLOCK];     // the R block, bucket by bucket
+  int2 buf[BN_WARPS][BN_BUF];  // matches {S key, R position}
+};
+struct BnSmem {
+  int32_t rval[BN_RBLOCK];  // the R block, bucket by bucket
   int32_t rkey[BN_RBLOCK];
-  uint32_t bucket[BN_RBLOCK];  // start << 16 | rows (both at most 2^14)
+  union {
+    BnStream st;
+    uint32_t count[BN_RBLOCK];  // the build's bucket counters
+  };
+  uint16_t start[BN_RBLOCK + 2];  // first row of each bucket, then the end
   unsigned long long bar[2];
   unsigned long long warp_tmp[BN_WARPS + 1];
   uint32_t scan_tmp[BN_WARPS + 1];
@@ -88,14 +99,19 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned
 }
 
 // bounded wait by one thread; true when the phase completed in time (limit
-// 0: only if it had completed at the first test)
+// 0: only if it had completed at the first test).  The clock is read when
+// the first test fails, then every 16 tests.
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity,
                                                   unsigned long long limit_ns) {
+  if (mbar_test_wait(bar, parity)) return true;
+  if (limit_ns == 0) return false;
   const unsigned long long t0 = ej_globaltimer();
-  while (!mbar_test_wait(bar, parity)) {
-    if (ej_globaltimer() - t0 >= limit_ns) return false;
-  }
-  return true;
+  do {
+#pragma unroll 1
+    for (int k = 0; k < 16; k++)
+      if (mbar_test_wait(bar, parity)) return true;
+  } while (ej_globaltimer() - t0 < limit_ns);
+  return false;
 }
 
 template <bool USE_TMA>
@@ -105,54 +121,73 @@ __device__ __forceinline__ void issue_tile(BnSmem& sm, int buf, const ej_tuple* 
       const uint32_t pairs = n >> 1;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_expect_tx(&sm.bar[buf], pairs * 16u);
-      if (pairs) tma_load_1d(&sm.tile[buf][0], S + t0, pairs * 16u, &sm.bar[buf]);
+      if (pairs) tma_load_1d(&sm.st.tile[buf][0], S + t0, pairs * 16u, &sm.bar[buf]);
       if (n & 1u) {  // odd tail tuple: plain load (TMA sizes are multiples of 16 bytes)
         const int2 last = *reinterpret_cast<const int2*>(S + t0 + n - 1);
-        reinterpret_cast<int2*>(&sm.tile[buf][0])[n - 1] = last;
+        reinterpret_cast<int2*>(&sm.st.tile[buf][0])[n - 1] = last;
       }
     }
   } else {
-    int2* dst = reinterpret_cast<int2*>(&sm.tile[buf][0]);
+    int2* dst = reinterpret_cast<int2*>(&sm.st.tile[buf][0]);
     const int2* src = reinterpret_cast<const int2*>(S + t0);
     for (uint32_t i = threadIdx.x; i < n; i += BN_THREADS) dst[i] = __ldcs(src + i);
   }
 }
 
 // The table of R[0, n) in shared memory over 2^lg buckets (2^lg >= n, a
-// multiple of 2 BN_THREADS): a counting sort by bucket.  The rows are read
+// multiple of 1024): a counting sort by bucket.  The rows are read
 // twice (they sit in L2), so that none has to wait in registers.
 __device__ __forceinline__ void bn_build(BnSmem& sm, const int2* __restrict__ R, uint32_t n, uint32_t lg) {
   const uint32_t nb = 1u << lg;
-  for (uint32_t b = threadIdx.x; b < nb; b += BN_THREADS) sm.bucket[b] = 0u;
+  for (uint32_t b = threadIdx.x; b < nb; b += BN_THREADS) sm.count[b] = 0u;
   __syncthreads();
+#pragma unroll 8
   for (uint32_t i = threadIdx.x; i < n; i += BN_THREADS)
-    atomicAdd(&sm.bucket[ej_hash32((uint32_t)__ldg(&R[i].y)) >> (32u - lg)], 1u);
+    atomicAdd(&sm.count[ej_hash32((uint32_t)__ldg(&R[i].y)) >> (32u - lg)], 1u);
   __syncthreads();
   // exclusive scan of the counts: each warp a contiguous share, 32 buckets a
-  // step, then the warps' totals
+  // step, then the warps' totals; the counters become row cursors
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t share = nb / BN_WARPS, b0 = warp * share;
   uint32_t run = 0;
-  for (uint32_t b = b0 + lane; b < b0 + share; b += 32) run += sm.bucket[b];
+  for (uint32_t b = b0 + lane; b < b0 + share; b += 32) run += sm.count[b];
   run = __reduce_add_sync(EJ_FULL_MASK, run);
   if (lane == 0) sm.scan_tmp[warp] = run;
   __syncthreads();
   run = __reduce_add_sync(EJ_FULL_MASK, lane < warp ? sm.scan_tmp[lane] : 0u);
   for (uint32_t b = b0 + lane; b < b0 + share; b += 32) {
-    const uint32_t c = sm.bucket[b];
+    const uint32_t c = sm.count[b];
     const uint32_t incl = ej_warp_inclusive_sum(c);
-    sm.bucket[b] = (run + incl - c) << 16;  // the count in the low half grows as rows are placed
+    sm.count[b] = run + incl - c;
+    sm.start[b] = (uint16_t)(run + incl - c);
     run += __shfl_sync(EJ_FULL_MASK, incl, 31);
   }
+  if (threadIdx.x == 0) sm.start[nb] = (uint16_t)n;
   __syncthreads();
+#pragma unroll 8
   for (uint32_t i = threadIdx.x; i < n; i += BN_THREADS) {
     const int2 r = __ldg(R + i);
-    const uint32_t w = atomicAdd(&sm.bucket[ej_hash32((uint32_t)r.y) >> (32u - lg)], 1u);
-    const uint32_t pos = (w >> 16) + (w & 0xFFFFu);
+    const uint32_t pos = atomicAdd(&sm.count[ej_hash32((uint32_t)r.y) >> (32u - lg)], 1u);
     sm.rval[pos] = r.y;
     sm.rkey[pos] = r.x;
   }
   __syncthreads();
+}
+
+// the n matches of a warp's buffer as rows
+__device__ __forceinline__ void bn_flush(const BnSmem& sm, const int2* buf, uint32_t n, ej_result* __restrict__ out,
+                                         uint64_t cap, unsigned long long* cursor) {
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();
+  unsigned long long off = 0;
+  if (lane == 0) off = atomicAdd(cursor, (unsigned long long)n);
+  off = __shfl_sync(EJ_FULL_MASK, off, 0);
+  for (uint32_t k = lane; k < n; k += 32) {
+    const int2 e = buf[k];
+    const int32_t v = sm.rval[e.y];
+    if (off + k < cap) __stcs(reinterpret_cast<int4*>(out + off + k), make_int4(sm.rkey[e.y], v, e.x, v));
+  }
+  __syncwarp();
 }
 
 template <bool USE_TMA, bool COUNT_ONLY>
@@ -178,6 +213,8 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
   }
   bn_build(sm, reinterpret_cast<const int2*>(R + rbase), (uint32_t)min((uint64_t)r_block, nR - rbase), lg);
 
+  int2* found = sm.st.buf[threadIdx.x >> 5];
+  uint32_t held = 0;  // matches in the warp's buffer
   unsigned long long local = 0;
   if (ntiles) issue_tile<USE_TMA>(sm, 0, S, s_begin, (uint32_t)min((uint64_t)BN_STILE, s_end - s_begin));
   uint64_t t;
@@ -195,10 +232,10 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
     }
     __syncthreads();
     if (sm.timed_out) break;
-    // the warp's 128 S tuples, lane l taking tuples l, 32 + l, ...: their
-    // buckets' words first, then all four buckets walked together, one row a
+    // the warp's 64 S tuples, lane l taking tuples l, 32 + l, ...: their
+    // buckets' words first, then all its buckets walked together, one row a
     // round
-    const int2* tile = reinterpret_cast<const int2*>(sm.tile[buf]) + (threadIdx.x >> 5) * (32 * BN_ITEMS);
+    const int2* tile = reinterpret_cast<const int2*>(sm.st.tile[buf]) + (threadIdx.x >> 5) * (32 * BN_ITEMS);
     const uint32_t left = n - min(n, (threadIdx.x >> 5) * (32u * BN_ITEMS));
     int2 s[BN_ITEMS];
     uint32_t at[BN_ITEMS], rows[BN_ITEMS], c[BN_ITEMS], hit[BN_ITEMS], deepest = 0;
@@ -206,9 +243,9 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
     for (int j = 0; j < BN_ITEMS; j++) {
       const bool ok = (uint32_t)j * 32u + lane < left;
       s[j] = ok ? tile[j * 32 + lane] : make_int2(0, 0);
-      const uint32_t w = ok ? sm.bucket[ej_hash32((uint32_t)s[j].y) >> (32u - lg)] : 0u;
-      at[j] = w >> 16;
-      rows[j] = w & 0xFFFFu;
+      const uint32_t b = ej_hash32((uint32_t)s[j].y) >> (32u - lg);
+      at[j] = ok ? sm.start[b] : 0u;
+      rows[j] = ok ? sm.start[b + 1] - at[j] : 0u;
       c[j] = hit[j] = 0;
       deepest = max(deepest, rows[j]);
     }
@@ -224,33 +261,44 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
 #pragma unroll
       for (int j = 0; j < BN_ITEMS; j++) local += c[j];
     } else {
-      // rows of item 0 first, then item 1, ...: lanes write consecutive rows
-      uint32_t excl[BN_ITEMS], all = 0;
+      uint32_t mine = 0;
 #pragma unroll
-      for (int j = 0; j < BN_ITEMS; j++) {
-        const uint32_t incl = ej_warp_inclusive_sum(c[j]);
-        excl[j] = all + incl - c[j];
-        all += __shfl_sync(EJ_FULL_MASK, incl, 31);
-      }
-      if (all) {
-        unsigned long long off = 0;
-        if (lane == 0) off = atomicAdd(cursor, (unsigned long long)all);
-        off = __shfl_sync(EJ_FULL_MASK, off, 0);
+      for (int j = 0; j < BN_ITEMS; j++) mine += c[j];
+      if (__any_sync(EJ_FULL_MASK, mine != 0)) {
+        const uint32_t incl = ej_warp_inclusive_sum(mine);
+        const uint32_t total = __shfl_sync(EJ_FULL_MASK, incl, 31);
+        if (held + total > BN_BUF) {
+          if (held) bn_flush(sm, found, held, out, cap, cursor);
+          held = 0;
+        }
+        // a step with more matches than the buffer holds writes its rows itself
+        const bool direct = total > BN_BUF;
+        unsigned long long pos = held + incl - mine;
+        if (direct) {
+          unsigned long long off = 0;
+          if (lane == 0) off = atomicAdd(cursor, (unsigned long long)total);
+          pos += __shfl_sync(EJ_FULL_MASK, off, 0);
+        } else {
+          held += total;
+        }
 #pragma unroll
         for (int j = 0; j < BN_ITEMS; j++) {
-          unsigned long long pos = off + excl[j];
-          // one match: its row is known; more: the bucket's rows up to the last one
-          for (uint32_t i = c[j] > 1 ? at[j] : hit[j]; c[j] && i <= hit[j]; i++) {
-            if (sm.rval[i] != s[j].y) continue;
-            if (pos < cap)
+          uint32_t i = hit[j];  // the last match, then those before it
+          for (uint32_t left = c[j]; left != 0; pos++) {
+            if (!direct)
+              found[pos] = make_int2(s[j].x, (int)i);
+            else if (pos < cap)
               __stcs(reinterpret_cast<int4*>(out + pos), make_int4(sm.rkey[i], s[j].y, s[j].x, s[j].y));
-            pos++;
+            if (--left)
+              do i--;
+              while (sm.rval[i] != s[j].y);
           }
         }
       }
     }
     __syncthreads();  // everyone is done with `buf` before it is refilled
   }
+  if (!COUNT_ONLY && held) bn_flush(sm, found, held, out, cap, cursor);
   if (sm.timed_out && threadIdx.x == 0) {
     ej_set_status(st, EJ_ERR_TIMEOUT, 2u);
     // drain copies still in flight so none lands after the CTA exits

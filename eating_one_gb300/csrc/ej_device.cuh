@@ -134,7 +134,8 @@ __device__ __forceinline__ void ej_lookback_publish(unsigned long long* status, 
 // come out too small, never too large, so positions derived from them stay
 // inside their buffers.  The clock is read every 64 polls, every poll when
 // the limit is under 100 us (limit 0: give up at the first poll that finds a
-// predecessor not ready).
+// predecessor not ready), and the wait counts from its first reading: a tile
+// whose predecessors are ready never reads it.
 __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long long* status, uint64_t tile,
                                                                   unsigned long long aggregate,
                                                                   ej_dev_status* st, unsigned int where,
@@ -143,7 +144,7 @@ __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long 
   if (tile == 0) return 0ull;
   unsigned long long exclusive = 0;
   int64_t k = (int64_t)tile - 1;
-  const unsigned long long t0 = ej_globaltimer();
+  unsigned long long t0 = 0;  // the clock at its first reading
   const unsigned int period = limit_ns < 100000ull ? 0u : 63u;
   bool gave_up = false;
   for (;;) {
@@ -157,7 +158,11 @@ __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long 
       }
       spins++;
       bool late = false;
-      if ((spins & period) == 0u) late = (ej_globaltimer() - t0) >= limit_ns;
+      if ((spins & period) == 0u) {
+        const unsigned long long now = ej_globaltimer();
+        if (t0 == 0) t0 = now;
+        late = now - t0 >= limit_ns;
+      }
       if (__shfl_sync(EJ_FULL_MASK, late ? 1 : 0, 0)) {
         gave_up = true;
         if ((w >> 62) == 0ull) w = (EJ_LB_PREFIX << 62);
