@@ -38,6 +38,7 @@
 #include "hash_join.cuh"
 #include "probe.cuh"
 #include "probe_write.cuh"
+#include "small_join.cuh"
 
 namespace {
 
@@ -160,13 +161,14 @@ __global__ void vbucket_header_kernel(const int32_t* __restrict__ rval, uint64_t
   *hdr = b;
 }
 
-// bounds of the value buckets: rows [r0, r0 + 256) per warp
+// bounds of the value buckets that hold rows (the others stay zero): rows
+// [r0, r0 + 256) per warp
 __global__ void __launch_bounds__(256)
-vbucket_start_kernel(const int32_t* __restrict__ rval, uint64_t nR, uint2* __restrict__ bucket, uint32_t hb,
+vbucket_start_kernel(const int32_t* __restrict__ rval, uint64_t nR, uint2* __restrict__ bucket,
                      const EjValueBuckets* __restrict__ hdr) {
   const uint64_t r0 = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 256;
   const EjValueBuckets b = *hdr;
-  if (r0 <= nR) ej_bucket_bounds_warp(rval, nR, r0, hb, bucket, EjValueBucketOf{b.vmin, b.vshift});
+  if (r0 <= nR) ej_bucket_edges_warp(rval, nR, r0, bucket, EjValueBucketOf{b.vmin, b.vshift});
 }
 
 // ---- count, then write from the run descriptors ---------------------------------
