@@ -30,6 +30,7 @@
 // by EJ_DEFAULT_WAIT_LIMIT_NS) for its own copies in flight before it exits.
 #include <algorithm>
 
+#include "block_table.cuh"
 #include "ej_device.cuh"
 #include "ej_entry.h"
 
@@ -37,28 +38,25 @@ namespace {
 
 constexpr int BN_THREADS = 1024;
 constexpr int BN_WARPS = BN_THREADS / 32;
-constexpr int BN_RBLOCK = 16384;   // most R rows per CTA: 128 KB of columns, 64 KB of buckets
-constexpr int BN_MIN_BUCKETS = 1024;
+constexpr uint32_t BN_MIN_BUCKETS = 32u * BN_WARPS;
 constexpr int BN_ITEMS = 2;                      // S tuples per thread and tile
 constexpr int BN_STILE = BN_THREADS * BN_ITEMS;  // S tuples per shared-memory tile (16 KB)
 
-constexpr int BN_BUF = 128;                      // matches a warp collects
-
 struct BnStream {
   int4 tile[2][BN_STILE / 2];  // two S tuples per int4
-  int2 buf[BN_WARPS][BN_BUF];  // matches {S key, R position}
+  int2 buf[BN_WARPS][BT_BUF];
 };
 struct BnSmem {
-  int32_t rval[BN_RBLOCK];  // the R block, bucket by bucket
-  int32_t rkey[BN_RBLOCK];
+  int32_t rval[BT_ROWS];
+  int32_t rkey[BT_ROWS];
   union {
     BnStream st;
-    uint32_t count[BN_RBLOCK];  // the build's bucket counters
+    uint32_t count[BT_ROWS];
   };
-  uint16_t start[BN_RBLOCK + 2];  // first row of each bucket, then the end
+  uint16_t start[BT_ROWS + 2];
   unsigned long long bar[2];
   unsigned long long warp_tmp[BN_WARPS + 1];
-  uint32_t scan_tmp[BN_WARPS + 1];
+  uint32_t scan_tmp[BN_WARPS];
   int timed_out;
 };
 static_assert(sizeof(BnSmem) <= 227 * 1024, "one CTA's shared memory");
@@ -134,64 +132,8 @@ __device__ __forceinline__ void issue_tile(BnSmem& sm, int buf, const ej_tuple* 
   }
 }
 
-// The table of R[0, n) in shared memory over 2^lg buckets (2^lg >= n, a
-// multiple of 1024): a counting sort by bucket.  The rows are read
-// twice (they sit in L2), so that none has to wait in registers.
-__device__ __forceinline__ void bn_build(BnSmem& sm, const int2* __restrict__ R, uint32_t n, uint32_t lg) {
-  const uint32_t nb = 1u << lg;
-  for (uint32_t b = threadIdx.x; b < nb; b += BN_THREADS) sm.count[b] = 0u;
-  __syncthreads();
-#pragma unroll 8
-  for (uint32_t i = threadIdx.x; i < n; i += BN_THREADS)
-    atomicAdd(&sm.count[ej_hash32((uint32_t)__ldg(&R[i].y)) >> (32u - lg)], 1u);
-  __syncthreads();
-  // exclusive scan of the counts: each warp a contiguous share, 32 buckets a
-  // step, then the warps' totals; the counters become row cursors
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t share = nb / BN_WARPS, b0 = warp * share;
-  uint32_t run = 0;
-  for (uint32_t b = b0 + lane; b < b0 + share; b += 32) run += sm.count[b];
-  run = __reduce_add_sync(EJ_FULL_MASK, run);
-  if (lane == 0) sm.scan_tmp[warp] = run;
-  __syncthreads();
-  run = __reduce_add_sync(EJ_FULL_MASK, lane < warp ? sm.scan_tmp[lane] : 0u);
-  for (uint32_t b = b0 + lane; b < b0 + share; b += 32) {
-    const uint32_t c = sm.count[b];
-    const uint32_t incl = ej_warp_inclusive_sum(c);
-    sm.count[b] = run + incl - c;
-    sm.start[b] = (uint16_t)(run + incl - c);
-    run += __shfl_sync(EJ_FULL_MASK, incl, 31);
-  }
-  if (threadIdx.x == 0) sm.start[nb] = (uint16_t)n;
-  __syncthreads();
-#pragma unroll 8
-  for (uint32_t i = threadIdx.x; i < n; i += BN_THREADS) {
-    const int2 r = __ldg(R + i);
-    const uint32_t pos = atomicAdd(&sm.count[ej_hash32((uint32_t)r.y) >> (32u - lg)], 1u);
-    sm.rval[pos] = r.y;
-    sm.rkey[pos] = r.x;
-  }
-  __syncthreads();
-}
-
-// the n matches of a warp's buffer as rows
-__device__ __forceinline__ void bn_flush(const BnSmem& sm, const int2* buf, uint32_t n, ej_result* __restrict__ out,
-                                         uint64_t cap, unsigned long long* cursor) {
-  const uint32_t lane = threadIdx.x & 31u;
-  __syncwarp();
-  unsigned long long off = 0;
-  if (lane == 0) off = atomicAdd(cursor, (unsigned long long)n);
-  off = __shfl_sync(EJ_FULL_MASK, off, 0);
-  for (uint32_t k = lane; k < n; k += 32) {
-    const int2 e = buf[k];
-    const int32_t v = sm.rval[e.y];
-    if (off + k < cap) __stcs(reinterpret_cast<int4*>(out + off + k), make_int4(sm.rkey[e.y], v, e.x, v));
-  }
-  __syncwarp();
-}
-
 template <bool USE_TMA, bool COUNT_ONLY>
-__global__ void __launch_bounds__(BN_THREADS)
+__global__ void __launch_bounds__(BN_THREADS, 1)
 bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32_t lg, const ej_tuple* __restrict__ S,
            uint64_t nS, uint64_t s_per_cta, ej_result* __restrict__ out, uint64_t cap, unsigned long long* cursor,
            ej_dev_status* st, unsigned long long wait_ns) {
@@ -211,10 +153,11 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
   }
-  bn_build(sm, reinterpret_cast<const int2*>(R + rbase), (uint32_t)min((uint64_t)r_block, nR - rbase), lg);
+  const BtTable table = {sm.rval, sm.rkey, sm.count, sm.start, sm.scan_tmp, lg};
+  bt_build<BN_THREADS>(table, reinterpret_cast<const int2*>(R + rbase), (uint32_t)min((uint64_t)r_block, nR - rbase));
 
-  int2* found = sm.st.buf[threadIdx.x >> 5];
-  uint32_t held = 0;  // matches in the warp's buffer
+  BtBuffer found = {sm.st.buf[threadIdx.x >> 5], 0u};
+  const BtOut rows = {out, cap, cursor, nullptr};
   unsigned long long local = 0;
   if (ntiles) issue_tile<USE_TMA>(sm, 0, S, s_begin, (uint32_t)min((uint64_t)BN_STILE, s_end - s_begin));
   uint64_t t;
@@ -232,73 +175,20 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
     }
     __syncthreads();
     if (sm.timed_out) break;
-    // the warp's 64 S tuples, lane l taking tuples l, 32 + l, ...: their
-    // buckets' words first, then all its buckets walked together, one row a
-    // round
-    const int2* tile = reinterpret_cast<const int2*>(sm.st.tile[buf]) + (threadIdx.x >> 5) * (32 * BN_ITEMS);
-    const uint32_t left = n - min(n, (threadIdx.x >> 5) * (32u * BN_ITEMS));
+    // the warp's 64 S tuples, lane l taking tuples l and 32 + l
+    const uint32_t w0 = (threadIdx.x >> 5) * (32u * BN_ITEMS);
+    const int2* tile = reinterpret_cast<const int2*>(sm.st.tile[buf]) + w0;
     int2 s[BN_ITEMS];
-    uint32_t at[BN_ITEMS], rows[BN_ITEMS], c[BN_ITEMS], hit[BN_ITEMS], deepest = 0;
+    bool ok[BN_ITEMS];
 #pragma unroll
     for (int j = 0; j < BN_ITEMS; j++) {
-      const bool ok = (uint32_t)j * 32u + lane < left;
-      s[j] = ok ? tile[j * 32 + lane] : make_int2(0, 0);
-      const uint32_t b = ej_hash32((uint32_t)s[j].y) >> (32u - lg);
-      at[j] = ok ? sm.start[b] : 0u;
-      rows[j] = ok ? sm.start[b + 1] - at[j] : 0u;
-      c[j] = hit[j] = 0;
-      deepest = max(deepest, rows[j]);
+      ok[j] = w0 + (uint32_t)j * 32u + lane < n;
+      s[j] = ok[j] ? tile[j * 32 + lane] : make_int2(0, 0);
     }
-    for (uint32_t k = 0; k < deepest; k++) {
-#pragma unroll
-      for (int j = 0; j < BN_ITEMS; j++)
-        if (k < rows[j] && sm.rval[at[j] + k] == s[j].y) {
-          c[j]++;
-          hit[j] = at[j] + k;
-        }
-    }
-    if (COUNT_ONLY) {
-#pragma unroll
-      for (int j = 0; j < BN_ITEMS; j++) local += c[j];
-    } else {
-      uint32_t mine = 0;
-#pragma unroll
-      for (int j = 0; j < BN_ITEMS; j++) mine += c[j];
-      if (__any_sync(EJ_FULL_MASK, mine != 0)) {
-        const uint32_t incl = ej_warp_inclusive_sum(mine);
-        const uint32_t total = __shfl_sync(EJ_FULL_MASK, incl, 31);
-        if (held + total > BN_BUF) {
-          if (held) bn_flush(sm, found, held, out, cap, cursor);
-          held = 0;
-        }
-        // a step with more matches than the buffer holds writes its rows itself
-        const bool direct = total > BN_BUF;
-        unsigned long long pos = held + incl - mine;
-        if (direct) {
-          unsigned long long off = 0;
-          if (lane == 0) off = atomicAdd(cursor, (unsigned long long)total);
-          pos += __shfl_sync(EJ_FULL_MASK, off, 0);
-        } else {
-          held += total;
-        }
-#pragma unroll
-        for (int j = 0; j < BN_ITEMS; j++) {
-          uint32_t i = hit[j];  // the last match, then those before it
-          for (uint32_t left = c[j]; left != 0; pos++) {
-            if (!direct)
-              found[pos] = make_int2(s[j].x, (int)i);
-            else if (pos < cap)
-              __stcs(reinterpret_cast<int4*>(out + pos), make_int4(sm.rkey[i], s[j].y, s[j].x, s[j].y));
-            if (--left)
-              do i--;
-              while (sm.rval[i] != s[j].y);
-          }
-        }
-      }
-    }
+    local += bt_probe<COUNT_ONLY, false, false>(table, s, ok, 0u, nullptr, found, rows);
     __syncthreads();  // everyone is done with `buf` before it is refilled
   }
-  if (!COUNT_ONLY && held) bn_flush(sm, found, held, out, cap, cursor);
+  if (!COUNT_ONLY && found.held) bt_flush<false>(table, found, nullptr, rows);
   if (sm.timed_out && threadIdx.x == 0) {
     ej_set_status(st, EJ_ERR_TIMEOUT, 2u);
     // drain copies still in flight so none lands after the CTA exits
@@ -327,7 +217,7 @@ ej_status launch_bnl(ej_handle* h, dim3 grid, const ej_tuple* R, uint64_t nR, ui
 ej_status bnl_launch(ej_handle* h, const ej_tuple* R, uint64_t nR, const ej_tuple* S, uint64_t nS,
                      ej_result* out, uint64_t cap, bool count_only, unsigned long long* cursor) {
   if (nR == 0 || nS == 0) return EJ_OK;
-  const uint64_t rchunks = (nR + BN_RBLOCK - 1) / BN_RBLOCK;
+  const uint64_t rchunks = (nR + BT_ROWS - 1) / BT_ROWS;
   if (rchunks > 0x7FFFFFFFull) return ej_fail(h, EJ_ERR_TOO_LARGE, "R too large for the nested loop");
   const uint32_t r_block = (uint32_t)((nR + rchunks - 1) / rchunks);  // blocks of even size
   const uint32_t lg = std::max(ej_ceil_log2(r_block), ej_ceil_log2(BN_MIN_BUCKETS));  // one row a bucket or less

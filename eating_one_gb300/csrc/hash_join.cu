@@ -556,8 +556,9 @@ ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple
     uint2* bucket = reinterpret_cast<uint2*>(static_cast<char*>(aux) + EJ_VBUCKET_HEADER_BYTES);
     vbucket_header_kernel<<<1, 1, 0, h->stream>>>(rval, tp.nR, tp.hb, vh);
     EJ_TRY(ej_check_launch(h, "vbucket_header_kernel"));
+    EJ_CUDA(h, cudaMemsetAsync(bucket, 0, sizeof(uint2) << tp.hb, h->stream));
     const uint64_t blocks = (tp.nR + 1 + 2047) / 2048;  // 256 rows per warp, 8 warps per block
-    vbucket_start_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(rval, tp.nR, bucket, tp.hb, vh);
+    vbucket_start_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(rval, tp.nR, bucket, vh);
     EJ_TRY(ej_check_launch(h, "vbucket_start_kernel"));
     view->bucket = bucket;
     view->vbuckets = vh;
@@ -728,6 +729,12 @@ ej_status ej_hash_join_run(ej_handle* h, const ej_tuple* R, uint64_t nR, const e
   if (mode == 0 && h->prep_valid && h->prep && h->prep->arena == h->arena && h->prep->R == R &&
       h->prep->nR == nR && h->prep->S == S && h->prep->nS == nS)
     return hash_join_write_kept(h, out, out_cap, d_count);
+  // build sides that fit in shared memory: one launch, nothing worth keeping
+  // for the write (the build-side-only join keeps its rows in probe order)
+  if (mode != 1 && ej_small_join_applies(h, nR)) {
+    h->prep_valid = false;
+    return ej_small_join(h, R, nR, S, nS, /*outer=*/false, mode == 2, out, out_cap, d_count ? d_count : h->d_words + 3);
+  }
   // a count keeps its table, partitioned S and run descriptors for the write
   // that follows it
   const bool keep = mode == 2 && h->opt_count_reuse;

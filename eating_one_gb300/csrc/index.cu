@@ -20,6 +20,7 @@
 #include "hash_join.cuh"
 #include "probe.cuh"
 #include "probe_write.cuh"
+#include "small_join.cuh"
 
 struct ej_index {
   int kind = EJ_TABLE_HASH;
@@ -332,6 +333,13 @@ extern "C" ej_status ej_left_outer_join(ej_handle* h, const ej_tuple* R, uint64_
   EJ_TRY(ej_check_rel(h, "R", R, nR));
   EJ_TRY(ej_check_rel(h, "S", S, nS));
   EJ_TRY(ej_check_out(h, out, out_cap, out_count));
+  if (ej_small_join_applies(h, nR)) {
+    EJ_TRY(ej_small_join(h, R, nR, S, nS, /*outer=*/true, /*count_only=*/false, out, out_cap, h->d_words));
+    uint64_t rows = 0;
+    EJ_TRY(ej_finish(h, &rows));
+    *out_count = rows;
+    return ej_capacity_result(h, rows, out_cap);
+  }
   const uint32_t pb = ej_probe_partition_bits(h, nR, nS);
   ej_plan_bytes p;
   ej_table_plan_t tp;

@@ -205,7 +205,11 @@ ej_status ej_hash_join(ej_handle* h, const ej_tuple* R, uint64_t nR, const ej_tu
  * with the same R, nR, S and nS only writes the rows from them.  R and S must
  * not change in between.  Any other call that uses the handle's scratch drops
  * what the count kept (the join then runs whole); a write cut short by
- * out_cap keeps it for the retry.  EJ_OPT_COUNT_REUSE = 0 turns this off. */
+ * out_cap keeps it for the retry.  EJ_OPT_COUNT_REUSE = 0 turns this off.
+ * Build sides of at most 16384 rows are joined in shared memory by one launch
+ * (unless EJ_OPT_BUILD, EJ_OPT_TABLE, EJ_OPT_BUCKET_BITS_DELTA,
+ * EJ_OPT_PROBE_PARTITION_BITS or EJ_OPT_PROBE_WARPS asks for a table in
+ * global memory); their count keeps nothing. */
 ej_status ej_hash_join_count(ej_handle* h, const ej_tuple* R, uint64_t nR, const ej_tuple* S,
                              uint64_t nS, uint64_t* out_count);
 /* Asynchronous form: no host synchronisation; the total count is written to
