@@ -220,6 +220,8 @@ ej_status ej_partition_pass_src(ej_handle* h, const ej_radix_plan& rp, ej_tuple*
 // EJ_TABLE_SORTED: sorted by val; bucket b of value v = (v - vmin) >> vshift
 //   is rows [bucket[b].x, bucket[b].y), with vmin, vmax and vshift in a
 //   16-byte device header (vbuckets) written after the sort.
+// Hash tables of at most EJ_SLOT_MAX_ROWS rows are not sorted: one slot per
+// distinct key, open addressing (pair, npairs, rkey; slot_table.cuh).
 // Both arrays carry EJ_TABLE_PAD readable elements past nR (vector loads).
 enum { EJ_TABLE_HASH = 0, EJ_TABLE_SORTED = 1 };
 constexpr uint64_t EJ_TABLE_PAD = 8;
@@ -231,6 +233,8 @@ struct ej_table_view {
   const uint2* dir = nullptr;        // (hash, single tables) key directory {hash, run start [, length]}
   const uint32_t* dir_bits = nullptr;  // device word: the directory has 2^bits home slots
   uint32_t dir_packed = 0;             // entries {hash, start << 5 | run length} (tables under 2^27 rows)
+  const uint4* pair = nullptr;       // (hash, slot tables) [npairs] pairs of slots
+  uint32_t npairs = 0;
   const void* vbuckets = nullptr;    // (sorted) device EjValueBuckets {vmin, vmax, vshift} of `bucket`
   uint64_t nR = 0;
   uint32_t hb = 1;

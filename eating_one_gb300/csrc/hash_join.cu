@@ -38,6 +38,7 @@
 #include "hash_join.cuh"
 #include "probe.cuh"
 #include "probe_write.cuh"
+#include "slot_table.cuh"
 #include "small_join.cuh"
 
 namespace {
@@ -169,6 +170,129 @@ vbucket_start_kernel(const int32_t* __restrict__ rval, uint64_t nR, uint2* __res
   const uint64_t r0 = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 256;
   const EjValueBuckets b = *hdr;
   if (r0 <= nR) ej_bucket_edges_warp(rval, nR, r0, bucket, EjValueBucketOf{b.vmin, b.vshift});
+}
+
+// ---- slot tables (slot_table.cuh) --------------------------------------------------
+
+constexpr int SLOT_ITEMS = 4;  // rows per thread and step of the build's kernels
+
+struct SlotHeader {
+  uint32_t marked;  // some row was marked: a key has several rows
+  uint32_t cursor;  // words of rkey[] reserved
+};
+static_assert(sizeof(SlotHeader) <= EJ_SLOT_HEADER_BYTES, "slot table header");
+
+// every row to its key's slot, or marked
+__global__ void __launch_bounds__(256)
+slot_insert_kernel(const int2* __restrict__ R, uint32_t n, unsigned long long* __restrict__ slot, uint32_t npairs,
+                   uint32_t* __restrict__ mark, uint2* __restrict__ rank, SlotHeader* hdr) {
+  const uint64_t base = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 * SLOT_ITEMS) + (threadIdx.x & 31u);
+  int32_t key[SLOT_ITEMS];
+  uint32_t hv[SLOT_ITEMS], any = 0;
+  EjSlotMark m[SLOT_ITEMS];
+  bool ok[SLOT_ITEMS];
+#pragma unroll
+  for (int j = 0; j < SLOT_ITEMS; j++) {
+    ok[j] = base + 32 * j < n;
+    const int2 r = ok[j] ? __ldg(R + base + 32 * j) : make_int2(0, 0);
+    key[j] = r.x;
+    hv[j] = ej_hash32((uint32_t)r.y);
+  }
+  ej_slot_insert<SLOT_ITEMS>(slot, npairs, key, hv, ok, m);
+#pragma unroll
+  for (int j = 0; j < SLOT_ITEMS; j++) {
+    if (ok[j]) mark[base + 32 * j] = m[j].mark;
+    if (m[j].mark) rank[base + 32 * j] = make_uint2(m[j].rank, (uint32_t)m[j].first);
+    any |= m[j].mark;
+  }
+  if (__any_sync(EJ_FULL_MASK, any != 0u) && (threadIdx.x & 31u) == 0u) hdr->marked = 1u;
+}
+
+// The passes over the marked rows: a few blocks per SM stride over the rows, so
+// that a launch costs next to nothing when there are none.
+__global__ void __launch_bounds__(256)
+slot_reserve_kernel(uint32_t n, uint2* __restrict__ slot, const uint32_t* __restrict__ mark,
+                    const uint2* __restrict__ rank, int32_t* __restrict__ rkey, SlotHeader* hdr) {
+  if (hdr->marked == 0u) return;
+  constexpr uint32_t SPAN = 32 * SLOT_ITEMS;
+  for (uint64_t b = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * SPAN; b < n; b += (uint64_t)gridDim.x * 8 * SPAN) {
+    uint32_t m[SLOT_ITEMS];
+    uint2 r[SLOT_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SLOT_ITEMS; j++) {
+      const uint64_t i = b + 32 * j + (threadIdx.x & 31u);
+      m[j] = i < n ? __ldg(mark + i) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < SLOT_ITEMS; j++)
+      r[j] = m[j] ? __ldg(rank + b + 32 * j + (threadIdx.x & 31u)) : make_uint2(0u, 0u);
+    ej_slot_reserve<SLOT_ITEMS>(slot, m, r, rkey, &hdr->cursor);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+slot_place_kernel(const int2* __restrict__ R, uint32_t n, const uint2* __restrict__ slot,
+                  const uint32_t* __restrict__ mark, const uint2* __restrict__ rank, int32_t* __restrict__ rkey,
+                  const SlotHeader* __restrict__ hdr) {
+  if (hdr->marked == 0u) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
+    const uint32_t m = __ldg(mark + i);
+    if (m) rkey[(__ldg(&slot[m - 1u].x) >> 5) + (__ldg(&rank[i].x) & ~EJ_SLOT_OPENER)] = __ldg(&R[i].x);
+  }
+}
+
+template <bool OUTER, bool DESC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 40 / WARPS)
+slot_count_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
+                          unsigned long long* __restrict__ wcount, uint64_t nwtiles, void* __restrict__ desc) {
+  const uint64_t w = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+  if (w >= nwtiles) return;
+  const unsigned long long total = ej_slot_count<OUTER, DESC>(P, w, nP, ej_slots_of(t), desc, nwtiles);
+  if ((threadIdx.x & 31u) == 0) wcount[w] = total;
+}
+
+template <bool OUTER, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
+slot_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc, uint64_t nP, ej_table_view t,
+                          const unsigned long long* __restrict__ woff, uint64_t nwtiles, ej_result* __restrict__ out,
+                          uint64_t cap, ej_dev_status* st) {
+  __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
+  const unsigned int warp = threadIdx.x >> 5;
+  const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
+  if (w >= nwtiles) return;
+  if (w == 0 && threadIdx.x == 0 && woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+  const unsigned long long off = woff[w];
+  if (off >= cap) return;
+  ej_slot_write<OUTER>(P, desc, w, nwtiles, nP, t, off, out, cap, stage[warp]);
+}
+
+// One pass, as probe_fused_kernel: find, one atomic add on the row cursor per
+// warp, write; the row order is not deterministic.
+template <bool OUTER, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
+slot_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, uint64_t nwtiles,
+                    unsigned long long* __restrict__ cursor, ej_result* __restrict__ out, uint64_t cap,
+                    ej_dev_status* st) {
+  __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
+  const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
+  if (w >= nwtiles) return;
+  EjProbeWarp p;
+  int32_t key[PR_ITEMS];
+  ej_slot_probe<OUTER>(P, w * PR_WTILE, nP, ej_slots_of(t), p, key);
+  unsigned long long mine = 0;
+#pragma unroll
+  for (int j = 0; j < PR_ITEMS; j++) mine += p.cnt[j];
+  const unsigned long long total = ej_warp_sum<unsigned long long>(mine);
+  if (total == 0) return;
+  unsigned long long off = 0;
+  if (lane == 0) {
+    off = atomicAdd(cursor, total);
+    if (off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+  }
+  off = __shfl_sync(EJ_FULL_MASK, off, 0);
+  if (off >= cap) return;
+  ej_slot_emit(p, key, t, off, out, cap, stage[warp]);
 }
 
 // ---- count, then write from the run descriptors ---------------------------------
@@ -349,6 +473,14 @@ ej_status launch_count_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
   const uint64_t ahead = (uint64_t)h->num_sms * 40;  // warp tiles of one resident wave
   const dim3 grid((unsigned)pp.ntiles);
   constexpr int TH = WARPS * 32;
+  if (KIND == EJ_TABLE_HASH && t.pair) {
+    if (desc)
+      slot_count_kernel<OUTER, true, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, desc);
+    else
+      slot_count_kernel<OUTER, false, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles,
+                                                                                 nullptr);
+    return ej_check_launch(h, "slot_count_kernel");
+  }
   // inner probes of a packed key directory, 16-byte aligned: the lean count
   // (8 warps of two tiles per block, 4 blocks per SM)
   if (KIND == EJ_TABLE_HASH && !OUTER && t.dir && t.dir_packed && (reinterpret_cast<uintptr_t>(P) & 15u) == 0 &&
@@ -388,6 +520,11 @@ ej_status launch_write_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
   const uint64_t ahead = (uint64_t)h->num_sms * 32;  // warp tiles of one resident wave
   const dim3 grid((unsigned)pp.ntiles);
   constexpr int TH = WARPS * 32;
+  if (KIND == EJ_TABLE_HASH && t.pair) {
+    slot_write_kernel<OUTER, WARPS><<<grid, TH, 0, h->stream>>>(P, desc, pp.nP, t, woff, pp.nwtiles, out, cap,
+                                                                        h->d_status);
+    return ej_check_launch(h, "slot_write_kernel");
+  }
   if (desc_form(t) == EJ_DESC_NONE)
     probe_write_kernel<KIND, OUTER, EJ_DESC_NONE, WARPS><<<grid, TH, 0, h->stream>>>(
         P, nullptr, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead);
@@ -420,7 +557,21 @@ uint32_t ej_table_bucket_bits(uint64_t nR, int delta) {
 // ---- table build --------------------------------------------------------
 
 
+// Slot tables up to this many rows are at most a quarter full, larger ones half.
+// 2^20 rows, one join of 2^22 probes: a quarter 151 us, half 171 (the inserts walk
+// longer); but two 2^20-row dimension tables probed by 2^26 facts 1.60 ms at a
+// quarter, 1.35 at half (32 MB less in L2), so probe-heavy callers take half.
+constexpr uint64_t SLOT_QUARTER_ROWS = 1ull << 20;
+
+bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {
+  return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table != EJ_TABLE_FORMAT_DIRECTORY;
+}
+
+// the runs of a slot table: every row, and a count for each of 31 rows and more
+static size_t ej_slot_run_bytes(uint64_t nR) { return ej_table_col_bytes(nR + nR / 31 + 1); }
+
 size_t ej_table_aux_bytes(const ej_table_plan_t& tp) {
+  if (tp.slots) return EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4) + ej_slot_run_bytes(tp.nR);
   const size_t buckets = (size_t(1) << tp.hb) * sizeof(uint2);
   if (tp.kind != EJ_TABLE_HASH) return EJ_VBUCKET_HEADER_BYTES + buckets;
   // a directory table keeps room for the bucket bounds its build may choose instead
@@ -441,12 +592,20 @@ void ej_table_plan(ej_plan_bytes& p, ej_table_plan_t& tp, uint64_t nR, bool own_
                    const ej_table_knobs& k, uint64_t n_probe) {
   tp.kind = kind;
   tp.nR = nR;
+  tp.slots = kind == EJ_TABLE_HASH && ej_table_is_slots(nR, k);
+  if (tp.slots) {
+    // at least one pair per row (the walks' bound); a quarter full while that
+    // keeps the table well inside L2 and the build is not dwarfed by the probes
+    tp.npairs = (uint32_t)(nR <= SLOT_QUARTER_ROWS && n_probe <= 16 * nR ? 2 * nR + 1 : nR + 1);
+    if (!own_storage) tp.aux_off = p.add(ej_table_aux_bytes(tp));
+    tp.mark_off = p.add((size_t)(nR ? nR : 1) * sizeof(uint32_t));
+    tp.rank_off = p.add((size_t)(nR ? nR : 1) * sizeof(uint2));
+    return;
+  }
   // a directory chosen by the tuning is kept whatever the runs' length
   tp.prefer_dir = n_probe > 16 * nR || k.table == EJ_TABLE_FORMAT_DIRECTORY;
-  tp.use_dir = kind == EJ_TABLE_HASH &&
-               (k.table == EJ_TABLE_FORMAT_DIRECTORY ||
-                (k.table == EJ_TABLE_FORMAT_PLANNER &&
-                 (nR >= EJ_DIR_MIN_ROWS || (tp.prefer_dir && nR >= EJ_DIR_PROBE_MIN_ROWS))));
+  tp.use_dir = kind == EJ_TABLE_HASH && (k.table == EJ_TABLE_FORMAT_DIRECTORY ||
+                                         (k.table == EJ_TABLE_FORMAT_PLANNER && nR >= EJ_DIR_MIN_ROWS));
   tp.hb = ej_table_bucket_bits(nR, k.delta);  // hash buckets, or value buckets of a sorted table
   tp.passes = 4;  // all 32 key bits: equal keys end up adjacent
   if (!own_storage) {
@@ -486,6 +645,33 @@ size_t ej_table_bytes(uint64_t nR, int delta) {
 
 ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple* R, int32_t* rkey, int32_t* rval,
                          void* aux, ej_table_view* view) {
+  if (tp.slots) {
+    SlotHeader* hdr = static_cast<SlotHeader*>(aux);
+    uint2* slot = reinterpret_cast<uint2*>(static_cast<char*>(aux) + EJ_SLOT_HEADER_BYTES);
+    unsigned long long* slot64 = reinterpret_cast<unsigned long long*>(slot);
+    int32_t* runs = reinterpret_cast<int32_t*>(slot + 2 * (size_t)tp.npairs);
+    uint32_t* mark = reinterpret_cast<uint32_t*>(ej_arena_at(h, tp.mark_off));
+    uint2* rank = reinterpret_cast<uint2*>(ej_arena_at(h, tp.rank_off));
+    const int2* R2 = reinterpret_cast<const int2*>(R);
+    const uint32_t n = (uint32_t)tp.nR;
+    const unsigned blocks = (n + 256 * SLOT_ITEMS - 1) / (256 * SLOT_ITEMS);
+    const unsigned few = std::min<unsigned>((n + 255) / 256, (unsigned)h->num_sms * 8);
+    EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4), h->stream));
+    if (n) {
+      slot_insert_kernel<<<blocks, 256, 0, h->stream>>>(R2, n, slot64, tp.npairs, mark, rank, hdr);
+      EJ_TRY(ej_check_launch(h, "slot_insert_kernel"));
+      slot_reserve_kernel<<<few, 256, 0, h->stream>>>(n, slot, mark, rank, runs, hdr);
+      EJ_TRY(ej_check_launch(h, "slot_reserve_kernel"));
+      slot_place_kernel<<<few, 256, 0, h->stream>>>(R2, n, slot, mark, rank, runs, hdr);
+      EJ_TRY(ej_check_launch(h, "slot_place_kernel"));
+    }
+    view->kind = EJ_TABLE_HASH;
+    view->nR = tp.nR;
+    view->rkey = runs;
+    view->pair = reinterpret_cast<const uint4*>(slot);
+    view->npairs = tp.npairs;
+    return EJ_OK;
+  }
   // LSD passes over the 32-bit key (hash32(val), or the order-preserving image
   // of val for a sorted index), least significant byte first; the last pass
   // writes the two columns
@@ -577,7 +763,8 @@ void ej_probe_plan(ej_plan_bytes& p, ej_probe_plan_t& pp, uint64_t nP, bool with
   pp.off_off = p.add((pp.nwtiles + 1) * sizeof(unsigned long long));
   pp.scan_off = p.add(ej_scan_scratch_bytes(pp.nwtiles));
   pp.with_desc = with_desc;
-  if (with_desc) pp.desc_off = p.add((size_t)(nP ? nP : 1) * sizeof(uint2));
+  // whole warp tiles of 8-byte descriptors: the wide form; the others take less
+  if (with_desc) pp.desc_off = p.add((size_t)(pp.nwtiles ? pp.nwtiles : 1) * PR_WTILE * sizeof(uint2));
 }
 
 ej_status ej_probe_count(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
@@ -617,9 +804,11 @@ ej_status ej_probe_write(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
 
 uint32_t ej_probe_partition_bits(const ej_handle* h, uint64_t nR, uint64_t nS) {
   (void)nS;
-  const uint32_t hb = ej_table_bucket_bits(nR, ej_tuned_bucket_delta(h, nR));
+  const ej_table_knobs k = ej_tuned_table_knobs(h, nR);
+  const uint32_t hb = ej_table_bucket_bits(nR, k.delta);
   const int forced = ej_tuned_partition_bits(h, nR);
   if (forced >= 0) return std::min<uint32_t>((uint32_t)forced, std::min(hb, 8u));
+  if (ej_table_is_slots(nR, k)) return 0;  // at most 64 MB of slots: L2 holds what the probes touch
   const double table = (double)ej_table_bytes(nR, ej_tuned_bucket_delta(h, nR));
   const double l2 = (double)(h->l2_bytes ? h->l2_bytes : (size_t)126 << 20);
   if (table <= l2 / 4.0) return 0;  // the whole table stays L2-resident
@@ -651,6 +840,12 @@ template <int KIND, bool OUTER, int WARPS>
 static ej_status launch_fused_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
                                 unsigned long long* cursor, ej_result* out, uint64_t cap) {
   const uint64_t ahead = (uint64_t)h->num_sms * 32;  // warp tiles of one resident wave
+  if (KIND == EJ_TABLE_HASH && t.pair) {
+    slot_fused_kernel<OUTER, WARPS><<<(unsigned)pp.ntiles, WARPS * 32, 0, h->stream>>>(P, pp.nP, t, pp.nwtiles,
+                                                                                          cursor, out, cap,
+                                                                                          h->d_status);
+    return ej_check_launch(h, "slot_fused_kernel");
+  }
   if (t.short_runs)
     probe_fused_kernel<KIND, OUTER, EJ_KEYS_CHUNKS, WARPS><<<(unsigned)pp.ntiles, WARPS * 32, 0, h->stream>>>(
         P, pp.nP, t, pp.nwtiles, cursor, out, cap, h->d_status, ahead);

@@ -9,15 +9,19 @@
 #include "msd.cuh"
 #include "onesweep.cuh"
 
+// Hash tables of at most EJ_SLOT_MAX_ROWS rows are slot tables
+// (slot_table.cuh) unless the handle's options or tuning table choose a sort, a
+// load factor or a key directory.  At 2^22 rows the slots take 64 MB, half of
+// L2; the largest sizes measured, 3 M and 2^22 rows, still join faster than with
+// the sorted tables (3 M unique keys 290 us against 424, 2^22 447 against 576).
+constexpr uint64_t EJ_SLOT_MAX_ROWS = 1ull << 22;
+constexpr size_t EJ_SLOT_HEADER_BYTES = 256;  // counters, cleared with the slots
 // Hash tables of at least EJ_DIR_MIN_ROWS rows may carry a key directory (one
 // load per probe, seven build launches): the build keeps it when the table's
 // runs average two rows or more and otherwise switches to bucket bounds (one
-// build launch); tables from EJ_DIR_PROBE_MIN_ROWS rows keep it whenever the
-// caller probes 16 rows per table row or more.  Smaller tables carry bucket
-// bounds (the bucket scan costs no more than a directory lookup while the
-// table sits in L2).
-constexpr uint64_t EJ_DIR_MIN_ROWS = 1ull << 22;
-constexpr uint64_t EJ_DIR_PROBE_MIN_ROWS = 1ull << 20;
+// build launch), whenever the caller probes 16 rows per table row or more it
+// keeps it.
+constexpr uint64_t EJ_DIR_MIN_ROWS = EJ_SLOT_MAX_ROWS;
 // a sorted table's aux storage: the value buckets' header, then the bounds
 constexpr size_t EJ_VBUCKET_HEADER_BYTES = 256;
 
@@ -31,6 +35,9 @@ struct ej_table_plan_t {
   uint32_t passes = 4;  // LSD radix passes over the 32-bit key
   bool msd = false;       // large hash tables: MSD passes + bucket sorts instead (msd.cuh)
   ej_msd_plan mplan;
+  bool slots = false;     // slot table: no sort, no columns
+  uint32_t npairs = 0;
+  size_t mark_off = 0, rank_off = 0;
   bool onesweep = false;  // sorted indexes (and hash tables when chosen): one scatter launch per digit
   ej_onesweep_plan oplan;
   // arena offsets; rkey/rval/aux are unused when the table has its own storage
@@ -71,6 +78,8 @@ struct ej_table_knobs {
   int table = EJ_TABLE_FORMAT_PLANNER;
 };
 ej_table_knobs ej_tuned_table_knobs(const ej_handle* h, uint64_t nR);
+// whether a hash table of nR rows is a slot table
+bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k);
 // n_probe: the probe rows the caller expects (0: unknown)
 void ej_table_plan(ej_plan_bytes& p, ej_table_plan_t& tp, uint64_t nR, bool own_storage, int kind,
                    const ej_table_knobs& k = ej_table_knobs(), uint64_t n_probe = 0);

@@ -34,6 +34,7 @@ constexpr int PW_PREFETCH = 4;                  // run keys held in registers pe
 constexpr uint32_t PW_STAGE_ROWS = 256;         // staged rows per warp (4 KB)
 constexpr uint32_t PW_BIG_RUN = 1u << 26;       // a run at least this long makes its group use 64-bit prefixes
 constexpr uint32_t NULL_RUN = 0xFFFFFFFFu;      // OUTER: the NULL-extended row
+constexpr uint32_t INLINE_RUN = 0xFFFFFFFEu;    // inline tables: one row, its key in the probe's slot
 
 struct EjProbeWarp {
   int2 s[PR_ITEMS];
@@ -101,9 +102,11 @@ __device__ __forceinline__ unsigned long long ej_group_rows(uint32_t c, uint32_t
 //                   loads (batched tables, whose runs are mostly of one or
 //                   two rows).
 enum { EJ_KEYS_WINDOW = 0, EJ_KEYS_CHUNKS = 1 };
-template <int KEYS = EJ_KEYS_WINDOW>
+// INL (inline tables): rows found in slots (INLINE_RUN) have their key in key[].
+template <int KEYS = EJ_KEYS_WINDOW, bool INL = false>
 __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const EjProbeWarp& w,
-                                                  int32_t (&kk)[PR_ITEMS][PW_PREFETCH]) {
+                                                  int32_t (&kk)[PR_ITEMS][PW_PREFETCH],
+                                                  const int32_t (&key)[PR_ITEMS] = {}) {
   static_assert(PW_PREFETCH == 4, "the window holds 4 keys past any offset");
   constexpr bool chunks = KEYS == EJ_KEYS_CHUNKS;
   const int4* rk4 = reinterpret_cast<const int4*>(t.rkey - t.voff);
@@ -114,7 +117,7 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
   for (int j = 0; j < PR_ITEMS; j++) {
     qa[j] = qb[j] = make_int4(EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY);
     o[j] = 0;
-    if (w.lo[j] != NULL_RUN && w.cnt[j]) {
+    if (w.lo[j] < (INL ? INLINE_RUN : NULL_RUN) && w.cnt[j]) {
       const uint32_t p = w.lo[j] + t.voff;
       if (chunks) {  // keys p .. p + min(cnt, 4) - 1 from the 8-byte chunks holding them
         const uint32_t last = (p + min(w.cnt[j], (uint32_t)PW_PREFETCH) - 1u) / 2u;
@@ -142,6 +145,7 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
       const int32_t v = o[j] == 0 ? x[e] : o[j] == 1 ? x[e + 1] : o[j] == 2 ? x[e + 2] : x[e + 3];
       kk[j][e] = (uint32_t)e < w.cnt[j] ? v : EJ_NULL_KEY;
     }
+    if (INL && w.lo[j] == INLINE_RUN) kk[j][0] = key[j];
   }
 }
 
@@ -174,9 +178,10 @@ __device__ __forceinline__ void ej_flush_stage(const int4* stage, uint32_t n, un
 }
 
 // a group with more rows than the buffer: 32 consecutive rows per round from out[a]
-__device__ __forceinline__ void ej_emit_big_group(uint32_t c, unsigned long long gsum, uint32_t lo, int32_t sk,
-                                                  int32_t sv, const ej_table_view& t, unsigned long long a,
-                                                  ej_result* __restrict__ out, uint64_t cap) {
+template <bool INL>
+__device__ __forceinline__ void ej_emit_big_group(uint32_t c, unsigned long long gsum, uint32_t lo, int32_t key0,
+                                                  int32_t sk, int32_t sv, const ej_table_view& t,
+                                                  unsigned long long a, ej_result* __restrict__ out, uint64_t cap) {
   const unsigned int lane = threadIdx.x & 31u;
   const unsigned long long pincl = ej_warp_inclusive_sum<unsigned long long>(c);
   const unsigned long long pre = pincl - c;  // group-relative first row of this lane
@@ -192,8 +197,10 @@ __device__ __forceinline__ void ej_emit_big_group(uint32_t c, unsigned long long
     const uint32_t rlo = __shfl_sync(EJ_FULL_MASK, lo, src);
     const int32_t rk = __shfl_sync(EJ_FULL_MASK, sk, src);
     const int32_t rs = __shfl_sync(EJ_FULL_MASK, sv, src);
+    const int32_t k0 = INL ? __shfl_sync(EJ_FULL_MASK, key0, src) : 0;
     if (o < gsum && a + o < cap) {
-      const int32_t key = rlo == NULL_RUN ? EJ_NULL_KEY : __ldg(t.rkey + rlo + e);
+      const int32_t key = rlo == NULL_RUN ? EJ_NULL_KEY
+                          : INL && rlo == INLINE_RUN ? k0 : __ldg(t.rkey + rlo + e);
       __stcs(reinterpret_cast<int4*>(out + a + o), make_int4(key, rlo == NULL_RUN ? EJ_NULL_KEY : rs, rk, rs));
     }
   }
@@ -202,6 +209,7 @@ __device__ __forceinline__ void ej_emit_big_group(uint32_t c, unsigned long long
 // The rows of a warp tile from out[off] on (rows at or past cap dropped):
 // group by group through the warp's buffer; kk: the prefetched keys of the
 // first rows of every run.
+template <bool INL = false>
 __device__ __forceinline__ void ej_emit_warp(const EjProbeWarp& w, const int32_t (&kk)[PR_ITEMS][PW_PREFETCH],
                                              const ej_table_view& t, unsigned long long a,
                                              ej_result* __restrict__ out, uint64_t cap, int4* stage) {
@@ -243,7 +251,7 @@ __device__ __forceinline__ void ej_emit_warp(const EjProbeWarp& w, const int32_t
       ej_flush_stage(stage, fill, a, out, cap);
       a += fill;
       fill = 0;
-      if (a < cap) ej_emit_big_group(w.cnt[j], gsum, w.lo[j], w.s[j].x, w.s[j].y, t, a, out, cap);
+      if (a < cap) ej_emit_big_group<INL>(w.cnt[j], gsum, w.lo[j], kk[j][0], w.s[j].x, w.s[j].y, t, a, out, cap);
       a += gsum;
     }
   }

@@ -124,9 +124,9 @@ typedef enum ej_option {
   EJ_OPT_PROBE_PARTITION_BITS = 0, /* radix bits of the one S partition pass, 0..8 (0 = probe
                                       in place); -1 (default) lets the planner choose */
   EJ_OPT_BUCKET_BITS_DELTA = 1,    /* hash-table buckets = 2^(ceil(log2|R|) - 2 + delta),
-                                      delta in -3..3; when neither this option nor the tuning
-                                      table sets it: 0 for single tables, 1 for the tables of
-                                      a batch */
+                                      delta in -3..3 (a hash table given one is hash-sorted);
+                                      when neither this option nor the tuning table sets it: 0
+                                      for single tables, 1 for the tables of a batch */
   EJ_OPT_WAIT_LIMIT_NS = 2,        /* bound of every device-side wait of this handle's kernels
                                       (look-back scans, the nested loop's copy waits), in ns,
                                       0..10^10; -1 restores the default of 10^9 (1 s).  A wait
@@ -144,8 +144,10 @@ typedef enum ej_option {
                                       threads per block (0: planner, 8) */
 } ej_option;
 
-/* Values of EJ_OPT_BUILD and ej_tune_entry.build.  The planner takes MSD for
- * hash tables of 2^20 rows and more, else LSD; sorted indexes sort by LSD
+/* Values of EJ_OPT_BUILD and ej_tune_entry.build.  The planner gives hash tables
+ * of at most 2^22 rows no sort (open addressing, one slot per key) unless
+ * a load factor or a key directory is chosen for them, and then takes MSD from
+ * 2^20 rows on, else LSD; larger ones MSD; sorted indexes sort by LSD
  * passes (their key is the value, whose top bits need not spread, so MSD does
  * not apply to them; EJ_BUILD_ONESWEEP applies to both kinds). */
 enum {
@@ -158,10 +160,11 @@ enum {
                             histogram pass for all four digits (tiles learn their offsets
                             by decoupled look-back) */
 };
-/* Values of EJ_OPT_TABLE and ej_tune_entry.table.  The planner gives tables
- * of 2^22 rows and more a key directory when their runs average two rows or
- * more (tables of 2^20 rows and more when probed by 16 rows per table row or
- * more), the others bucket bounds. */
+/* Values of EJ_OPT_TABLE and ej_tune_entry.table, for hash-sorted tables.  The
+ * planner gives those of more than 2^22 rows a key directory when their runs
+ * average two rows or more (or they are probed by 16 rows per table row or
+ * more), the others bucket bounds; smaller tables are not sorted (see above)
+ * unless EJ_OPT_BUILD or a load factor asks for it. */
 enum {
   EJ_TABLE_FORMAT_PLANNER = 0,
   EJ_TABLE_FORMAT_BUCKETS = 1,  /* bucket bounds: one 8-byte load, then a scan of the bucket */
