@@ -87,12 +87,14 @@ extern "C" ej_status ej_create(int device, ej_handle** out) {
   int l2 = 0;
   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
   h->l2_bytes = (size_t)l2;
-  bool ok = ej_dev_alloc(&h->d_status, sizeof(ej_dev_status)) == cudaSuccess &&
-            ej_dev_alloc(&h->d_words, 8 * sizeof(unsigned long long)) == cudaSuccess &&
-            ej_host_alloc(&h->h_words, 8 * sizeof(unsigned long long)) == cudaSuccess &&
-            ej_host_alloc(&h->h_status, sizeof(ej_dev_status)) == cudaSuccess;
-  if (ok) ok = cudaMemset(h->d_status, 0, sizeof(ej_dev_status)) == cudaSuccess &&
-               cudaMemset(h->d_words, 0, 8 * sizeof(unsigned long long)) == cudaSuccess;
+  bool ok = ej_dev_alloc(&h->d_block, sizeof(ej_dev_words)) == cudaSuccess &&
+            ej_host_alloc(&h->h_block, sizeof(ej_dev_words)) == cudaSuccess;
+  if (ok) {
+    h->d_status = &h->d_block->status;
+    h->d_words = h->d_block->words;
+    h->h_words = h->h_block->words;
+    ok = cudaMemset(h->d_block, 0, sizeof(ej_dev_words)) == cudaSuccess;
+  }
   if (!ok) {
     cudaGetLastError();
     ej_destroy(h);
@@ -109,11 +111,9 @@ extern "C" ej_status ej_destroy(ej_handle* h) {
   ej_stream_release(h);
   cudaFree(h->arena);
   cudaFree(h->stage);
-  cudaFree(h->d_status);
-  cudaFree(h->d_words);
+  cudaFree(h->d_block);
   cudaFree(h->zipf.d_cdf);
-  cudaFreeHost(h->h_words);
-  cudaFreeHost(h->h_status);
+  cudaFreeHost(h->h_block);
   cudaFree(h->d_batch_counts);
   cudaFreeHost(h->h_batch_counts);
   for (cudaEvent_t e : h->ring) cudaEventDestroy(e);
@@ -323,26 +323,32 @@ ej_status ej_begin(ej_handle* h) {
   return EJ_OK;
 }
 
+// Synchronise, with the device status and count word in the host mirror; a
+// status that was set is cleared (before anything later on the stream).
+static ej_status ej_read_status(ej_handle* h) {
+  EJ_CUDA(h, cudaMemcpyAsync(h->h_block, h->d_block, sizeof(ej_dev_status) + sizeof(unsigned long long),
+                             cudaMemcpyDeviceToHost, h->stream));
+  EJ_CUDA(h, cudaStreamSynchronize(h->stream));
+  if (h->h_block->status.code != 0)
+    EJ_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), h->stream));
+  return EJ_OK;
+}
+
 // Synchronise, fetch the device count word and status, clear the status.
 ej_status ej_finish(ej_handle* h, uint64_t* count) {
-  EJ_CUDA(h, cudaMemcpyAsync(h->h_words, h->d_words, sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-  EJ_CUDA(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(ej_dev_status), cudaMemcpyDeviceToHost, h->stream));
-  EJ_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), h->stream));
-  EJ_CUDA(h, cudaStreamSynchronize(h->stream));
+  EJ_TRY(ej_read_status(h));
   if (count) *count = h->h_words[0];
-  const unsigned int code = h->h_status->code;
+  const unsigned int code = h->h_block->status.code;
   if (code != 0 && code != EJ_ERR_CAPACITY)
     return ej_fail(h, (ej_status)code, "device reported %s (site %u)", ej_status_name((ej_status)code),
-                   h->h_status->info);
+                   h->h_block->status.info);
   return EJ_OK;
 }
 
 extern "C" ej_status ej_sync_status(ej_handle* h) {
   EJ_TRY(ej_begin(h));
-  EJ_CUDA(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(ej_dev_status), cudaMemcpyDeviceToHost, h->stream));
-  EJ_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), h->stream));
-  EJ_CUDA(h, cudaStreamSynchronize(h->stream));
-  return (ej_status)h->h_status->code;
+  EJ_TRY(ej_read_status(h));
+  return (ej_status)h->h_block->status.code;
 }
 
 // ---- argument checks --------------------------------------------------------

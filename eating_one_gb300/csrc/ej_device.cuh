@@ -46,6 +46,13 @@ __device__ __forceinline__ void ej_st_relaxed(unsigned long long* p, unsigned lo
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// The grid's threads clear n words (n at most the grid's threads): the scratch
+// of a scan that follows, which would otherwise take a memset of its own.
+__device__ __forceinline__ void ej_clear_words(unsigned long long* p, uint64_t n) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) p[i] = 0ull;
+}
+
 // Record the first device error (later errors keep the first one).
 __device__ __forceinline__ void ej_set_status(ej_dev_status* st, unsigned int code, unsigned int info) {
   if (st && atomicCAS(&st->code, 0u, code) == 0u) st->info = info;

@@ -22,6 +22,11 @@ struct ej_dev_status {
   unsigned long long aux;
 };
 
+struct ej_dev_words {
+  ej_dev_status status;
+  unsigned long long words[8];
+};
+
 // the table, partitioned probe side and run descriptors that a hash-join
 // count leaves for the write of the same join (hash_join.cu)
 struct ej_prepared_join;
@@ -41,11 +46,13 @@ struct ej_handle {
   void* arena = nullptr;
   size_t arena_cap = 0;
   size_t arena_peak = 0;
-  // small device words
-  ej_dev_status* d_status = nullptr;
-  unsigned long long* d_words = nullptr;  // [0] = join count, [1..7] scratch
-  unsigned long long* h_words = nullptr;  // pinned host mirror
-  ej_dev_status* h_status = nullptr;      // pinned host mirror of d_status
+  // small device words, one allocation: the status word and the join count lie
+  // together, so that a call reads both back with one copy
+  ej_dev_words* d_block = nullptr;
+  ej_dev_words* h_block = nullptr;        // pinned host mirror
+  ej_dev_status* d_status = nullptr;      // &d_block->status
+  unsigned long long* d_words = nullptr;  // d_block->words: [0] = join count, [1..7] scratch
+  unsigned long long* h_words = nullptr;  // h_block->words
   std::string last_error;
   // phase timing: a ring of EJ_PHASE_RING sets of EJ_PHASES+1 events
   bool timing = false;
@@ -166,11 +173,17 @@ static inline uint32_t ej_ceil_log2(uint64_t x) {
 // Exclusive scan of n inputs into n+1 outputs (out[n] = total).  `scratch`
 // must hold ej_scan_scratch_bytes(n) bytes of device memory.
 size_t ej_scan_scratch_bytes(uint64_t n);
-ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch);
+// the scratch words of a scan of n inputs; a caller whose own kernel before the
+// scan clears them (ej_clear_words, ej_device.cuh) passes cleared = true
+inline uint64_t ej_scan_words(uint64_t n) { return ej_scan_scratch_bytes(n) / sizeof(unsigned long long); }
+ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch,
+                          bool cleared = false);
 ej_status ej_scan_u32_u64(ej_handle* h, const uint32_t* in, uint64_t n, unsigned long long* out,
                           void* scratch);
+// total: also stored there when not null
 ej_status ej_scan_u64_u64(ej_handle* h, const unsigned long long* in, uint64_t n,
-                          unsigned long long* out, void* scratch);
+                          unsigned long long* out, void* scratch, bool cleared = false,
+                          unsigned long long* total = nullptr);
 
 // ---- radix partitioning (radix.cu) ---------------------------------------
 // Stable partition of tuples by digit = (key(val) >> shift) & ((1<<bits)-1),

@@ -244,7 +244,9 @@ slot_place_kernel(const int2* __restrict__ R, uint32_t n, const uint2* __restric
 template <bool OUTER, bool DESC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS)
 slot_count_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
-                          unsigned long long* __restrict__ wcount, uint64_t nwtiles, void* __restrict__ desc) {
+                  unsigned long long* __restrict__ wcount, uint64_t nwtiles, void* __restrict__ desc,
+                  unsigned long long* __restrict__ scan_scratch, uint64_t scan_words) {
+  ej_clear_words(scan_scratch, scan_words);  // of the scan that follows
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (w >= nwtiles) return;
   const unsigned long long total = ej_slot_count<OUTER, DESC>(P, w, nP, ej_slots_of(t), desc, nwtiles);
@@ -254,13 +256,16 @@ slot_count_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
 template <bool OUTER, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 slot_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc, uint64_t nP, ej_table_view t,
-                          const unsigned long long* __restrict__ woff, uint64_t nwtiles, ej_result* __restrict__ out,
-                          uint64_t cap, ej_dev_status* st) {
+                  const unsigned long long* __restrict__ woff, uint64_t nwtiles, ej_result* __restrict__ out,
+                  uint64_t cap, ej_dev_status* st, unsigned long long* total) {
   __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
   const unsigned int warp = threadIdx.x >> 5;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
   if (w >= nwtiles) return;
-  if (w == 0 && threadIdx.x == 0 && woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+  if (w == 0 && threadIdx.x == 0) {
+    if (woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (total) *total = woff[nwtiles];
+  }
   const unsigned long long off = woff[w];
   if (off >= cap) return;
   ej_slot_write<OUTER>(P, desc, w, nwtiles, nP, t, off, out, cap, stage[warp]);
@@ -271,8 +276,8 @@ slot_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc,
 template <bool OUTER, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 slot_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, uint64_t nwtiles,
-                    unsigned long long* __restrict__ cursor, ej_result* __restrict__ out, uint64_t cap,
-                    ej_dev_status* st) {
+                  unsigned long long* __restrict__ cursor, ej_result* __restrict__ out, uint64_t cap,
+                  ej_dev_status* st) {
   __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
   const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
@@ -311,7 +316,9 @@ __device__ __forceinline__ void ej_prefetch_tile(const void* base, uint64_t w, u
 template <int KIND, bool OUTER, int DESC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS)  // 40 warps per SM hide the table loads
 probe_count_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, unsigned long long* __restrict__ wcount,
-                   uint64_t nwtiles, void* __restrict__ desc, uint64_t ahead) {
+                   uint64_t nwtiles, void* __restrict__ desc, uint64_t ahead,
+                   unsigned long long* __restrict__ scan_scratch, uint64_t scan_words) {
+  ej_clear_words(scan_scratch, scan_words);  // of the scan that follows
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (w >= nwtiles) return;
   ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);  // the tile a warp one resident wave later takes
@@ -335,7 +342,8 @@ template <bool STORE>
 __global__ void __launch_bounds__(256, 4)
 probe_count_dir_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
                        unsigned long long* __restrict__ wcount, uint64_t nwtiles, uint32_t* __restrict__ desc,
-                       uint64_t ahead) {
+                       uint64_t ahead, unsigned long long* __restrict__ scan_scratch, uint64_t scan_words) {
+  ej_clear_words(scan_scratch, scan_words);  // of the scan that follows
   const unsigned lane = threadIdx.x & 31u;
   const uint64_t w0 = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * PCD_TILES;
   if (w0 >= nwtiles) return;
@@ -403,12 +411,15 @@ template <int KIND, bool OUTER, int DESC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 probe_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc, uint64_t nP, ej_table_view t,
                    const unsigned long long* __restrict__ woff, uint64_t nwtiles, ej_result* __restrict__ out,
-                   uint64_t cap, ej_dev_status* st, uint64_t ahead) {
+                   uint64_t cap, ej_dev_status* st, uint64_t ahead, unsigned long long* total) {
   __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
   const unsigned int warp = threadIdx.x >> 5;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
   if (w >= nwtiles) return;
-  if (w == 0 && threadIdx.x == 0 && woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+  if (w == 0 && threadIdx.x == 0) {
+    if (woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (total) *total = woff[nwtiles];
+  }
   ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);  // the tile a warp one resident wave later takes
   // the tile's descriptors: 1 KB (wide, lanes 8..15) or 512 bytes (packed, lanes 8..11)
   if (DESC == EJ_DESC_NONE) {
@@ -473,12 +484,16 @@ ej_status launch_count_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
   const uint64_t ahead = (uint64_t)h->num_sms * 40;  // warp tiles of one resident wave
   const dim3 grid((unsigned)pp.ntiles);
   constexpr int TH = WARPS * 32;
+  // the scratch of the scan after the count, cleared by it: two words and one
+  // per 4096 warp tiles, fewer than threads
+  unsigned long long* sw = reinterpret_cast<unsigned long long*>(ej_arena_at(h, pp.scan_off));
+  const uint64_t nsw = ej_scan_words(pp.nwtiles);
   if (KIND == EJ_TABLE_HASH && t.pair) {
     if (desc)
-      slot_count_kernel<OUTER, true, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, desc);
+      slot_count_kernel<OUTER, true, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, desc, sw, nsw);
     else
-      slot_count_kernel<OUTER, false, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles,
-                                                                                 nullptr);
+      slot_count_kernel<OUTER, false, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, nullptr, sw,
+                                                                         nsw);
     return ej_check_launch(h, "slot_count_kernel");
   }
   // inner probes of a packed key directory, 16-byte aligned: the lean count
@@ -489,21 +504,22 @@ ej_status launch_count_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
     const uint64_t ahead2 = (uint64_t)h->num_sms * 4 * 8 * PCD_TILES;  // warp tiles of one resident wave
     if (desc)
       probe_count_dir_kernel<true><<<(unsigned)blocks, 256, 0, h->stream>>>(
-          P, pp.nP, t, wcount, pp.nwtiles, static_cast<uint32_t*>(desc), ahead2);
+          P, pp.nP, t, wcount, pp.nwtiles, static_cast<uint32_t*>(desc), ahead2, sw, nsw);
     else
       probe_count_dir_kernel<false><<<(unsigned)blocks, 256, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles,
-                                                                              nullptr, ahead2);
+                                                                              nullptr, ahead2, sw, nsw);
     return ej_check_launch(h, "probe_count_dir_kernel");
   }
   if (!desc || desc_form(t) == EJ_DESC_NONE)
     probe_count_kernel<KIND, OUTER, EJ_DESC_NONE, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles,
-                                                                                     nullptr, ahead);
+                                                                                     nullptr, ahead, sw, nsw);
   else if (desc_form(t) == EJ_DESC_PACKED)
     probe_count_kernel<KIND, OUTER, EJ_DESC_PACKED, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount,
-                                                                                       pp.nwtiles, desc, ahead);
+                                                                                       pp.nwtiles, desc, ahead, sw,
+                                                                                       nsw);
   else
     probe_count_kernel<KIND, OUTER, EJ_DESC_WIDE, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles,
-                                                                                     desc, ahead);
+                                                                                     desc, ahead, sw, nsw);
   return ej_check_launch(h, "probe_count_kernel");
 }
 
@@ -516,32 +532,34 @@ ej_status launch_count(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* 
 
 template <int KIND, bool OUTER, int WARPS>
 ej_status launch_write_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
-                         const void* desc, const unsigned long long* woff, ej_result* out, uint64_t cap) {
+                         const void* desc, const unsigned long long* woff, ej_result* out, uint64_t cap,
+                         unsigned long long* total) {
   const uint64_t ahead = (uint64_t)h->num_sms * 32;  // warp tiles of one resident wave
   const dim3 grid((unsigned)pp.ntiles);
   constexpr int TH = WARPS * 32;
   if (KIND == EJ_TABLE_HASH && t.pair) {
     slot_write_kernel<OUTER, WARPS><<<grid, TH, 0, h->stream>>>(P, desc, pp.nP, t, woff, pp.nwtiles, out, cap,
-                                                                        h->d_status);
+                                                                        h->d_status, total);
     return ej_check_launch(h, "slot_write_kernel");
   }
   if (desc_form(t) == EJ_DESC_NONE)
     probe_write_kernel<KIND, OUTER, EJ_DESC_NONE, WARPS><<<grid, TH, 0, h->stream>>>(
-        P, nullptr, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead);
+        P, nullptr, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead, total);
   else if (desc_form(t) == EJ_DESC_PACKED)
     probe_write_kernel<KIND, OUTER, EJ_DESC_PACKED, WARPS><<<grid, TH, 0, h->stream>>>(
-        P, desc, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead);
+        P, desc, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead, total);
   else
     probe_write_kernel<KIND, OUTER, EJ_DESC_WIDE, WARPS><<<grid, TH, 0, h->stream>>>(
-        P, desc, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead);
+        P, desc, pp.nP, t, woff, pp.nwtiles, out, cap, h->d_status, ahead, total);
   return ej_check_launch(h, "probe_write_kernel");
 }
 
 template <int KIND, bool OUTER>
 ej_status launch_write(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
-                       const void* desc, const unsigned long long* woff, ej_result* out, uint64_t cap) {
-  return pp.warps == 4 ? launch_write_w<KIND, OUTER, 4>(h, pp, P, t, desc, woff, out, cap)
-                       : launch_write_w<KIND, OUTER, 8>(h, pp, P, t, desc, woff, out, cap);
+                       const void* desc, const unsigned long long* woff, ej_result* out, uint64_t cap,
+                       unsigned long long* total) {
+  return pp.warps == 4 ? launch_write_w<KIND, OUTER, 4>(h, pp, P, t, desc, woff, out, cap, total)
+                       : launch_write_w<KIND, OUTER, 8>(h, pp, P, t, desc, woff, out, cap, total);
 }
 
 }  // namespace
@@ -567,8 +585,7 @@ bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {
   return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table != EJ_TABLE_FORMAT_DIRECTORY;
 }
 
-// the runs of a slot table: every row, and a count for each of 31 rows and more
-static size_t ej_slot_run_bytes(uint64_t nR) { return ej_table_col_bytes(nR + nR / 31 + 1); }
+size_t ej_slot_run_bytes(uint64_t nR) { return ej_table_col_bytes(nR + nR / 31 + 1); }
 
 size_t ej_table_aux_bytes(const ej_table_plan_t& tp) {
   if (tp.slots) return EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4) + ej_slot_run_bytes(tp.nR);
@@ -780,24 +797,23 @@ ej_status ej_probe_count(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
       EJ_TRY(outer ? launch_count<EJ_TABLE_SORTED, true>(h, pp, P, t, wcount, desc)
                    : launch_count<EJ_TABLE_SORTED, false>(h, pp, P, t, wcount, desc));
   }
-  EJ_TRY(ej_scan_u64_u64(h, wcount, pp.nwtiles, woff, ej_arena_at(h, pp.scan_off)));
-  if (d_count)
-    EJ_CUDA(h, cudaMemcpyAsync(d_count, woff + pp.nwtiles, sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
-                               h->stream));
-  return EJ_OK;
+  return ej_scan_u64_u64(h, wcount, pp.nwtiles, woff, ej_arena_at(h, pp.scan_off), /*cleared=*/true, d_count);
 }
 
 ej_status ej_probe_write(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
-                         ej_result* out, uint64_t cap, bool outer) {
-  if (!pp.ntiles) return EJ_OK;
+                         ej_result* out, uint64_t cap, bool outer, unsigned long long* total) {
+  if (!pp.ntiles) {
+    if (total) EJ_CUDA(h, cudaMemsetAsync(total, 0, sizeof(unsigned long long), h->stream));
+    return EJ_OK;
+  }
   if (!pp.with_desc) return ej_fail(h, EJ_ERR_INTERNAL, "probe write planned without run descriptors");
   const void* desc = ej_arena_at(h, pp.desc_off);
   const unsigned long long* woff = reinterpret_cast<const unsigned long long*>(ej_arena_at(h, pp.off_off));
   if (t.kind == EJ_TABLE_HASH)
-    return outer ? launch_write<EJ_TABLE_HASH, true>(h, pp, P, t, desc, woff, out, cap)
-                 : launch_write<EJ_TABLE_HASH, false>(h, pp, P, t, desc, woff, out, cap);
-  return outer ? launch_write<EJ_TABLE_SORTED, true>(h, pp, P, t, desc, woff, out, cap)
-               : launch_write<EJ_TABLE_SORTED, false>(h, pp, P, t, desc, woff, out, cap);
+    return outer ? launch_write<EJ_TABLE_HASH, true>(h, pp, P, t, desc, woff, out, cap, total)
+                 : launch_write<EJ_TABLE_HASH, false>(h, pp, P, t, desc, woff, out, cap, total);
+  return outer ? launch_write<EJ_TABLE_SORTED, true>(h, pp, P, t, desc, woff, out, cap, total)
+               : launch_write<EJ_TABLE_SORTED, false>(h, pp, P, t, desc, woff, out, cap, total);
 }
 
 // ---- partition bits for the probe side ------------------------------------
@@ -907,11 +923,7 @@ static ej_status hash_join_write_kept(ej_handle* h, ej_result* out, uint64_t out
   const ej_prepared_join& pj = *h->prep;
   ej_phase_begin(h);
   for (int k = 1; k <= 3; k++) ej_phase_mark(h, k);  // build, partition and count were the count's
-  EJ_TRY(ej_probe_write(h, pj.L.pp, pj.P, pj.t, out, out_cap));
-  const unsigned long long* woff = reinterpret_cast<const unsigned long long*>(ej_arena_at(h, pj.L.pp.off_off));
-  if (d_count)
-    EJ_CUDA(h, cudaMemcpyAsync(d_count, woff + pj.L.pp.nwtiles, sizeof(unsigned long long),
-                               cudaMemcpyDeviceToDevice, h->stream));
+  EJ_TRY(ej_probe_write(h, pj.L.pp, pj.P, pj.t, out, out_cap, /*outer=*/false, d_count));
   ej_phase_mark(h, 4);
   // kept for another write only when this one was cut short by the capacity
   h->prep_valid = pj.count_known && out_cap < pj.count;

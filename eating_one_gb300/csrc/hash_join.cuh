@@ -78,6 +78,8 @@ struct ej_table_knobs {
   int table = EJ_TABLE_FORMAT_PLANNER;
 };
 ej_table_knobs ej_tuned_table_knobs(const ej_handle* h, uint64_t nR);
+// bytes of a slot table's runs: every row, and a count for each of 31 rows and more
+size_t ej_slot_run_bytes(uint64_t nR);
 // whether a hash table of nR rows is a slot table
 bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k);
 // n_probe: the probe rows the caller expects (0: unknown)
@@ -92,9 +94,10 @@ void ej_probe_plan(ej_plan_bytes& p, ej_probe_plan_t& pp, uint64_t nP, bool with
 ej_status ej_probe_count(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
                          bool outer, unsigned long long* d_count);
 // write pass from the run descriptors and offsets of ej_probe_count (same
-// plan, same inputs, same outer flag)
+// plan, same inputs, same outer flag); the total also to the device word
+// *total when not null
 ej_status ej_probe_write(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
-                         ej_result* out, uint64_t cap, bool outer = false);
+                         ej_result* out, uint64_t cap, bool outer = false, unsigned long long* total = nullptr);
 
 uint32_t ej_probe_partition_bits(const ej_handle* h, uint64_t nR, uint64_t nS);
 // two_pass: plan the run descriptors of ej_probe_count + ej_probe_write (for

@@ -66,7 +66,9 @@ __device__ __forceinline__ RxTile rx_tile(const ej_tuple* in, const ej_rx_tile* 
 template <int KIND, bool SRC = false>
 __global__ void __launch_bounds__(RX_THREADS)
 rx_hist_kernel(const ej_tuple* __restrict__ in, uint64_t n, const ej_rx_tile* __restrict__ tiles,
-               uint32_t* __restrict__ hist, uint32_t ntiles, uint32_t shift, uint32_t mask) {
+               uint32_t* __restrict__ hist, uint32_t ntiles, uint32_t shift, uint32_t mask,
+               unsigned long long* __restrict__ scan_scratch, uint64_t scan_words) {
+  ej_clear_words(scan_scratch, scan_words);  // of the scan that follows
   __shared__ uint32_t cnt[RX_WARPS][RX_MAX_DIGITS];
   const uint32_t ndig = mask + 1u;
   for (int i = threadIdx.x; i < RX_WARPS * RX_MAX_DIGITS; i += RX_THREADS) (&cnt[0][0])[i] = 0u;
@@ -237,10 +239,12 @@ static ej_status radix_pass_kind(ej_handle* h, const ej_radix_plan& rp, const ej
   uint32_t* hist = reinterpret_cast<uint32_t*>(ej_arena_at(h, rp.hist_off));
   uint32_t* offs = reinterpret_cast<uint32_t*>(ej_arena_at(h, rp.offs_off));
   if (rp.tiles && bits != 8) return ej_fail(h, EJ_ERR_INTERNAL, "segmented radix passes use 8-bit digits");
-  rx_hist_kernel<KIND, SRC><<<rp.ntiles, RX_THREADS, 0, h->stream>>>(in, rp.n, rp.tiles, hist, rp.ntiles, shift,
-                                                                     mask);
+  // one scan word per 4096 cells, at most 16 tiles' worth each: fewer than threads
+  rx_hist_kernel<KIND, SRC><<<rp.ntiles, RX_THREADS, 0, h->stream>>>(
+      in, rp.n, rp.tiles, hist, rp.ntiles, shift, mask,
+      reinterpret_cast<unsigned long long*>(ej_arena_at(h, rp.scan_off)), ej_scan_words(cells));
   EJ_TRY(ej_check_launch(h, "rx_hist_kernel"));
-  EJ_TRY(ej_scan_u32_u32(h, hist, cells, offs, ej_arena_at(h, rp.scan_off)));
+  EJ_TRY(ej_scan_u32_u32(h, hist, cells, offs, ej_arena_at(h, rp.scan_off), /*cleared=*/true));
   EJ_CUDA(h, cudaFuncSetAttribute(rx_scatter_kernel<KIND, SOA, STABLE, SRC>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RxScatterSmem)));
   rx_scatter_kernel<KIND, SOA, STABLE, SRC><<<rp.ntiles, RX_THREADS, sizeof(RxScatterSmem), h->stream>>>(

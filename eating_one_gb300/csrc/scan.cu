@@ -19,7 +19,7 @@ constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 template <typename In, typename Out>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_kernel(const In* __restrict__ in, uint64_t n, Out* __restrict__ out, unsigned long long* status,
-            unsigned int* tile_ctr, uint64_t ntiles, ej_dev_status* st, unsigned long long wait_ns) {
+            unsigned int* tile_ctr, uint64_t ntiles, ej_dev_status* st, unsigned long long wait_ns, Out* total) {
   __shared__ Out sbuf[SCAN_TILE + SCAN_TILE / 32];
   __shared__ Out warp_tmp[SCAN_THREADS / 32 + 1];
   __shared__ unsigned int s_tile;
@@ -70,22 +70,27 @@ scan_kernel(const In* __restrict__ in, uint64_t n, Out* __restrict__ out, unsign
     const uint64_t idx = base + (uint64_t)s;
     if (idx < n) out[idx] = sbuf[s + (s >> 5)];
   }
-  if (tile == ntiles - 1 && threadIdx.x == 0) out[n] = s_prefix + aggregate;
+  if (tile == ntiles - 1 && threadIdx.x == 0) {
+    out[n] = s_prefix + aggregate;
+    if (total) *total = s_prefix + aggregate;
+  }
 }
 
 template <typename In, typename Out>
-ej_status launch_scan(ej_handle* h, const In* in, uint64_t n, Out* out, void* scratch) {
+ej_status launch_scan(ej_handle* h, const In* in, uint64_t n, Out* out, void* scratch, bool cleared = false,
+                      Out* total = nullptr) {
   if (n == 0) {
     EJ_CUDA(h, cudaMemsetAsync(out, 0, sizeof(Out), h->stream));
+    if (total) EJ_CUDA(h, cudaMemsetAsync(total, 0, sizeof(Out), h->stream));
     return EJ_OK;
   }
   const uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (ntiles > 0xFFFFFFFFull) return ej_fail(h, EJ_ERR_TOO_LARGE, "scan: %llu elements", (unsigned long long)n);
   unsigned long long* status = static_cast<unsigned long long*>(scratch);
   unsigned int* ctr = reinterpret_cast<unsigned int*>(status + ntiles);
-  EJ_CUDA(h, cudaMemsetAsync(scratch, 0, ntiles * sizeof(unsigned long long) + 16, h->stream));
+  if (!cleared) EJ_CUDA(h, cudaMemsetAsync(scratch, 0, ntiles * sizeof(unsigned long long) + 16, h->stream));
   scan_kernel<In, Out><<<(unsigned)ntiles, SCAN_THREADS, 0, h->stream>>>(in, n, out, status, ctr, ntiles,
-                                                                         h->d_status, h->wait_limit_ns);
+                                                                         h->d_status, h->wait_limit_ns, total);
   return ej_check_launch(h, "scan_kernel");
 }
 
@@ -96,8 +101,8 @@ size_t ej_scan_scratch_bytes(uint64_t n) {
   return (size_t)(ntiles * sizeof(unsigned long long) + 16);
 }
 
-ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch) {
-  return launch_scan<uint32_t, uint32_t>(h, in, n, out, scratch);
+ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch, bool cleared) {
+  return launch_scan<uint32_t, uint32_t>(h, in, n, out, scratch, cleared);
 }
 
 ej_status ej_scan_u32_u64(ej_handle* h, const uint32_t* in, uint64_t n, unsigned long long* out,
@@ -106,8 +111,8 @@ ej_status ej_scan_u32_u64(ej_handle* h, const uint32_t* in, uint64_t n, unsigned
 }
 
 ej_status ej_scan_u64_u64(ej_handle* h, const unsigned long long* in, uint64_t n,
-                          unsigned long long* out, void* scratch) {
-  return launch_scan<unsigned long long, unsigned long long>(h, in, n, out, scratch);
+                          unsigned long long* out, void* scratch, bool cleared, unsigned long long* total) {
+  return launch_scan<unsigned long long, unsigned long long>(h, in, n, out, scratch, cleared, total);
 }
 
 // ---- scan without allocation ------------------------------------------------
@@ -185,7 +190,7 @@ extern "C" ej_status ej_exclusive_scan_u32_noalloc(const uint32_t* in, uint64_t 
   }
   unsigned int* ctr = reinterpret_cast<unsigned int*>(d.scratch + ntiles);
   scan_kernel<uint32_t, unsigned long long><<<(unsigned)ntiles, SCAN_THREADS, 0, s>>>(
-      in, n, o, d.scratch, ctr, ntiles, d.status, EJ_DEFAULT_WAIT_LIMIT_NS);
+      in, n, o, d.scratch, ctr, ntiles, d.status, EJ_DEFAULT_WAIT_LIMIT_NS, nullptr);
   if (cudaGetLastError() != cudaSuccess) return EJ_ERR_CUDA;
   ej_dev_status host_status;
   if (cudaMemcpyAsync(&host_status, d.status, sizeof(host_status), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
