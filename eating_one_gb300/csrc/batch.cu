@@ -5,31 +5,39 @@
 // For a stream of joins of uneven sizes (most of them small) that is launch-
 // and latency-bound.  Here a batch of joins is one fixed sequence of launches,
 // whatever the number of joins in it:
-//   build       four segmented LSD radix passes over the joins that are not
-//               small: tiles never cross a join and
-//               the digit histograms are laid out join by join, so one scan
-//               places every join's rows in its own range, hash-sorted (the
-//               first pass reads every join's R where it lies)
-//   starts      every join's bucket starts in one launch (its own bucket bits;
-//               a batch's tables are small enough for L2, where the bucket
-//               scan is as fast as a key directory and one launch builds it)
+//   build       every join that is not small gets a slot table (slot_table.cuh)
+//               in its own part of the scratch: one launch over all joins' R
+//               tiles claims the slots, two more finish keys with several rows
+//               (and exit at once when no join has any)
 //   probe       one launch over a task list, a task per block: whole small
 //               joins (R of at most 2048 rows: table built and probed in
 //               shared memory by one CTA, no radix pass) and the probe tiles
 //               of the others (each warp finds its runs, reserves its rows
 //               with one atomic add on its join's count and writes them, as
 //               the one-pass probe of single joins does).
+// Joins of more than 2^26 R rows, past a slot's 27-bit run starts, run as single
+// joins after the batch's launches, on the same stream.
 // Every join's rows are the rows it gives alone; their order within the join
 // is not specified (warps reserve their ranges in the order they arrive).
+#include <string.h>
+
+#include <algorithm>
+
 #include "ej_device.cuh"
 #include "ej_entry.h"
 #include "hash_join.cuh"
-#include "probe_write.cuh"
+#include "slot_table.cuh"
 
 namespace {
 
-constexpr uint32_t BX_RX_TILE = EJ_RX_TILE;
-static_assert(BX_RX_TILE % 256 == 0, "bucket bounds take 256-row warp spans that must not cross an R tile");
+constexpr int BX_ITEMS = 4;                              // R rows per thread and tile
+constexpr uint32_t BX_RTILE = 256 * BX_ITEMS;            // R rows per build tile
+constexpr uint64_t BX_MAX_R = 1ull << 26;                // larger joins run as single joins
+
+// {runs' cursor of the join's table, ...}: cleared with the slots
+struct BatchTableHeader {
+  uint32_t cursor, pad;
+};
 
 // per join, on the device
 struct BatchJoin {
@@ -40,59 +48,119 @@ struct BatchJoin {
   unsigned long long* d_count;  // the join's row cursor, then its count
   unsigned long long nS;
   unsigned long long nwtiles;  // warp tiles of the join
-  unsigned long long r_row0;   // first row of the join in the concatenated R
+  unsigned long long r_row0;   // first row of the join in the marks and ranks
   const ej_tuple* R;
+  unsigned long long* slot;    // the join's slots (view.pair)
+  int32_t* runs;               // and their runs (view.rkey)
 };
 
-// a task of the batch's task list: one probe tile of a join (local = the
-// tile), or a whole small join (local = BX_SMALL_TASK)
+// a build tile: rows [row0, row0 + BX_RTILE) of a join's R
+struct BatchTile {
+  uint32_t join, row0;
+};
+
+// a task of the batch's task list: BX_TASK_TILES consecutive probe tiles of a
+// join (the first of them local), or a whole small join (local = BX_SMALL_TASK)
 struct BatchTask {
   uint32_t join, local;
 };
+// 4096 probes: a task per 1024 made the list, planned and copied up per call,
+// four times as long (52000 tasks for 32 joins of 53 M probes)
+constexpr uint32_t BX_TASK_TILES = 4;
 constexpr uint32_t BX_SMALL_TASK = 0xFFFFFFFFu;
 // joins of at most this many R rows are built and probed in shared memory
 constexpr uint32_t BX_SMALL_R = 2048;
-// the planner's load of a batch's bucket bounds, about 2 rows a bucket (its
-// probe, bound by the latency of its loads, finds empty buckets without the
-// scan; the served stream's 256-instance batch 12.3 -> 11.9 ms against 4
-// rows a bucket, 12.3 ms at 1): explicit options and the tuning table first
-constexpr int BX_BUCKET_DELTA = 1;
 
-// bucket bounds of every join: the block of one R tile fills the gaps
-// between the buckets of consecutive rows of its join; the join's last row
-// also fills the tail up to 2^hb
-__global__ void batch_bucket_start_kernel(const ej_rx_tile* __restrict__ tiles, const BatchJoin* __restrict__ joins,
-                                          uint2* __restrict__ bucket_all, const unsigned long long* bucket_base) {
-  const ej_rx_tile d = tiles[blockIdx.x];
-  const BatchJoin& j = joins[d.pad];
-  const ej_table_view& t = j.view;
-  uint2* bucket = bucket_all + bucket_base[d.pad];
-  const uint64_t first = d.start - j.r_row0;  // local row index of the tile's first row
-  // the join's last tile also takes the end row (local row nR)
-  const uint64_t end = first + d.n + (first + d.n == t.nR ? 1u : 0u);
-  // tiles are multiples of 256 rows except a join's last, so a warp's 256
-  // rows never reach into the next tile
-  for (uint64_t r0 = first + (threadIdx.x >> 5) * 256; r0 < end; r0 += (blockDim.x >> 5) * 256)
-    ej_bucket_bounds_warp(t.rval, t.nR, r0, t.hb, bucket, EjHashBucketOf{t.hb});
+// ---- build: slot_table.cuh's steps over the tiles of all joins ---------------------
+
+__global__ void __launch_bounds__(256)
+batch_insert_kernel(const BatchTile* __restrict__ tiles, const BatchJoin* __restrict__ joins,
+                    uint32_t* __restrict__ mark, uint2* __restrict__ rank, uint32_t* __restrict__ marked) {
+  const BatchTile d = tiles[blockIdx.x];
+  const BatchJoin& j = joins[d.join];
+  const int2* R = reinterpret_cast<const int2*>(j.R);
+  const uint32_t n = (uint32_t)j.view.nR, lane = threadIdx.x & 31u;
+  const uint32_t base = d.row0 + (threadIdx.x >> 5) * (32 * BX_ITEMS) + lane;
+  int32_t key[BX_ITEMS];
+  uint32_t hv[BX_ITEMS], any = 0;
+  EjSlotMark m[BX_ITEMS];
+  bool ok[BX_ITEMS];
+#pragma unroll
+  for (int q = 0; q < BX_ITEMS; q++) {
+    ok[q] = base + 32u * q < n;
+    const int2 r = ok[q] ? __ldg(R + base + 32u * q) : make_int2(0, 0);
+    key[q] = r.x;
+    hv[q] = ej_hash32((uint32_t)r.y);
+  }
+  ej_slot_insert<BX_ITEMS>(j.slot, j.view.npairs, key, hv, ok, m);
+#pragma unroll
+  for (int q = 0; q < BX_ITEMS; q++) {
+    if (ok[q]) mark[j.r_row0 + base + 32u * q] = m[q].mark;
+    if (m[q].mark) rank[j.r_row0 + base + 32u * q] = make_uint2(m[q].rank, (uint32_t)m[q].first);
+    any |= m[q].mark;
+  }
+  if (__any_sync(EJ_FULL_MASK, any != 0u) && lane == 0u) *marked = 1u;
 }
 
-// one probe tile of a join whose table the segmented passes built: each warp
-// reserves its rows on its join's cursor (d_count, zeroed before the launch),
-// so the cursor ends at the join's count
+// the passes over the marked rows: a few blocks per SM stride over the tiles
+__global__ void __launch_bounds__(256)
+batch_reserve_kernel(const BatchTile* __restrict__ tiles, uint32_t ntiles, const BatchJoin* __restrict__ joins,
+                     const uint32_t* __restrict__ mark, const uint2* __restrict__ rank,
+                     BatchTableHeader* __restrict__ hdr, const uint32_t* __restrict__ marked) {
+  if (__ldg(marked) == 0u) return;
+  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BatchTile d = tiles[t];
+    const BatchJoin& j = joins[d.join];
+    const uint32_t base = d.row0 + (threadIdx.x >> 5) * (32 * BX_ITEMS) + (threadIdx.x & 31u);
+    uint32_t m[BX_ITEMS];
+    uint2 r[BX_ITEMS];
+#pragma unroll
+    for (int q = 0; q < BX_ITEMS; q++)
+      m[q] = base + 32u * q < j.view.nR ? __ldg(mark + j.r_row0 + base + 32u * q) : 0u;
+#pragma unroll
+    for (int q = 0; q < BX_ITEMS; q++)
+      r[q] = m[q] ? __ldg(rank + j.r_row0 + base + 32u * q) : make_uint2(0u, 0u);
+    ej_slot_reserve<BX_ITEMS>(reinterpret_cast<uint2*>(j.slot), m, r, j.runs, &hdr[d.join].cursor);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+batch_place_kernel(const BatchTile* __restrict__ tiles, uint32_t ntiles, const BatchJoin* __restrict__ joins,
+                   const uint32_t* __restrict__ mark, const uint2* __restrict__ rank,
+                   const uint32_t* __restrict__ marked) {
+  if (__ldg(marked) == 0u) return;
+  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const BatchTile d = tiles[t];
+    const BatchJoin& j = joins[d.join];
+    for (uint32_t i = d.row0 + threadIdx.x; i < min(d.row0 + BX_RTILE, (uint32_t)j.view.nR); i += 256) {
+      const uint32_t m = __ldg(mark + j.r_row0 + i);
+      if (m)
+        j.runs[(reinterpret_cast<const uint2*>(j.slot)[m - 1u].x >> 5) +
+               (__ldg(&rank[j.r_row0 + i].x) & ~EJ_SLOT_OPENER)] = j.R[i].key;
+    }
+  }
+}
+
+// one probe tile of a join with a slot table: each warp reserves its rows on its
+// join's cursor (d_count, zeroed before the launch), so the cursor ends at the
+// join's count
 __device__ __forceinline__ void batch_probe_tile(const BatchJoin& j, uint32_t local, int4 (*stage)[PW_STAGE_ROWS],
                                                  ej_dev_status* st) {
   const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint64_t w = (uint64_t)local * PR_WARPS + warp;
   if (w >= j.nwtiles) return;
+  {  // the next tile of the warp, 1 KB, lanes 0..7
+    const uint64_t off = (w + PR_WARPS) * (PR_WTILE * 8) + (uint64_t)lane * 128u;
+    if (lane < 8u && off < j.nS * 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(j.S) + off));
+  }
   EjProbeWarp pw;
-  ej_probe_runs_warp<EJ_TABLE_HASH, false>(j.S, w * PR_WTILE, j.nS, j.view, pw);
+  int32_t key[PR_ITEMS];
+  ej_slot_probe<false>(j.S, w * PR_WTILE, j.nS, ej_slots_of(j.view), pw, key);
   unsigned long long mine = 0;
 #pragma unroll
   for (int q = 0; q < PR_ITEMS; q++) mine += pw.cnt[q];
   const unsigned long long total = ej_warp_sum<unsigned long long>(mine);
   if (total == 0) return;
-  int32_t kk[PR_ITEMS][PW_PREFETCH];
-  ej_probe_prefetch<EJ_KEYS_CHUNKS>(j.view, pw, kk);
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(j.d_count, total);
@@ -100,7 +168,7 @@ __device__ __forceinline__ void batch_probe_tile(const BatchJoin& j, uint32_t lo
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= j.cap) return;
-  ej_emit_warp(pw, kk, j.view, off, j.out, j.cap, stage[warp]);
+  ej_slot_emit(pw, key, j.view, off, j.out, j.cap, stage[warp]);
 }
 
 // A join small enough for shared memory (nR <= BX_SMALL_R), whole, by one
@@ -159,11 +227,10 @@ __device__ __forceinline__ void batch_small_join(const BatchJoin& j, int4* smem,
 // built and probed in shared memory) or one 1024-probe tile of a larger join
 // (table from the segmented passes).  The small joins come first, so that no
 // large task waits behind them at the end.  (A resident grid pulling tasks
-// from an atomic counter measured slower: its loop needs 80 registers a
-// thread, three blocks per SM instead of four.)
-// (Four blocks per SM: 64 registers a thread; left free it takes 78, three
-// blocks, and the 256-instance batch ran 1% slower; at five blocks the
-// spills cost 20%.)
+// from an atomic counter measured slower.)  32 served requests of 13.3 M
+// R rows in all: four segmented radix passes, bucket bounds and this kernel over
+// them 0.46 + 0.05 + 0.73 ms, slots and this kernel 0.42 + 0.55; the call 1.57 ->
+// 1.25 ms.
 __global__ void __launch_bounds__(PR_THREADS, 4)
 batch_task_kernel(const BatchJoin* __restrict__ joins, const BatchTask* __restrict__ tasks, ej_dev_status* st) {
   __shared__ int4 smem[PR_WARPS * PW_STAGE_ROWS];  // staging rows, or a small join's table
@@ -174,7 +241,8 @@ batch_task_kernel(const BatchJoin* __restrict__ joins, const BatchTask* __restri
   if (task.local == BX_SMALL_TASK)
     batch_small_join(j, smem, st);
   else
-    batch_probe_tile(j, task.local, reinterpret_cast<int4(*)[PW_STAGE_ROWS]>(smem), st);
+    for (uint32_t k = 0; k < BX_TASK_TILES; k++)
+      batch_probe_tile(j, task.local + k, reinterpret_cast<int4(*)[PW_STAGE_ROWS]>(smem), st);
 }
 
 }  // namespace
@@ -183,10 +251,11 @@ batch_task_kernel(const BatchJoin* __restrict__ joins, const BatchTask* __restri
 static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, unsigned long long* d_counts) {
   // host-side layout of the batch
   std::vector<BatchJoin> joins(n);
-  std::vector<ej_rx_tile> rtiles;
+  std::vector<BatchTile> tiles;
   std::vector<BatchTask> small_tasks, tile_tasks;
-  std::vector<unsigned long long> sbase(n);
-  uint64_t nr_total = 0, start_total = 0, cells = 0;
+  std::vector<uint64_t> pair0(n), run0(n);
+  std::vector<uint32_t> large;
+  uint64_t nr_total = 0, pairs = 0, run_words = 0;
   for (uint32_t i = 0; i < n; i++) {
     const uint64_t nR = jd[i].nR, nS = jd[i].nS;
     BatchJoin& b = joins[i];
@@ -199,111 +268,91 @@ static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, uns
     b.r_row0 = nr_total;
     b.view.kind = EJ_TABLE_HASH;
     b.view.nR = nR;
-    b.view.hb = ej_table_bucket_bits(nR, ej_tuned_bucket_delta(h, nR, BX_BUCKET_DELTA));
     b.nwtiles = (nS + PR_WTILE - 1) / PR_WTILE;
-    sbase[i] = start_total;
+    pair0[i] = pairs;
+    run0[i] = run_words;
+    if (nR > BX_MAX_R) {
+      large.push_back(i);
+      continue;
+    }
     if (nR && nR <= BX_SMALL_R) {  // built and probed by one CTA in shared memory
       if (nS) small_tasks.push_back({i, BX_SMALL_TASK});
       continue;
     }
-    const uint32_t rt = (uint32_t)((nR + BX_RX_TILE - 1) / BX_RX_TILE);
-    for (uint32_t t = 0; t < rt; t++) {
-      ej_rx_tile d;
-      d.start = nr_total + (uint64_t)t * BX_RX_TILE;
-      d.n = (uint32_t)std::min<uint64_t>(BX_RX_TILE, nR - (uint64_t)t * BX_RX_TILE);
-      d.cell0 = (uint32_t)(cells + t);
-      d.stride = rt;
-      d.pad = i;
-      d.src = nullptr;
-      rtiles.push_back(d);
-    }
-    cells += (uint64_t)rt * 256;
-    start_total += 1ull << b.view.hb;
+    b.view.npairs = (uint32_t)nR + 1u;  // at most half full
+    pairs += b.view.npairs;
+    run_words += (ej_slot_run_bytes(nR) / sizeof(int32_t) + 3) & ~uint64_t(3);
+    for (uint64_t r = 0; r < nR; r += BX_RTILE) tiles.push_back({i, (uint32_t)r});
     const uint32_t nptiles = (uint32_t)((nS + PR_TILE - 1) / PR_TILE);
-    for (uint32_t t = 0; t < nptiles; t++) tile_tasks.push_back({i, t});
+    for (uint32_t t = 0; t < nptiles && nR; t += BX_TASK_TILES) tile_tasks.push_back({i, t});
     nr_total += nR;
   }
-  // the task list: small joins first, then every probe tile
-  std::vector<BatchTask> tasks(small_tasks);
-  tasks.insert(tasks.end(), tile_tasks.begin(), tile_tasks.end());
-  if (cells > 0xFFFFFFFFull || nr_total >= 0xFFFFFFFFull)
+  if (tiles.size() > 0x7FFFFFFFull || tile_tasks.size() + small_tasks.size() > 0x7FFFFFFFull)
     return ej_fail(h, EJ_ERR_TOO_LARGE, "batch of %llu R rows is too large", (unsigned long long)nr_total);
 
-  // arena layout
+  // arena layout: first what one copy brings (descriptors, the task list with the
+  // small joins first), then what one memset clears (headers, slots), then the rest
+  const size_t ntasks = small_tasks.size() + tile_tasks.size();
   ej_plan_bytes p;
   const size_t joins_off = p.add(n * sizeof(BatchJoin));
-  const size_t rtiles_off = p.add(std::max<size_t>(rtiles.size(), 1) * sizeof(ej_rx_tile));
-  const size_t rtiles0_off = p.add(std::max<size_t>(rtiles.size(), 1) * sizeof(ej_rx_tile));
-  const size_t tasks_off = p.add(std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask));
-  const size_t sbase_off = p.add(n * sizeof(unsigned long long));
-  const size_t tmpa_off = p.add(std::max<uint64_t>(nr_total, 1) * sizeof(ej_tuple));
-  const size_t tmpb_off = p.add(std::max<uint64_t>(nr_total, 1) * sizeof(ej_tuple));
-  const size_t rkey_off = p.add(ej_table_col_bytes(nr_total));
-  const size_t rval_off = p.add(ej_table_col_bytes(nr_total));
-  const size_t start_off = p.add(start_total * sizeof(uint2));
-  ej_radix_plan rp;
-  rp.n = nr_total;
-  rp.ntiles = (uint32_t)rtiles.size();
-  rp.hist_off = p.add(cells * sizeof(uint32_t));
-  rp.offs_off = p.add((cells + 1) * sizeof(uint32_t));
-  rp.scan_off = p.add(ej_scan_scratch_bytes(cells));
+  const size_t tiles_off = p.add(tiles.size() * sizeof(BatchTile));
+  const size_t tasks_off = p.add(ntasks * sizeof(BatchTask));
+  const size_t up_bytes = p.bytes;
+  const size_t hdr_off = p.add(n * sizeof(BatchTableHeader));
+  const size_t marked_off = p.add(sizeof(uint32_t));
+  const size_t slots_off = p.add(pairs * sizeof(uint4));
+  const size_t clear_bytes = p.bytes - hdr_off;
+  const size_t runs_off = p.add(run_words * sizeof(int32_t));
+  const size_t mark_off = p.add(nr_total * sizeof(uint32_t));
+  const size_t rank_off = p.add(nr_total * sizeof(uint2));
   EJ_TRY(ej_arena_reserve(h, p.bytes));
 
   char* A = static_cast<char*>(h->arena);
-  int32_t* rkey = reinterpret_cast<int32_t*>(A + rkey_off);
-  int32_t* rval = reinterpret_cast<int32_t*>(A + rval_off);
-  uint2* bucket = reinterpret_cast<uint2*>(A + start_off);
   for (uint32_t i = 0; i < n; i++) {
     BatchJoin& b = joins[i];
-    b.view.rkey = rkey + b.r_row0;
-    b.view.rval = rval + b.r_row0;
-    b.view.voff = (uint32_t)(b.r_row0 & 3u);  // the arena column is 16-byte aligned
-    b.view.bucket = bucket + sbase[i];
+    b.slot = reinterpret_cast<unsigned long long*>(A + slots_off + pair0[i] * sizeof(uint4));
+    b.runs = reinterpret_cast<int32_t*>(A + runs_off) + run0[i];
+    b.view.pair = reinterpret_cast<const uint4*>(b.slot);
+    b.view.rkey = b.runs;
   }
-  // descriptors go up with the batch (stream-ordered copies)
-  const size_t jb = n * sizeof(BatchJoin), rb = rtiles.size() * sizeof(ej_rx_tile),
-               pb = tasks.size() * sizeof(BatchTask), sb = n * sizeof(unsigned long long);
-  EJ_CUDA(h, cudaMemcpyAsync(A + joins_off, joins.data(), jb, cudaMemcpyHostToDevice, h->stream));
-  if (rb) EJ_CUDA(h, cudaMemcpyAsync(A + rtiles_off, rtiles.data(), rb, cudaMemcpyHostToDevice, h->stream));
-  // the first radix pass reads every join's R where it lies: the same tiles
-  // with their source rows
-  for (ej_rx_tile& d : rtiles) d.src = joins[d.pad].R + (d.start - joins[d.pad].r_row0);
-  if (rb) EJ_CUDA(h, cudaMemcpyAsync(A + rtiles0_off, rtiles.data(), rb, cudaMemcpyHostToDevice, h->stream));
-  if (pb) EJ_CUDA(h, cudaMemcpyAsync(A + tasks_off, tasks.data(), pb, cudaMemcpyHostToDevice, h->stream));
-  EJ_CUDA(h, cudaMemcpyAsync(A + sbase_off, sbase.data(), sb, cudaMemcpyHostToDevice, h->stream));
+  std::vector<char> up(up_bytes);
+  memcpy(up.data() + joins_off, joins.data(), n * sizeof(BatchJoin));
+  if (!tiles.empty()) memcpy(up.data() + tiles_off, tiles.data(), tiles.size() * sizeof(BatchTile));
+  BatchTask* up_tasks = reinterpret_cast<BatchTask*>(up.data() + tasks_off);
+  std::copy(tile_tasks.begin(), tile_tasks.end(), std::copy(small_tasks.begin(), small_tasks.end(), up_tasks));
+  EJ_CUDA(h, cudaMemcpyAsync(A, up.data(), up_bytes, cudaMemcpyHostToDevice, h->stream));
+  EJ_CUDA(h, cudaMemsetAsync(A + hdr_off, 0, clear_bytes, h->stream));
   EJ_CUDA(h, cudaMemsetAsync(d_counts, 0, n * sizeof(unsigned long long), h->stream));
   const BatchJoin* djoins = reinterpret_cast<const BatchJoin*>(A + joins_off);
-  const ej_rx_tile* drt = reinterpret_cast<const ej_rx_tile*>(A + rtiles_off);
-  rp.tiles = drt;
+  const BatchTile* dtiles = reinterpret_cast<const BatchTile*>(A + tiles_off);
+  uint32_t* mark = reinterpret_cast<uint32_t*>(A + mark_off);
+  uint2* rank = reinterpret_cast<uint2*>(A + rank_off);
+  uint32_t* marked = reinterpret_cast<uint32_t*>(A + marked_off);
+  BatchTableHeader* hdr = reinterpret_cast<BatchTableHeader*>(A + hdr_off);
 
   ej_phase_begin(h);
-  if (!rtiles.empty()) {
-    ej_tuple* tmp[2] = {reinterpret_cast<ej_tuple*>(A + tmpa_off), reinterpret_cast<ej_tuple*>(A + tmpb_off)};
-    ej_radix_plan rp0 = rp;
-    rp0.tiles = reinterpret_cast<const ej_rx_tile*>(A + rtiles0_off);
-    // pass 0 reads the joins' R arrays in place; its order within a digit is
-    // never used (unordered ranking)
-    EJ_TRY(ej_partition_pass_src(h, rp0, tmp[0], 0u, 8u));
-    EJ_TRY(ej_radix_pass(h, rp, tmp[0], tmp[1], 8u, 8u, EJ_DIGIT_HASH));
-    EJ_TRY(ej_radix_pass(h, rp, tmp[1], tmp[0], 16u, 8u, EJ_DIGIT_HASH));
-    EJ_TRY(ej_radix_pass_soa(h, rp, tmp[0], rkey, rval, 24u, 8u, EJ_DIGIT_HASH));
-  }
-  // joins with an empty R keep all-zero bucket starts
-  EJ_CUDA(h, cudaMemsetAsync(bucket, 0, start_total * sizeof(uint2), h->stream));
-  if (!rtiles.empty()) {
-    batch_bucket_start_kernel<<<(unsigned)rtiles.size(), 256, 0, h->stream>>>(
-        drt, djoins, bucket, reinterpret_cast<const unsigned long long*>(A + sbase_off));
-    EJ_TRY(ej_check_launch(h, "batch_bucket_start_kernel"));
+  if (!tiles.empty()) {
+    const uint32_t nt = (uint32_t)tiles.size();
+    const unsigned few = std::min<unsigned>(nt, (unsigned)h->num_sms * 8);
+    batch_insert_kernel<<<nt, 256, 0, h->stream>>>(dtiles, djoins, mark, rank, marked);
+    EJ_TRY(ej_check_launch(h, "batch_insert_kernel"));
+    batch_reserve_kernel<<<few, 256, 0, h->stream>>>(dtiles, nt, djoins, mark, rank, hdr, marked);
+    EJ_TRY(ej_check_launch(h, "batch_reserve_kernel"));
+    batch_place_kernel<<<few, 256, 0, h->stream>>>(dtiles, nt, djoins, mark, rank, marked);
+    EJ_TRY(ej_check_launch(h, "batch_place_kernel"));
   }
   ej_phase_mark(h, 1);
   ej_phase_mark(h, 2);  // no partition pass: every table of a batch is probed in place
   ej_phase_mark(h, 3);  // one pass: recorded as the write phase
-  if (!tasks.empty()) {
-    batch_task_kernel<<<(unsigned)tasks.size(), PR_THREADS, 0, h->stream>>>(
+  if (ntasks) {
+    batch_task_kernel<<<(unsigned)ntasks, PR_THREADS, 0, h->stream>>>(
         djoins, reinterpret_cast<const BatchTask*>(A + tasks_off), h->d_status);
     EJ_TRY(ej_check_launch(h, "batch_task_kernel"));
   }
   ej_phase_mark(h, 4);
+  // the large joins take the arena over, after the launches above
+  for (const uint32_t i : large)
+    EJ_TRY(ej_hash_join_run(h, jd[i].R, jd[i].nR, jd[i].S, jd[i].nS, jd[i].out, jd[i].out_cap, d_counts + i, 0));
   return EJ_OK;
 }
 

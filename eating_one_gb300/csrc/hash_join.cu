@@ -172,6 +172,14 @@ vbucket_start_kernel(const int32_t* __restrict__ rval, uint64_t nR, uint2* __res
   if (r0 <= nR) ej_bucket_edges_warp(rval, nR, r0, bucket, EjValueBucketOf{b.vmin, b.vshift});
 }
 
+// L2 prefetch of the 1 KB of one warp tile's probe tuples (or descriptors,
+// also 8 bytes per probe), one 128-byte line per lane of the first eight;
+// lines past the nP probes are skipped
+__device__ __forceinline__ void ej_prefetch_tile(const void* base, uint64_t w, uint64_t nP, unsigned lane) {
+  const uint64_t off = w * (PR_WTILE * 8) + (uint64_t)lane * 128u;
+  if (lane < 8u && off < nP * 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(base) + off));
+}
+
 // ---- slot tables (slot_table.cuh) --------------------------------------------------
 
 constexpr int SLOT_ITEMS = 4;  // rows per thread and step of the build's kernels
@@ -183,7 +191,7 @@ struct SlotHeader {
 static_assert(sizeof(SlotHeader) <= EJ_SLOT_HEADER_BYTES, "slot table header");
 
 // every row to its key's slot, or marked
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 slot_insert_kernel(const int2* __restrict__ R, uint32_t n, unsigned long long* __restrict__ slot, uint32_t npairs,
                    uint32_t* __restrict__ mark, uint2* __restrict__ rank, SlotHeader* hdr) {
   const uint64_t base = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 * SLOT_ITEMS) + (threadIdx.x & 31u);
@@ -244,11 +252,12 @@ slot_place_kernel(const int2* __restrict__ R, uint32_t n, const uint2* __restric
 template <bool OUTER, bool DESC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS)
 slot_count_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
-                  unsigned long long* __restrict__ wcount, uint64_t nwtiles, void* __restrict__ desc,
+                  unsigned long long* __restrict__ wcount, uint64_t nwtiles, void* __restrict__ desc, uint64_t ahead,
                   unsigned long long* __restrict__ scan_scratch, uint64_t scan_words) {
   ej_clear_words(scan_scratch, scan_words);  // of the scan that follows
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (w >= nwtiles) return;
+  ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);  // the tile a warp one resident wave later takes
   const unsigned long long total = ej_slot_count<OUTER, DESC>(P, w, nP, ej_slots_of(t), desc, nwtiles);
   if ((threadIdx.x & 31u) == 0) wcount[w] = total;
 }
@@ -257,11 +266,12 @@ template <bool OUTER, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 slot_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc, uint64_t nP, ej_table_view t,
                   const unsigned long long* __restrict__ woff, uint64_t nwtiles, ej_result* __restrict__ out,
-                  uint64_t cap, ej_dev_status* st, unsigned long long* total) {
+                  uint64_t cap, ej_dev_status* st, uint64_t ahead, unsigned long long* total) {
   __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
   const unsigned int warp = threadIdx.x >> 5;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
   if (w >= nwtiles) return;
+  ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);  // the tile a warp one resident wave later takes
   if (w == 0 && threadIdx.x == 0) {
     if (woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
     if (total) *total = woff[nwtiles];
@@ -277,11 +287,12 @@ template <bool OUTER, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 slot_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, uint64_t nwtiles,
                   unsigned long long* __restrict__ cursor, ej_result* __restrict__ out, uint64_t cap,
-                  ej_dev_status* st) {
+                  ej_dev_status* st, uint64_t ahead) {
   __shared__ int4 stage[WARPS][PW_STAGE_ROWS];
   const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
   if (w >= nwtiles) return;
+  ej_prefetch_tile(P, w + ahead, nP, lane);  // the tile a warp one resident wave later takes
   EjProbeWarp p;
   int32_t key[PR_ITEMS];
   ej_slot_probe<OUTER>(P, w * PR_WTILE, nP, ej_slots_of(t), p, key);
@@ -302,14 +313,6 @@ slot_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, 
 
 // ---- count, then write from the run descriptors ---------------------------------
 // (probe_write.cuh); the warp-tile totals are scanned in between
-
-// L2 prefetch of the 1 KB of one warp tile's probe tuples (or descriptors,
-// also 8 bytes per probe), one 128-byte line per lane of the first eight;
-// lines past the nP probes are skipped
-__device__ __forceinline__ void ej_prefetch_tile(const void* base, uint64_t w, uint64_t nP, unsigned lane) {
-  const uint64_t off = w * (PR_WTILE * 8) + (uint64_t)lane * 128u;
-  if (lane < 8u && off < nP * 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(base) + off));
-}
 
 // The probe kernels come in two block shapes, WARPS = 8 or 4 warps of one
 // 128-probe warp tile each (EJ_OPT_PROBE_WARPS and the tuning table choose).
@@ -490,10 +493,11 @@ ej_status launch_count_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
   const uint64_t nsw = ej_scan_words(pp.nwtiles);
   if (KIND == EJ_TABLE_HASH && t.pair) {
     if (desc)
-      slot_count_kernel<OUTER, true, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, desc, sw, nsw);
+      slot_count_kernel<OUTER, true, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, desc, ahead,
+                                                                        sw, nsw);
     else
-      slot_count_kernel<OUTER, false, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, nullptr, sw,
-                                                                         nsw);
+      slot_count_kernel<OUTER, false, WARPS><<<grid, TH, 0, h->stream>>>(P, pp.nP, t, wcount, pp.nwtiles, nullptr, ahead,
+                                                                         sw, nsw);
     return ej_check_launch(h, "slot_count_kernel");
   }
   // inner probes of a packed key directory, 16-byte aligned: the lean count
@@ -539,7 +543,7 @@ ej_status launch_write_w(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
   constexpr int TH = WARPS * 32;
   if (KIND == EJ_TABLE_HASH && t.pair) {
     slot_write_kernel<OUTER, WARPS><<<grid, TH, 0, h->stream>>>(P, desc, pp.nP, t, woff, pp.nwtiles, out, cap,
-                                                                        h->d_status, total);
+                                                                        h->d_status, ahead, total);
     return ej_check_launch(h, "slot_write_kernel");
   }
   if (desc_form(t) == EJ_DESC_NONE)
@@ -859,7 +863,7 @@ static ej_status launch_fused_w(ej_handle* h, const ej_probe_plan_t& pp, const e
   if (KIND == EJ_TABLE_HASH && t.pair) {
     slot_fused_kernel<OUTER, WARPS><<<(unsigned)pp.ntiles, WARPS * 32, 0, h->stream>>>(P, pp.nP, t, pp.nwtiles,
                                                                                           cursor, out, cap,
-                                                                                          h->d_status);
+                                                                                          h->d_status, ahead);
     return ej_check_launch(h, "slot_fused_kernel");
   }
   if (t.short_runs)

@@ -13,8 +13,8 @@
 // The hash is a bijection of val, so an equal hash is an equal val; its top bit,
 // which the shift drops, is told by the slot's place: hashes that differ only
 // there have homes npairs / 2 apart, and a walk is shorter (it crosses full
-// pairs only, of which n rows fill fewer than npairs / 2).  One row whose y
-// would be zero takes the several-rows form.
+// pairs only, of which n rows fill fewer than npairs / 2).  One row whose slot
+// would be all zeros (key 0, hash << 1 = 0) takes the several-rows form.
 // A probe of a present or an absent key is answered by one 16-byte load of its
 // home pair unless the pair is full of other keys (under 2% of the probes at a
 // quarter load, a tenth at half), and for a single row the load brings its key.
@@ -27,8 +27,8 @@
 // place the marked rows.  Rows of one key in a warp go together, so that a key
 // with very many rows costs 1/32 of the atomics.
 //
-// What bounds it: the build, the L2's random read-modify-writes (about 45 G
-// slots/s); the probe, its gathers' L2 round trips and, with runs of several
+// What bounds it: the build, the round trips of its compare-and-swaps (40 to 60 G
+// rows/s; the L2 takes 75 to 115 G random ones/s while the slots fit it); the probe, its gathers' L2 round trips and, with runs of several
 // rows, the run keys' gathers.  One GB300, |S| = 4 |R|, a tenth of S absent,
 // build and one-pass probe in us, this table and the hash-sorted one it replaced
 // (MSD passes, bucket sort, bucket bounds), then the whole call into a given
@@ -89,11 +89,11 @@ __device__ __forceinline__ void ej_slot_insert(unsigned long long* __restrict__ 
     for (int j = 0; j < N; j++)
       if (walk >> j & 1u) {
         // the final form, or a counter: of several rows in this warp, or of a
-        // hash without a single-row form (y would be zero)
+        // row whose final form would be all zeros
         const uint32_t y = hash[j] << 1, n = __popc(peers[j]);
         old[j] = atomicCAS(slot + at[j], 0ull,
-                           y && n == 1u ? (unsigned long long)y << 32 | (uint32_t)key[j]
-                                        : (unsigned long long)(y | 1u) << 32 | n);
+                           n == 1u && (y | (uint32_t)key[j]) ? (unsigned long long)y << 32 | (uint32_t)key[j]
+                                                             : (unsigned long long)(y | 1u) << 32 | n);
       }
 #pragma unroll
     for (int j = 0; j < N; j++) {
@@ -102,7 +102,7 @@ __device__ __forceinline__ void ej_slot_insert(unsigned long long* __restrict__ 
       unsigned long long w = old[j];
       if (w == 0ull) {
         walk &= ~(1u << j);
-        if (y && n == 1u) alone |= 1u << j; else m[j].rank = EJ_SLOT_OPENER;
+        if (n == 1u && (y | (uint32_t)key[j])) alone |= 1u << j; else m[j].rank = EJ_SLOT_OPENER;
       } else if (((uint32_t)(w >> 32) | 1u) != (y | 1u)) {
         if (++at[j] == end) at[j] = 0;
       } else {
@@ -160,6 +160,8 @@ __device__ __forceinline__ void ej_slot_reserve(uint2* __restrict__ slot, const 
 
 // ---- probe ----------------------------------------------------------------------
 
+__device__ __forceinline__ bool ej_pair_full(const uint4& q) { return (q.x | q.y) != 0u && (q.z | q.w) != 0u; }
+
 // The matches of N probe values (ok[j] false: none): c[j] rows, the first at
 // rkey[lo[j]], or lo[j] = INLINE_RUN and c[j] = 1: the row with key key[j].
 template <int N>
@@ -177,7 +179,7 @@ __device__ __forceinline__ void ej_slot_find(const EjSlotTable& t, const int32_t
   }
 #pragma unroll
   for (int j = 0; j < N; j++)
-    if (q[j].y != 0u && q[j].w != 0u && (q[j].y | 1u) != h2[j] && (q[j].w | 1u) != h2[j]) walk |= 1u << j;
+    if (ej_pair_full(q[j]) && (q[j].y | 1u) != h2[j] && (q[j].w | 1u) != h2[j]) walk |= 1u << j;
   while (walk) {  // the pairs were full of other keys
 #pragma unroll
     for (int j = 0; j < N; j++)
@@ -187,15 +189,16 @@ __device__ __forceinline__ void ej_slot_find(const EjSlotTable& t, const int32_t
       }
 #pragma unroll
     for (int j = 0; j < N; j++)
-      if ((walk >> j & 1u) && (q[j].y == 0u || q[j].w == 0u || (q[j].y | 1u) == h2[j] || (q[j].w | 1u) == h2[j]))
+      if ((walk >> j & 1u) && (!ej_pair_full(q[j]) || (q[j].y | 1u) == h2[j] || (q[j].w | 1u) == h2[j]))
         walk &= ~(1u << j);
   }
   uint32_t longest = 0;
 #pragma unroll
   for (int j = 0; j < N; j++) {
-    const bool second = (q[j].w | 1u) == h2[j] && q[j].w != 0u;
+    // an empty slot can only look like a key whose hash << 1 is zero
+    const bool second = (q[j].w | 1u) == h2[j] && (q[j].z | q[j].w) != 0u;
     const uint32_t x = second ? q[j].z : q[j].x, y = second ? q[j].w : q[j].y;
-    const bool run = y == h2[j], one = (y ^ 1u) == h2[j] && y != 0u;
+    const bool run = y == h2[j], one = (y ^ 1u) == h2[j] && (x | y) != 0u;
     key[j] = (int32_t)x;
     lo[j] = run ? x >> 5 : INLINE_RUN;
     c[j] = run ? x & 31u : one ? 1u : 0u;
