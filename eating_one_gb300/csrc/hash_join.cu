@@ -8,7 +8,11 @@
 // compares per block, and the write pass repeats all of them.
 //
 // Here:
-//   build  R is sorted by hash32(val): tables of 2^20 rows and more by two
+//   build  Hash tables of up to 2^25 rows by open addressing, one slot per
+//          key (slot_table.cuh; above 2^21 rows by bucket groups, msd.cu; hash
+//          and outer joins of up to 16384 build rows run whole in shared
+//          memory instead, small_join.cu).  Larger ones, and those for which
+//          the options ask, are sorted by hash32(val): from 2^20 rows by two
 //          unordered MSD passes and a shared-memory sort per 16-bit bucket
 //          (msd.cu), smaller ones and sorted indexes by four 8-bit LSD radix
 //          passes (radix.cu); either writes it as two arrays rkey[]/rval[],
@@ -27,8 +31,7 @@
 //          probes with their descriptors, fetches the run keys and writes the
 //          rows through shared memory as coalesced 16-byte streaming stores.
 //          No warp ever waits for another.  The *_count entry points run the
-//          count pass without descriptors.  Output order is deterministic:
-//          probe order, then R run order.
+//          count pass without descriptors.
 // The same kernels serve the sort index (runs by binary search) and the left
 // outer join (OUTER: a probe without matches yields one NULL-extended row).
 #include <climits>
@@ -186,7 +189,8 @@ constexpr int SLOT_ITEMS = 4;  // rows per thread and step of the build's kernel
 
 struct SlotHeader {
   uint32_t marked;  // some row was marked: a key has several rows
-  uint32_t cursor;  // words of rkey[] reserved
+  uint32_t cursor;  // words of rkey[] reserved (direct build)
+  uint32_t nspill;  // rows spilled (build by bucket groups)
 };
 static_assert(sizeof(SlotHeader) <= EJ_SLOT_HEADER_BYTES, "slot table header");
 
@@ -271,7 +275,13 @@ slot_write_kernel(const ej_tuple* __restrict__ P, const void* __restrict__ desc,
   const unsigned int warp = threadIdx.x >> 5;
   const uint64_t w = (uint64_t)blockIdx.x * WARPS + warp;
   if (w >= nwtiles) return;
-  ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);  // the tile a warp one resident wave later takes
+  // the tile a warp one resident wave later takes: its probes and, lanes 8..11, its descriptors
+  ej_prefetch_tile(P, w + ahead, nP, threadIdx.x & 31u);
+  {
+    const uint64_t doff = (w + ahead) * (PR_WTILE * 4) + (uint64_t)((threadIdx.x & 31u) - 8u) * 128u;
+    if ((threadIdx.x & 31u) - 8u < 4u && doff < nP * 4)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(desc) + doff));
+  }
   if (w == 0 && threadIdx.x == 0) {
     if (woff[nwtiles] > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
     if (total) *total = woff[nwtiles];
@@ -589,7 +599,9 @@ bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {
   return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table != EJ_TABLE_FORMAT_DIRECTORY;
 }
 
-size_t ej_slot_run_bytes(uint64_t nR) { return ej_table_col_bytes(nR + nR / 31 + 1); }
+size_t ej_slot_run_bytes(uint64_t nR) {
+  return ej_table_col_bytes(nR + nR / 31 + 1 + (nR > EJ_SLOT_DIRECT_ROWS ? 4ull * EJ_MSD_GROUPS : 0));
+}
 
 size_t ej_table_aux_bytes(const ej_table_plan_t& tp) {
   if (tp.slots) return EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4) + ej_slot_run_bytes(tp.nR);
@@ -617,10 +629,18 @@ void ej_table_plan(ej_plan_bytes& p, ej_table_plan_t& tp, uint64_t nR, bool own_
   if (tp.slots) {
     // at least one pair per row (the walks' bound); a quarter full while that
     // keeps the table well inside L2 and the build is not dwarfed by the probes
-    tp.npairs = (uint32_t)(nR <= SLOT_QUARTER_ROWS && n_probe <= 16 * nR ? 2 * nR + 1 : nR + 1);
+    tp.npairs = nR > EJ_SLOT_DIRECT_ROWS ? ej_msd_slot_pairs(nR)
+                : (uint32_t)(nR <= SLOT_QUARTER_ROWS && n_probe <= 16 * nR ? 2 * nR + 1 : nR + 1);
     if (!own_storage) tp.aux_off = p.add(ej_table_aux_bytes(tp));
     tp.mark_off = p.add((size_t)(nR ? nR : 1) * sizeof(uint32_t));
-    tp.rank_off = p.add((size_t)(nR ? nR : 1) * sizeof(uint2));
+    if (nR > EJ_SLOT_DIRECT_ROWS) {
+      tp.tmp_a_off = p.add((size_t)nR * sizeof(ej_tuple));
+      tp.tmp_b_off = p.add((size_t)nR * sizeof(ej_tuple));
+      tp.gcursor_off = p.add(EJ_MSD_GROUPS * sizeof(uint32_t));
+      ej_msd_plan_add(p, tp.mplan, nR);
+    } else {
+      tp.rank_off = p.add((size_t)(nR ? nR : 1) * sizeof(uint2));
+    }
     return;
   }
   // a directory chosen by the tuning is kept whatever the runs' length
@@ -677,8 +697,16 @@ ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple
     const uint32_t n = (uint32_t)tp.nR;
     const unsigned blocks = (n + 256 * SLOT_ITEMS - 1) / (256 * SLOT_ITEMS);
     const unsigned few = std::min<unsigned>((n + 255) / 256, (unsigned)h->num_sms * 8);
-    EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4), h->stream));
-    if (n) {
+    if (n > EJ_SLOT_DIRECT_ROWS) {
+      EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES, h->stream));
+      EJ_TRY(ej_msd_slots(h, tp.mplan, R, reinterpret_cast<ej_tuple*>(ej_arena_at(h, tp.tmp_a_off)),
+                          reinterpret_cast<ej_tuple*>(ej_arena_at(h, tp.tmp_b_off)), reinterpret_cast<uint4*>(slot),
+                          tp.npairs, runs, reinterpret_cast<uint32_t*>(ej_arena_at(h, tp.gcursor_off)), mark,
+                          &hdr->nspill));
+    } else {
+      EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4), h->stream));
+    }
+    if (n && n <= EJ_SLOT_DIRECT_ROWS) {
       slot_insert_kernel<<<blocks, 256, 0, h->stream>>>(R2, n, slot64, tp.npairs, mark, rank, hdr);
       EJ_TRY(ej_check_launch(h, "slot_insert_kernel"));
       slot_reserve_kernel<<<few, 256, 0, h->stream>>>(n, slot, mark, rank, runs, hdr);
@@ -828,10 +856,14 @@ uint32_t ej_probe_partition_bits(const ej_handle* h, uint64_t nR, uint64_t nS) {
   const uint32_t hb = ej_table_bucket_bits(nR, k.delta);
   const int forced = ej_tuned_partition_bits(h, nR);
   if (forced >= 0) return std::min<uint32_t>((uint32_t)forced, std::min(hb, 8u));
-  if (ej_table_is_slots(nR, k)) return 0;  // at most 64 MB of slots: L2 holds what the probes touch
-  const double table = (double)ej_table_bytes(nR, ej_tuned_bucket_delta(h, nR));
+  const bool slots = ej_table_is_slots(nR, k);
+  const double table = slots ? 16.0 * (double)nR : (double)ej_table_bytes(nR, k.delta);
   const double l2 = (double)(h->l2_bytes ? h->l2_bytes : (size_t)126 << 20);
-  if (table <= l2 / 4.0) return 0;  // the whole table stays L2-resident
+  // what the probes touch stays in L2: a sorted table of a quarter of it; half
+  // full slots, one 16-byte pair a probe, up to 0.6 (4.5 M unique keys and 18 M
+  // probes 435 us against 504 partitioned, 6 M 562 / 618, but 6 M rows of four a
+  // key 828 / 759)
+  if (table <= l2 * (slots ? 0.5 : 0.25)) return 0;
   // one partition's table region should be several MB so that the partitions
   // in flight share L2 with the streaming probe and output traffic (C3's
   // 2^26-row tables: 6 bits, a region of L2/8 by the rows and buckets; with

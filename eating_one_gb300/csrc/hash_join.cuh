@@ -11,17 +11,25 @@
 
 // Hash tables of at most EJ_SLOT_MAX_ROWS rows are slot tables
 // (slot_table.cuh) unless the handle's options or tuning table choose a sort, a
-// load factor or a key directory.  At 2^22 rows the slots take 64 MB, half of
-// L2; the largest sizes measured, 3 M and 2^22 rows, still join faster than with
-// the sorted tables (3 M unique keys 290 us against 424, 2^22 447 against 576).
-constexpr uint64_t EJ_SLOT_MAX_ROWS = 1ull << 22;
+// load factor or a key directory.  At 2^25 rows and four probes a row the join
+// takes 2.71 ms against the sorted tables' 3.48 (unique keys), 3.74 / 4.04 (three
+// rows a key) and 5.07 / 5.02 (eight).  At 2^26 rows unique keys would still gain,
+// but four rows a key, counted and then written, took 7.46 ms against 7.37.
+constexpr uint64_t EJ_SLOT_MAX_ROWS = 1ull << 25;
+// Up to EJ_SLOT_DIRECT_ROWS the slots are claimed through L2, above it group by
+// group in shared memory after two radix passes (msd.cu).  Claims through L2 are
+// quick for unique keys (3 M rows: the join with 12 M probes 275 us against 322
+// in groups) but not once the table leaves half of L2 and keys repeat (two rows
+// each 403 against 388, three 454 against 425; with 1.5 M probes 250 against
+// 219); at 2 M rows the two are level for repeated keys (295 / 288 and 324 / 325).
+constexpr uint64_t EJ_SLOT_DIRECT_ROWS = 1ull << 21;
 constexpr size_t EJ_SLOT_HEADER_BYTES = 256;  // counters, cleared with the slots
 // Hash tables of at least EJ_DIR_MIN_ROWS rows may carry a key directory (one
 // load per probe, seven build launches): the build keeps it when the table's
 // runs average two rows or more and otherwise switches to bucket bounds (one
 // build launch), whenever the caller probes 16 rows per table row or more it
 // keeps it.
-constexpr uint64_t EJ_DIR_MIN_ROWS = EJ_SLOT_MAX_ROWS;
+constexpr uint64_t EJ_DIR_MIN_ROWS = 1ull << 22;
 // a sorted table's aux storage: the value buckets' header, then the bounds
 constexpr size_t EJ_VBUCKET_HEADER_BYTES = 256;
 
@@ -37,7 +45,7 @@ struct ej_table_plan_t {
   ej_msd_plan mplan;
   bool slots = false;     // slot table: no sort, no columns
   uint32_t npairs = 0;
-  size_t mark_off = 0, rank_off = 0;
+  size_t mark_off = 0, rank_off = 0, gcursor_off = 0;
   bool onesweep = false;  // sorted indexes (and hash tables when chosen): one scatter launch per digit
   ej_onesweep_plan oplan;
   // arena offsets; rkey/rval/aux are unused when the table has its own storage
@@ -78,7 +86,8 @@ struct ej_table_knobs {
   int table = EJ_TABLE_FORMAT_PLANNER;
 };
 ej_table_knobs ej_tuned_table_knobs(const ej_handle* h, uint64_t nR);
-// bytes of a slot table's runs: every row, and a count for each of 31 rows and more
+// bytes of a slot table's runs: every row, a count for each of 31 rows and more,
+// and the alignment of the bucket groups' parts
 size_t ej_slot_run_bytes(uint64_t nR);
 // whether a hash table of nR rows is a slot table
 bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k);

@@ -18,11 +18,18 @@
 // (many rows of few keys) is sorted by its CTA through global memory
 // instead, one 8-bit digit at a time.
 //
+// The slot tables of large build sides (slot_table.cuh) share the two passes:
+// their third step builds each bucket group's part of the slot array in shared
+// memory and writes it out whole (msd_slots_kernel).
+//
 // Replaces, for the hash join's build side, the reference's partitioning of
 // R (joins/hashJoin_gpu/main_street/partitioning.cu:133-271, rcount_partitioning
 // + rpartitioning, one 6-bit digit per pass with a host round trip each).
+#include <algorithm>
+
 #include "ej_device.cuh"
 #include "msd.cuh"
+#include "slot_table.cuh"
 
 namespace {
 
@@ -363,6 +370,221 @@ msd_local_kernel(const ej_tuple* __restrict__ in, ej_tuple* __restrict__ tmp, co
   }
 }
 
+// ---- slot tables of large build sides -----------------------------------------------
+// A group of 2^g buckets holds a contiguous range of hashes, so with as many
+// pairs per group (pp) everywhere, the group's keys have their homes in its own
+// pp pairs.  One CTA claims the group's slots in shared memory, gives the keys
+// with several rows their runs (words [lo + lo / 31 + 4 group, ...) of rkey[], where
+// the group's rows begin at lo: room for its rows and the long runs' counts), and
+// writes slots and runs out.  A key whose walk passes the group's end is
+// spilled: its rows go to a list that the passes below insert into the finished
+// array (a row or two per group at half load; its run comes from the group's
+// own words).  Random slot updates through L2 (slot_insert_kernel) run at 40 to
+// 60 G rows/s; here they stay in shared memory and the slots leave in
+// coalesced stores.  Bound by the shared memory's compare-and-swaps (random
+// 8-byte words, a warp's longest walk of about five rounds): 2^24 rows in 193 to
+// 200 us, 84 G rows/s, where the local sort and the directory or bucket launches
+// took 230 to 250; four CTAs an SM with the runs' cursors in shared memory too
+// were level with six.  The build of a 2^24-row table in all: 446 us (432 with
+// the sort), and the probes of unique keys then take 665 us instead of 1052.
+constexpr uint32_t SB_PER = 12;           // rows per thread kept in registers (groups up to 3072 rows)
+constexpr uint32_t SB_SPILLED = 0xFFFFu;  // a row's slot within its group (of 4098 at most): walked past the end
+constexpr uint32_t SB_NONE = 0xFFFEu;     // no row
+constexpr int SB_BLOCKS = 6;  // CTAs per SM
+
+// row of hash hv into the group's array (pairs p0 ..., `end` slots): its slot, and
+// its rank among its key's rows
+__device__ __forceinline__ uint32_t sb_claim(unsigned long long* slot, uint32_t hv, uint32_t npairs, uint32_t p0,
+                                             uint32_t end, uint32_t* rank) {
+  const uint32_t y = hv << 1 | 1u;
+  *rank = 0u;
+  for (uint32_t s = 2u * (ej_home_pair(hv, npairs) - p0); s < end; s++) {
+    const unsigned long long old = atomicCAS(slot + s, 0ull, (unsigned long long)y << 32 | 1u);
+    if (old == 0ull) return s;
+    if ((uint32_t)(old >> 32) == y) {
+      *rank = atomicAdd(reinterpret_cast<uint32_t*>(slot + s), 1u);
+      return s;
+    }
+  }
+  return SB_SPILLED;
+}
+
+// that slot again, once the slots have their final form
+__device__ __forceinline__ uint32_t sb_find(const unsigned long long* slot, uint32_t hv, uint32_t npairs, uint32_t p0,
+                                            uint32_t end) {
+  for (uint32_t s = 2u * (ej_home_pair(hv, npairs) - p0); s < end; s++)
+    if (((uint32_t)(slot[s] >> 32) | 1u) == (hv << 1 | 1u) && slot[s] != 0ull) return s;
+  return SB_SPILLED;
+}
+
+// a row to its place once the runs are laid out: its key into the slot, or to
+// its place in the run
+__device__ __forceinline__ void sb_place(unsigned long long* slot, uint32_t s, uint32_t rank, int32_t key,
+                                         int32_t* __restrict__ rkey) {
+  const unsigned long long w = slot[s];
+  if (w >> 32 & 1u)
+    rkey[((uint32_t)w >> 5) + rank] = key;
+  else
+    reinterpret_cast<int32_t*>(slot + s)[0] = key;
+}
+
+__global__ void __launch_bounds__(LS_THREADS, SB_BLOCKS)
+msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ bstart, uint32_t g, uint32_t npairs,
+                 uint32_t pp, uint4* __restrict__ pair, int32_t* __restrict__ rkey, uint32_t* __restrict__ gcursor,
+                 uint2* __restrict__ spill, uint32_t* __restrict__ nspill, uint32_t* __restrict__ ranks) {
+  extern __shared__ __align__(16) unsigned char sb_smem_raw[];
+  unsigned long long* slot = reinterpret_cast<unsigned long long*>(sb_smem_raw);
+  __shared__ uint32_t s_runs;
+  const uint32_t t = threadIdx.x, lane = t & 31u, end = 2u * pp, p0 = blockIdx.x * pp;
+  // bounds clamped to [0, n) and ordered (they are, unless a scan timed out)
+  const uint32_t n = bstart[MSD_BUCKETS];
+  const uint32_t lo = min(bstart[blockIdx.x << g], n);
+  const uint32_t m = max(min(bstart[(blockIdx.x + 1u) << g], n), lo) - lo;
+  // the group's words begin at a multiple of four, so that runs of four rows
+  // throughout (one 16-byte load each) stay aligned
+  const uint32_t words0 = ((lo + lo / 31u) & ~3u) + 4u * blockIdx.x;
+  const int2* rows = reinterpret_cast<const int2*>(in) + lo;
+  for (uint32_t i = t; i < pp; i += LS_THREADS) reinterpret_cast<uint4*>(slot)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (t == 0) s_runs = 0u;
+  __syncthreads();
+  // 1. every row's slot, claimed or counted in; rows past the group's end listed
+  int32_t key[SB_PER];
+  uint32_t at[SB_PER];  // slot | rank << 16
+  const bool big = m > SB_PER * LS_THREADS;
+  for (uint32_t j0 = 0; j0 < m; j0 += SB_PER * LS_THREADS) {
+#pragma unroll
+    for (uint32_t q = 0; q < SB_PER; q++) {  // the loads together
+      const uint32_t j = j0 + t + q * LS_THREADS;
+      const int2 r = j < m ? __ldcs(rows + j) : make_int2(0, 0);
+      key[q] = r.x;
+      at[q] = (uint32_t)r.y;
+    }
+    // one row after the other, each warp until its longest walk ends (all rows'
+    // walks advancing together took 2.5 times the instructions: 464 us at 2^24)
+#pragma unroll
+    for (uint32_t q = 0; q < SB_PER; q++) {
+      const uint32_t j = j0 + t + q * LS_THREADS, val = at[q];
+      at[q] = SB_NONE;
+      if (j >= m) continue;
+      uint32_t rank;
+      const uint32_t s = sb_claim(slot, ej_hash32(val), npairs, p0, end, &rank);
+      if (s == SB_SPILLED) spill[atomicAdd(nspill, 1u)] = make_uint2((uint32_t)key[q], val);
+      if (big) ranks[lo + j] = rank; else at[q] = s | rank << 16;
+    }
+  }
+  __syncthreads();
+  // 2. the final form of every slot but the single rows' keys; runs laid out
+  for (uint32_t s0 = 0; s0 < end; s0 += LS_THREADS) {
+    const uint32_t s = s0 + t;
+    const unsigned long long w = s < end ? slot[s] : 0ull;
+    const uint32_t c = (uint32_t)w, y = (uint32_t)(w >> 32);
+    const bool run = y != 0u && (c > 1u || y == 1u);
+    const uint32_t need = run ? c + (c >= 31u ? 1u : 0u) : 0u;
+    if (y != 0u && !run) slot[s] = (unsigned long long)(y & ~1u) << 32;
+    if (!__any_sync(EJ_FULL_MASK, run)) continue;
+    const uint32_t incl = ej_warp_inclusive_sum(need);
+    uint32_t first = 0;
+    if (lane == 31u) first = atomicAdd(&s_runs, incl);
+    first = words0 + __shfl_sync(EJ_FULL_MASK, first, 31) + incl - need;
+    if (!run) continue;
+    if (c >= 31u) rkey[first++] = (int32_t)c;
+    slot[s] = (unsigned long long)y << 32 | (first << 5 | min(c, 31u));
+  }
+  __syncthreads();
+  // 3. every row to its slot or run
+  if (!big) {
+#pragma unroll
+    for (uint32_t q = 0; q < SB_PER; q++)
+      if ((at[q] & 0xFFFFu) < SB_NONE) sb_place(slot, at[q] & 0xFFFFu, at[q] >> 16, key[q], rkey);
+  } else {
+    for (uint32_t j = t; j < m; j += LS_THREADS) {
+      const int2 r = __ldg(rows + j);
+      const uint32_t s = sb_find(slot, ej_hash32((uint32_t)r.y), npairs, p0, end);
+      if (s != SB_SPILLED) sb_place(slot, s, ranks[lo + j], r.x, rkey);
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = t; i < pp; i += LS_THREADS) pair[p0 + i] = reinterpret_cast<const uint4*>(slot)[i];
+  if (t == 0) gcursor[blockIdx.x] = words0 + s_runs;
+}
+
+// The spilled rows, by slot_table.cuh's steps on the whole array; their runs come
+// from their home groups' words.  A spilled row's key is in none of its group's
+// slots from its home on, so its walk starts behind the group, and passes the
+// slots that hold other keys for good eight at a time (one compare-and-swap a
+// slot from the home on took 19 us for a few hundred rows).
+__global__ void __launch_bounds__(256)
+spill_insert_kernel(const uint2* __restrict__ spill, const uint32_t* __restrict__ nspill,
+                    unsigned long long* slot, uint32_t npairs, uint32_t pp, uint32_t g, uint32_t* __restrict__ mark,
+                    uint2* __restrict__ rank) {
+  const uint32_t n = *nspill;
+  for (uint64_t i0 = ((uint64_t)blockIdx.x * 256 + threadIdx.x) & ~31ull; i0 < n; i0 += (uint64_t)gridDim.x * 256) {
+    const uint64_t i = i0 + (threadIdx.x & 31u);
+    const bool ok[1] = {i < n};
+    const uint2 r = ok[0] ? __ldg(spill + i) : make_uint2(0u, 0u);
+    const int32_t key[1] = {(int32_t)r.x};
+    const uint32_t hv[1] = {ej_hash32(r.y)};
+    uint32_t q = ((hv[0] >> (32u - MSD_BUCKET_BITS + g)) + 1u) * pp;  // pair behind the group
+    for (bool found = !ok[0]; !found;) {  // ends: more than half of the slots stay empty
+      uint4 w[4];
+#pragma unroll
+      for (uint32_t e = 0; e < 4; e++) {
+        const uint32_t a = q + e < npairs ? q + e : q + e - npairs;
+        w[e] = __ldcg(reinterpret_cast<const uint4*>(slot) + a);
+      }
+#pragma unroll
+      for (uint32_t e = 0; e < 4; e++) {
+        const uint32_t y = hv[0] << 1 | 1u;
+        found = found || (w[e].x | w[e].y) == 0u || (w[e].z | w[e].w) == 0u || (w[e].y | 1u) == y || (w[e].w | 1u) == y;
+        if (!found) q++;
+      }
+      if (q >= npairs) q -= npairs;
+    }
+    const uint32_t at[1] = {2u * (q < npairs ? q : q - npairs)};
+    EjSlotMark m[1];
+    ej_slot_insert<1, true>(slot, npairs, key, hv, ok, m, at);
+    if (ok[0]) {
+      mark[i] = m[0].mark;
+      rank[i] = make_uint2(m[0].rank, (uint32_t)m[0].first);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256)
+spill_reserve_kernel(const uint2* __restrict__ spill, const uint32_t* __restrict__ nspill, uint2* __restrict__ slot,
+                     const uint32_t* __restrict__ mark, const uint2* __restrict__ rank, uint32_t g,
+                     int32_t* __restrict__ rkey, uint32_t* __restrict__ gcursor) {
+  const uint32_t n = *nspill;
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
+    const uint32_t m = __ldg(mark + i);
+    const uint2 r = __ldg(rank + i);
+    if (!m || !(r.x & EJ_SLOT_OPENER)) continue;
+    const uint32_t c = slot[m - 1u].x;
+    uint32_t lo = atomicAdd(gcursor + (ej_hash32(__ldg(&spill[i].y)) >> (32u - MSD_BUCKET_BITS + g)),
+                            c + (c >= 31u ? 1u : 0u));
+    if (c >= 31u) rkey[lo++] = (int32_t)c;
+    if (r.x & 1u) rkey[lo] = (int32_t)r.y;
+    slot[m - 1u].x = lo << 5 | min(c, 31u);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+spill_place_kernel(const uint2* __restrict__ spill, const uint32_t* __restrict__ nspill, const uint2* __restrict__ slot,
+                   const uint32_t* __restrict__ mark, const uint2* __restrict__ rank, int32_t* __restrict__ rkey) {
+  const uint32_t n = *nspill;
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
+    const uint32_t m = __ldg(mark + i);
+    if (m) rkey[(__ldg(&slot[m - 1u].x) >> 5) + (__ldg(&rank[i].x) & ~EJ_SLOT_OPENER)] = (int32_t)__ldg(&spill[i].x);
+  }
+}
+
+// bucket groups of 2^g buckets of about LS_ROWS rows in all
+uint32_t msd_group_bits(uint64_t n) {
+  uint32_t g = 0;
+  while (g < LS_MAX_GROUP_BITS && ((uint64_t)LS_ROWS << MSD_BUCKET_BITS) >= (n << (g + 1))) g++;
+  return g;
+}
+
 }  // namespace
 
 void ej_msd_plan_add(ej_plan_bytes& p, ej_msd_plan& mp, uint64_t n) {
@@ -380,10 +602,14 @@ void ej_msd_plan_add(ej_plan_bytes& p, ej_msd_plan& mp, uint64_t n) {
   mp.bstart_off = p.add((MSD_BUCKETS + 1) * sizeof(uint32_t));
 }
 
-ej_status ej_msd_sort(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
-                      int32_t* rkey, int32_t* rval) {
-  if (mp.n == 0) return EJ_OK;
-  if (mp.n >= 0xFFFFFFFFull) return ej_fail(h, EJ_ERR_TOO_LARGE, "table of %llu rows", (unsigned long long)mp.n);
+uint32_t ej_msd_slot_pairs(uint64_t n) {
+  const uint64_t groups = MSD_BUCKETS >> msd_group_bits(n);
+  return (uint32_t)((n + groups) / groups * groups);  // above n, the same for every group
+}
+
+// the two radix passes (rows in tmp_b, tmp_a free again) and the bucket bounds
+static ej_status msd_passes(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
+                            uint32_t** bounds) {
   // 1. by bits 24..31
   EJ_TRY(ej_partition_pass(h, mp.pass1, R, tmp_a, 24u, 8u, EJ_DIGIT_HASH));
   // 2. by bits 16..23 inside every segment, tiles laid out on the device
@@ -397,14 +623,49 @@ ej_status ej_msd_sort(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej
   ej_radix_plan p2 = mp.pass2;
   p2.tiles = desc;
   EJ_TRY(ej_partition_pass(h, p2, tmp_a, tmp_b, 16u, 8u, EJ_DIGIT_HASH));
-  // 3. bucket bounds, then every bucket by bits 0..15 into the columns
+  // 3. bucket bounds
   uint32_t* bstart = reinterpret_cast<uint32_t*>(ej_arena_at(h, mp.bstart_off));
   const uint32_t* offs2 = reinterpret_cast<const uint32_t*>(ej_arena_at(h, mp.pass2.offs_off));
   msd_bucket_kernel<<<(MSD_BUCKETS + 1 + 255) / 256, 256, 0, h->stream>>>(seg, offs2, mp.n, bstart);
   EJ_TRY(ej_check_launch(h, "msd_bucket_kernel"));
-  // groups of 2^g buckets of about LS_ROWS rows in all
-  uint32_t g = 0;
-  while (g < LS_MAX_GROUP_BITS && ((uint64_t)LS_ROWS << MSD_BUCKET_BITS) >= (mp.n << (g + 1))) g++;
+  *bounds = bstart;
+  return EJ_OK;
+}
+
+ej_status ej_msd_slots(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
+                       uint4* pair, uint32_t npairs, int32_t* rkey, uint32_t* gcursor, uint32_t* mark,
+                       uint32_t* nspill) {
+  uint32_t* bstart = nullptr;
+  EJ_TRY(msd_passes(h, mp, R, tmp_a, tmp_b, &bstart));
+  const uint32_t g = msd_group_bits(mp.n), groups = MSD_BUCKETS >> g, pp = npairs / groups;
+  const int smem = (int)(2u * pp * sizeof(unsigned long long));
+  EJ_CUDA(h, cudaFuncSetAttribute(msd_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  uint2* spill = reinterpret_cast<uint2*>(tmp_a);
+  msd_slots_kernel<<<groups, LS_THREADS, smem, h->stream>>>(tmp_b, bstart, g, npairs, pp, pair, rkey, gcursor, spill,
+                                                           nspill, mark);
+  EJ_TRY(ej_check_launch(h, "msd_slots_kernel"));
+  // the spilled rows' marks (mark held large groups' ranks before); their ranks
+  // in tmp_b, whose rows are in the table now
+  uint2* rank = reinterpret_cast<uint2*>(tmp_b);
+  uint2* slot = reinterpret_cast<uint2*>(pair);
+  const unsigned blocks = (unsigned)h->num_sms * 2;
+  spill_insert_kernel<<<blocks, 256, 0, h->stream>>>(spill, nspill, reinterpret_cast<unsigned long long*>(pair), npairs,
+                                                    pp, g, mark, rank);
+  EJ_TRY(ej_check_launch(h, "spill_insert_kernel"));
+  spill_reserve_kernel<<<blocks, 256, 0, h->stream>>>(spill, nspill, slot, mark, rank, g, rkey, gcursor);
+  EJ_TRY(ej_check_launch(h, "spill_reserve_kernel"));
+  spill_place_kernel<<<blocks, 256, 0, h->stream>>>(spill, nspill, slot, mark, rank, rkey);
+  return ej_check_launch(h, "spill_place_kernel");
+}
+
+ej_status ej_msd_sort(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
+                      int32_t* rkey, int32_t* rval) {
+  if (mp.n == 0) return EJ_OK;
+  if (mp.n >= 0xFFFFFFFFull) return ej_fail(h, EJ_ERR_TOO_LARGE, "table of %llu rows", (unsigned long long)mp.n);
+  uint32_t* bstart = nullptr;
+  EJ_TRY(msd_passes(h, mp, R, tmp_a, tmp_b, &bstart));
+  // every bucket by bits 0..15 into the columns
+  const uint32_t g = msd_group_bits(mp.n);
   EJ_CUDA(h, cudaFuncSetAttribute(msd_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LsSmem)));
   msd_local_kernel<<<MSD_BUCKETS >> g, LS_THREADS, sizeof(LsSmem), h->stream>>>(tmp_b, tmp_a, bstart, g, rkey, rval);
   return ej_check_launch(h, "msd_local_kernel");

@@ -2,16 +2,17 @@
 //
 // A table stores R as rkey[]/rval[] in one order (ej_table_view).  In both
 // kinds the matches of a value v form one contiguous run [lo, lo + c):
-//   EJ_TABLE_HASH    rows sorted by hash32(val).  Single tables of 2^22 rows
-//                    or more whose runs average two rows or more, and those
-//                    of 2^20 rows or more whose caller probes 16 rows per
-//                    table row, carry a key directory (8-byte entries {hash, lo} in hash order,
-//                    linear probing from slot hash >> (32 - bits), each slot
-//                    holding the first key at or after it, so c is the next
-//                    slot's start minus lo); the others, smaller and batched
-//                    tables carry bucket bounds: the run lies inside bucket b
-//                    = top hb hash bits, rows [bucket[b].x, bucket[b].y) (one
-//                    8-byte load);
+//   EJ_TABLE_HASH    rows sorted by hash32(val) (tables of more than 2^25 rows,
+//                    and those for which a sort, a load factor or a directory
+//                    was chosen; the others are slot tables, slot_table.cuh).
+//                    Tables of 2^22 rows or more whose runs average two rows
+//                    or more, or whose caller probes 16 rows per table row,
+//                    carry a key directory (8-byte entries {hash, lo} in hash
+//                    order, linear probing from slot hash >> (32 - bits), each
+//                    slot holding the first key at or after it, so c is the
+//                    next slot's start minus lo); the others bucket bounds:
+//                    the run lies inside bucket b = top hb hash bits, rows
+//                    [bucket[b].x, bucket[b].y) (one 8-byte load);
 //   EJ_TABLE_SORTED  rows sorted by val, with bucket bounds over value
 //                    prefixes: bucket b = (v - vmin) >> vshift (the table's
 //                    smallest and largest vals and the shift in a small

@@ -1,6 +1,7 @@
 // slot_table.cuh - hash tables by open addressing (device code): the build's
 // steps and the probe's find, shared by the single joins (hash_join.cu), the
-// star join (index.cu) and the batched joins (batch.cu).
+// star join (index.cu), the batched joins (batch.cu) and, for the rows that its
+// bucket groups spill, the build of large tables (msd.cu).
 //
 // A table of n rows has one 8-byte slot {x, y} per distinct key, in an array of
 // npairs >= n aligned pairs (so at most half full), found from the key's home
@@ -28,13 +29,15 @@
 // with very many rows costs 1/32 of the atomics.
 //
 // What bounds it: the build, the round trips of its compare-and-swaps (40 to 60 G
-// rows/s; the L2 takes 75 to 115 G random ones/s while the slots fit it); the probe, its gathers' L2 round trips and, with runs of several
-// rows, the run keys' gathers.  One GB300, |S| = 4 |R|, a tenth of S absent,
+// rows/s; the L2 takes 75 to 115 G random ones/s while the slots fit it); the
+// probe, its gathers' L2 round trips and, with runs of several rows, the run
+// keys' gathers.  One GB300, |S| = 4 |R|, a tenth of S absent,
 // build and one-pass probe in us, this table and the hash-sorted one it replaced
 // (MSD passes, bucket sort, bucket bounds), then the whole call into a given
 // output: 2^18 rows 32 + 17 and 80 + 25 (89, 152); 2^20 50 + 45 and 94 + 73 (136,
-// 213); 3 M 121 + 130 and 126 + 179 (290, 424); 3 M rows of 1 M keys 172 + 249 and
-// 134 + 267 (464, 526); 3 M of 375 K 158 + 394 and 139 + 411 (594, 674).  Tried and
+// 213).  Above 2^21 rows (built by groups, msd.cu) the whole call: 3 M 322 and 349;
+// 3 M rows of 1 M keys 425 and 454; 3 M of 375 K 575 and 663; 12 M 1075 and 1325;
+// 12 M of 4 M keys 1437 and 1524; 2^25 2711 and 3475.  Tried and
 // dropped on the way: buckets by hash with the row in the slot when alone, else a
 // pointer to the bucket's rows - unsorted rows walked by each probe (2^20 151, but
 // 3 M of 375 K 975), rows grouped by key in a further pass (180 and 660): the
@@ -69,17 +72,19 @@ constexpr uint32_t EJ_SLOT_OPENER = 0x80000000u;
 
 // N rows of this lane (ok[j]: there is one) claim slots of the zeroed array or
 // are marked.  All lanes' walks advance together, one compare-and-swap per row
-// and round.
-template <int N>
+// and round.  FROM: the walks begin at slot from[j], which the key's walk from
+// its home has to pass, instead of the home.
+template <int N, bool FROM = false>
 __device__ __forceinline__ void ej_slot_insert(unsigned long long* __restrict__ slot, uint32_t npairs,
                                                const int32_t (&key)[N], const uint32_t (&hash)[N],
-                                               const bool (&ok)[N], EjSlotMark (&m)[N]) {
+                                               const bool (&ok)[N], EjSlotMark (&m)[N],
+                                               const uint32_t* from = nullptr) {
   const uint32_t lane = threadIdx.x & 31u, end = 2u * npairs;
   uint32_t walk = 0, alone = 0, peers[N], at[N];
 #pragma unroll
   for (int j = 0; j < N; j++) {
     peers[j] = __match_any_sync(EJ_FULL_MASK, hash[j]) & __ballot_sync(EJ_FULL_MASK, ok[j]);
-    at[j] = 2u * ej_home_pair(hash[j], npairs);
+    at[j] = FROM ? from[j] : 2u * ej_home_pair(hash[j], npairs);
     m[j] = {0u, 0u, 0};
     if (ok[j] && __ffs(peers[j]) - 1 == (int)lane) walk |= 1u << j;  // the first of the key's rows in the warp
   }
@@ -238,11 +243,20 @@ __device__ __forceinline__ void ej_slot_probe(const ej_tuple* __restrict__ P, ui
 }
 
 // The rows of a warp tile with runs, from out[off] on: a function of its own, so
-// that its registers (the run keys) do not burden the tiles without.
-static __device__ __noinline__ void ej_slot_emit_runs(EjProbeWarp p, int4 key4, const ej_table_view& t,
-                                                      unsigned long long off, ej_result* __restrict__ out,
-                                                      uint64_t cap, int4* stage) {
+// that its registers (the run keys) do not burden the tiles without.  Its
+// arguments travel in registers (a structure passed by reference would live in
+// local memory: 1242 us instead of 1098 for the one-pass probes of 2^24 rows of
+// four a key).
+static __device__ __noinline__ void ej_slot_emit_runs(int4 skey, int4 sval, uint4 lo, uint4 cnt, int4 key4,
+                                                      const int32_t* __restrict__ rkey, unsigned long long off,
+                                                      ej_result* __restrict__ out, uint64_t cap, int4* stage) {
+  const EjProbeWarp p = {{make_int2(skey.x, sval.x), make_int2(skey.y, sval.y), make_int2(skey.z, sval.z),
+                          make_int2(skey.w, sval.w)},
+                         {lo.x, lo.y, lo.z, lo.w},
+                         {cnt.x, cnt.y, cnt.z, cnt.w}};
   const int32_t key[PR_ITEMS] = {key4.x, key4.y, key4.z, key4.w};
+  ej_table_view t;
+  t.rkey = rkey;
   int32_t kk[PR_ITEMS][PW_PREFETCH];
   ej_probe_prefetch<EJ_KEYS_WINDOW, true>(t, p, kk, key);
   ej_emit_warp<true>(p, kk, t, off, out, cap, stage);
@@ -271,8 +285,10 @@ __device__ __forceinline__ void ej_slot_emit(const EjProbeWarp& p, const int32_t
     }
     return;
   }
-  static_assert(PR_ITEMS == 4, "the keys travel as one int4");
-  ej_slot_emit_runs(p, make_int4(key[0], key[1], key[2], key[3]), t, off, out, cap, stage);
+  static_assert(PR_ITEMS == 4, "four probes travel as vectors");
+  ej_slot_emit_runs(make_int4(p.s[0].x, p.s[1].x, p.s[2].x, p.s[3].x), make_int4(p.s[0].y, p.s[1].y, p.s[2].y, p.s[3].y),
+                    make_uint4(p.lo[0], p.lo[1], p.lo[2], p.lo[3]), make_uint4(p.cnt[0], p.cnt[1], p.cnt[2], p.cnt[3]),
+                    make_int4(key[0], key[1], key[2], key[3]), t.rkey, off, out, cap, stage);
 }
 
 // Run descriptors of the two-pass probe: per probe one word, the key of a
@@ -310,8 +326,7 @@ __device__ __forceinline__ unsigned long long ej_slot_count(const ej_tuple* __re
 }
 
 // write pass of warp tile w, whose output starts at out[off], from the count
-// pass's descriptors (runs of 31 rows and more: the tile's probes are found
-// again)
+// pass's descriptors
 template <bool OUTER>
 __device__ __forceinline__ void ej_slot_write(const ej_tuple* __restrict__ P, const void* __restrict__ desc,
                                               uint64_t w, uint64_t nwtiles, uint64_t nP, const ej_table_view& t,
@@ -339,6 +354,10 @@ __device__ __forceinline__ void ej_slot_write(const ej_tuple* __restrict__ P, co
       p.lo[j] = NULL_RUN;
     }
   }
-  if (__any_sync(EJ_FULL_MASK, escape)) ej_slot_probe<OUTER>(P, w * PR_WTILE, nP, ej_slots_of(t), p, key);
+  if (__any_sync(EJ_FULL_MASK, escape)) {  // runs of 31 rows and more: their lengths precede them
+#pragma unroll
+    for (int j = 0; j < PR_ITEMS; j++)
+      if (p.cnt[j] == EJ_PACKED_ESCAPE) p.cnt[j] = (uint32_t)__ldg(t.rkey + p.lo[j] - 1);
+  }
   ej_slot_emit(p, key, t, off, out, cap, stage);
 }

@@ -1,8 +1,9 @@
-"""Slot tables (open addressing, 16385 to 2^22 rows) where they can go wrong, in
+"""Slot tables (open addressing, 16385 to 2^26 rows) where they can go wrong, in
 every join that probes one, against the oracle: the hashes whose low 31 bits
 are zero (no single-row form), keys of 30, 31, 32 and thousands of rows, homes
-crowded at both ends of the array (long walks, wrapping round), the ends of
-the size range."""
+crowded at both ends of the array (long walks, wrapping round, and past the
+bucket groups of the large build, above 2^21 rows), the ends of the size
+range."""
 import numpy as np
 import pytest
 import torch
@@ -56,10 +57,15 @@ def _rel(vals, base, rng):
     return a
 
 
+@pytest.mark.parametrize("large", [False, True], ids=["direct", "grouped"])
 @pytest.mark.parametrize("name", ["special_hashes", "absent_special", "run_lengths", "crowded_homes", "smallest"])
-def test_slot_table(engine, name):
+def test_slot_table(engine, name, large):
     rng = np.random.default_rng(len(name))
     rv, sv = _case(name, rng)
+    if large:  # enough other rows for the build by bucket groups
+        rv = np.concatenate([rv, np.arange(1100000000, 1100000000 + (1 << 21))])
+        if name == "run_lengths":  # a bucket group far larger than shared memory
+            rv = np.concatenate([rv, np.repeat(10, 20000)])
     R, S = _rel(rv, 0, rng), _rel(sv, 1 << 20, rng)
     Rd, Sd = torch.from_numpy(R).cuda(), torch.from_numpy(S).cuda()
     inner, outer = O.canon(O.hash_join(R, S)), O.canon(O.left_outer_join(R, S))
@@ -77,9 +83,9 @@ def test_slot_table(engine, name):
     assert np.array_equal(O.canon(engine.star_join3(*args).cpu().numpy()), want)
 
 
-def test_largest(engine):
-    """The last size with a slot table and the first without, and a capacity one short."""
-    for n in (1 << 22, (1 << 22) + 1):
+def test_build_sizes(engine):
+    """The last size of the direct build, the first built by bucket groups, and a larger one."""
+    for n in (1 << 21, (1 << 21) + 1, 1 << 24):
         R = torch.empty((n, 2), dtype=torch.int32, device="cuda")
         R[:, 0] = torch.arange(n, device="cuda")
         R[:, 1] = torch.randperm(n, device="cuda") * 3
