@@ -914,16 +914,22 @@ static ej_status launch_fused(ej_handle* h, const ej_probe_plan_t& pp, const ej_
                        : launch_fused_w<KIND, OUTER, 8>(h, pp, P, t, cursor, out, cap);
 }
 
-// [partition +] the fused pass; the count ends in *cursor (zeroed here)
-static ej_status ej_probe_fused(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
-                                bool outer, ej_result* out, uint64_t cap, unsigned long long* cursor) {
-  EJ_CUDA(h, cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), h->stream));
+// the fused pass, rows from *cursor on
+ej_status ej_probe_append(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
+                          bool outer, ej_result* out, uint64_t cap, unsigned long long* cursor) {
   if (!pp.ntiles) return EJ_OK;
   if (t.kind == EJ_TABLE_HASH)
     return outer ? launch_fused<EJ_TABLE_HASH, true>(h, pp, P, t, cursor, out, cap)
                  : launch_fused<EJ_TABLE_HASH, false>(h, pp, P, t, cursor, out, cap);
   return outer ? launch_fused<EJ_TABLE_SORTED, true>(h, pp, P, t, cursor, out, cap)
                : launch_fused<EJ_TABLE_SORTED, false>(h, pp, P, t, cursor, out, cap);
+}
+
+// the fused pass; the count ends in *cursor (zeroed here)
+static ej_status ej_probe_fused(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
+                                bool outer, ej_result* out, uint64_t cap, unsigned long long* cursor) {
+  EJ_CUDA(h, cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), h->stream));
+  return ej_probe_append(h, pp, P, t, outer, out, cap, cursor);
 }
 
 // Partition S (when the layout says so), count (+ scan), then write unless

@@ -108,6 +108,11 @@ ej_status ej_probe_count(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple
 ej_status ej_probe_write(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
                          ej_result* out, uint64_t cap, bool outer = false, unsigned long long* total = nullptr);
 
+// one pass: the matches of P from row *cursor (a device word) on, which ends
+// behind them; rows at or past cap are counted, not written
+ej_status ej_probe_append(ej_handle* h, const ej_probe_plan_t& pp, const ej_tuple* P, const ej_table_view& t,
+                          bool outer, ej_result* out, uint64_t cap, unsigned long long* cursor);
+
 uint32_t ej_probe_partition_bits(const ej_handle* h, uint64_t nR, uint64_t nS);
 // two_pass: plan the run descriptors of ej_probe_count + ej_probe_write (for
 // callers that read the count in between); ej_probe_exec needs none

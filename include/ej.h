@@ -406,8 +406,9 @@ ej_status ej_join_host(ej_handle* h, ej_algo algo, const ej_tuple* R, uint64_t n
  * block's table once); S streams through in chunks of at most s_chunk_rows,
  * double-buffered, so the upload of one chunk and the download of the
  * previous chunk's rows overlap the join of the current one.  Pinned host
- * buffers are used in place (a pinned out receives rows straight from the
- * write pass); pageable ones are staged.  Rows come in (R block, S chunk)
+ * buffers are used in place: a pinned out receives rows straight from the
+ * write pass, and a hash join whose probes need no partitioning reads a pinned
+ * S (16-byte aligned) from there too, in the same pass; pageable ones are staged.  Rows come in (R block, S chunk)
  * order; past out_cap they are counted only (EJ_ERR_CAPACITY, *out_count =
  * the full count).  Replaces the whole-relation transfers around the
  * reference kernels (joins/hashJoin_gpu/main_street/hj.cc:345-354, :1124) and
