@@ -164,7 +164,7 @@ __device__ __forceinline__ void batch_probe_tile(const BatchJoin& j, uint32_t lo
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(j.d_count, total);
-    if (off + total > j.cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (off <= j.cap && off + total > j.cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= j.cap) return;
@@ -211,7 +211,7 @@ __device__ __forceinline__ void batch_small_join(const BatchJoin& j, int4* smem,
     unsigned long long off = 0;
     if (lane == 0) {
       off = atomicAdd(j.d_count, (unsigned long long)total);
-      if (off + total > j.cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+      if (off <= j.cap && off + total > j.cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
     }
     off = __shfl_sync(EJ_FULL_MASK, off, 0) + (incl - c);
     for (int i = first; c && i >= 0; i = nxt[i]) {

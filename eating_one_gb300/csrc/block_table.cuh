@@ -77,7 +77,7 @@ struct BtOut {
     unsigned long long off = 0;
     if ((threadIdx.x & 31u) == 0) {
       off = atomicAdd(cursor, (unsigned long long)n);
-      if (st && off + n > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+      if (st && off <= cap && off + n > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
     }
     return __shfl_sync(EJ_FULL_MASK, off, 0);
   }

@@ -314,7 +314,7 @@ slot_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t, 
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(cursor, total);
-    if (off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (off <= cap && off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= cap) return;
@@ -479,7 +479,7 @@ probe_fused_kernel(const ej_tuple* __restrict__ P, uint64_t nP, ej_table_view t,
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(cursor, total);
-    if (off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (off <= cap && off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= cap) return;

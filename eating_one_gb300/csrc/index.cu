@@ -274,7 +274,7 @@ merge_probe_kernel(const ej_tuple* __restrict__ S, uint64_t nS, ej_table_view t,
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(cursor, total);
-    if (off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (off <= cap && off + total > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= cap) return;
@@ -433,7 +433,7 @@ star_fused_kernel(const ej_tuple* __restrict__ F1, const ej_tuple* __restrict__ 
   unsigned long long off = 0;
   if (lane == 0) {
     off = atomicAdd(cursor, all);
-    if (off + all > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
+    if (off <= cap && off + all > cap) ej_set_status(st, EJ_ERR_CAPACITY, 0u);
   }
   off = __shfl_sync(EJ_FULL_MASK, off, 0);
   if (off >= cap) return;
