@@ -30,7 +30,7 @@
 
 namespace {
 
-constexpr int BX_ITEMS = 4;                              // R rows per thread and tile
+constexpr int BX_ITEMS = 4;                              // R rows per thread and tile (the insert: one, 4 blocks a tile)
 constexpr uint32_t BX_RTILE = 256 * BX_ITEMS;            // R rows per build tile
 constexpr uint64_t BX_MAX_R = 1ull << 26;                // larger joins run as single joins
 
@@ -73,33 +73,24 @@ constexpr uint32_t BX_SMALL_R = 2048;
 
 // ---- build: slot_table.cuh's steps over the tiles of all joins ---------------------
 
-__global__ void __launch_bounds__(256)
+// One row a thread (as slot_insert_kernel, but over tables that L2 does not hold
+// all at once): 32 served requests of 13.3 M R rows, with the clear, 420 us with
+// four rows, 387 with two, 348 with one.
+__global__ void __launch_bounds__(256, 8)
 batch_insert_kernel(const BatchTile* __restrict__ tiles, const BatchJoin* __restrict__ joins,
                     uint32_t* __restrict__ mark, uint2* __restrict__ rank, uint32_t* __restrict__ marked) {
-  const BatchTile d = tiles[blockIdx.x];
+  const BatchTile d = tiles[blockIdx.x / BX_ITEMS];
   const BatchJoin& j = joins[d.join];
-  const int2* R = reinterpret_cast<const int2*>(j.R);
-  const uint32_t n = (uint32_t)j.view.nR, lane = threadIdx.x & 31u;
-  const uint32_t base = d.row0 + (threadIdx.x >> 5) * (32 * BX_ITEMS) + lane;
-  int32_t key[BX_ITEMS];
-  uint32_t hv[BX_ITEMS], any = 0;
-  EjSlotMark m[BX_ITEMS];
-  bool ok[BX_ITEMS];
-#pragma unroll
-  for (int q = 0; q < BX_ITEMS; q++) {
-    ok[q] = base + 32u * q < n;
-    const int2 r = ok[q] ? __ldg(R + base + 32u * q) : make_int2(0, 0);
-    key[q] = r.x;
-    hv[q] = ej_hash32((uint32_t)r.y);
-  }
-  ej_slot_insert<BX_ITEMS>(j.slot, j.view.npairs, key, hv, ok, m);
-#pragma unroll
-  for (int q = 0; q < BX_ITEMS; q++) {
-    if (ok[q]) mark[j.r_row0 + base + 32u * q] = m[q].mark;
-    if (m[q].mark) rank[j.r_row0 + base + 32u * q] = make_uint2(m[q].rank, (uint32_t)m[q].first);
-    any |= m[q].mark;
-  }
-  if (__any_sync(EJ_FULL_MASK, any != 0u) && lane == 0u) *marked = 1u;
+  const uint32_t i = d.row0 + blockIdx.x % BX_ITEMS * 256 + threadIdx.x;
+  const bool ok[1] = {i < (uint32_t)j.view.nR};
+  const int2 r = ok[0] ? __ldg(reinterpret_cast<const int2*>(j.R) + i) : make_int2(0, 0);
+  const int32_t key[1] = {r.x};
+  const uint32_t hv[1] = {ej_hash32((uint32_t)r.y)};
+  EjSlotMark m[1];
+  ej_slot_insert<1>(j.slot, j.view.npairs, key, hv, ok, m);
+  if (ok[0]) mark[j.r_row0 + i] = m[0].mark;
+  if (m[0].mark) rank[j.r_row0 + i] = make_uint2(m[0].rank, (uint32_t)m[0].first);
+  if (__any_sync(EJ_FULL_MASK, m[0].mark != 0u) && (threadIdx.x & 31u) == 0u) *marked = 1u;
 }
 
 // the passes over the marked rows: a few blocks per SM stride over the tiles
@@ -229,8 +220,8 @@ __device__ __forceinline__ void batch_small_join(const BatchJoin& j, int4* smem,
 // large task waits behind them at the end.  (A resident grid pulling tasks
 // from an atomic counter measured slower.)  32 served requests of 13.3 M
 // R rows in all: four segmented radix passes, bucket bounds and this kernel over
-// them 0.46 + 0.05 + 0.73 ms, slots and this kernel 0.42 + 0.55; the call 1.57 ->
-// 1.25 ms.
+// them 0.46 + 0.05 + 0.73 ms, slots and this kernel 0.35 + 0.55; the call 1.57 ->
+// 1.19 ms.
 __global__ void __launch_bounds__(PR_THREADS, 4)
 batch_task_kernel(const BatchJoin* __restrict__ joins, const BatchTask* __restrict__ tasks, ej_dev_status* st) {
   __shared__ int4 smem[PR_WARPS * PW_STAGE_ROWS];  // staging rows, or a small join's table
@@ -287,7 +278,7 @@ static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, uns
     for (uint32_t t = 0; t < nptiles && nR; t += BX_TASK_TILES) tile_tasks.push_back({i, t});
     nr_total += nR;
   }
-  if (tiles.size() > 0x7FFFFFFFull || tile_tasks.size() + small_tasks.size() > 0x7FFFFFFFull)
+  if (tiles.size() > 0x7FFFFFFFull / BX_ITEMS || tile_tasks.size() + small_tasks.size() > 0x7FFFFFFFull)
     return ej_fail(h, EJ_ERR_TOO_LARGE, "batch of %llu R rows is too large", (unsigned long long)nr_total);
 
   // arena layout: first what one copy brings (descriptors, the task list with the
@@ -334,7 +325,7 @@ static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, uns
   if (!tiles.empty()) {
     const uint32_t nt = (uint32_t)tiles.size();
     const unsigned few = std::min<unsigned>(nt, (unsigned)h->num_sms * 8);
-    batch_insert_kernel<<<nt, 256, 0, h->stream>>>(dtiles, djoins, mark, rank, marked);
+    batch_insert_kernel<<<nt * BX_ITEMS, 256, 0, h->stream>>>(dtiles, djoins, mark, rank, marked);
     EJ_TRY(ej_check_launch(h, "batch_insert_kernel"));
     batch_reserve_kernel<<<few, 256, 0, h->stream>>>(dtiles, nt, djoins, mark, rank, hdr, marked);
     EJ_TRY(ej_check_launch(h, "batch_reserve_kernel"));

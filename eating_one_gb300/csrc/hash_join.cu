@@ -185,7 +185,8 @@ __device__ __forceinline__ void ej_prefetch_tile(const void* base, uint64_t w, u
 
 // ---- slot tables (slot_table.cuh) --------------------------------------------------
 
-constexpr int SLOT_ITEMS = 4;  // rows per thread and step of the build's kernels
+constexpr int SLOT_INSERT_ITEMS = 2;  // rows per thread of the insert
+constexpr int SLOT_ITEMS = 4;         // rows per thread and step of the passes over the marked rows
 
 struct SlotHeader {
   uint32_t marked;  // some row was marked: a key has several rows
@@ -194,25 +195,30 @@ struct SlotHeader {
 };
 static_assert(sizeof(SlotHeader) <= EJ_SLOT_HEADER_BYTES, "slot table header");
 
-// every row to its key's slot, or marked
-__global__ void __launch_bounds__(256, 4)
+// every row to its key's slot, or marked.  Two rows a thread and 48 warps an SM: a
+// warp is done with the longest of 64 walks (2^20 unique keys, the whole build: 47
+// us with four rows a thread and 32 warps, 44 with two, 42 with one; 2 M rows of
+// eight a key 109, 111 and 126, the chain of a repeated key's updates wanting
+// rows side by side).
+__global__ void __launch_bounds__(256, 6)
 slot_insert_kernel(const int2* __restrict__ R, uint32_t n, unsigned long long* __restrict__ slot, uint32_t npairs,
                    uint32_t* __restrict__ mark, uint2* __restrict__ rank, SlotHeader* hdr) {
-  const uint64_t base = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 * SLOT_ITEMS) + (threadIdx.x & 31u);
-  int32_t key[SLOT_ITEMS];
-  uint32_t hv[SLOT_ITEMS], any = 0;
-  EjSlotMark m[SLOT_ITEMS];
-  bool ok[SLOT_ITEMS];
+  constexpr int SI = SLOT_INSERT_ITEMS;
+  const uint64_t base = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 * SI) + (threadIdx.x & 31u);
+  int32_t key[SI];
+  uint32_t hv[SI], any = 0;
+  EjSlotMark m[SI];
+  bool ok[SI];
 #pragma unroll
-  for (int j = 0; j < SLOT_ITEMS; j++) {
+  for (int j = 0; j < SI; j++) {
     ok[j] = base + 32 * j < n;
     const int2 r = ok[j] ? __ldg(R + base + 32 * j) : make_int2(0, 0);
     key[j] = r.x;
     hv[j] = ej_hash32((uint32_t)r.y);
   }
-  ej_slot_insert<SLOT_ITEMS>(slot, npairs, key, hv, ok, m);
+  ej_slot_insert<SI>(slot, npairs, key, hv, ok, m);
 #pragma unroll
-  for (int j = 0; j < SLOT_ITEMS; j++) {
+  for (int j = 0; j < SI; j++) {
     if (ok[j]) mark[base + 32 * j] = m[j].mark;
     if (m[j].mark) rank[base + 32 * j] = make_uint2(m[j].rank, (uint32_t)m[j].first);
     any |= m[j].mark;
@@ -695,7 +701,7 @@ ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple
     uint2* rank = reinterpret_cast<uint2*>(ej_arena_at(h, tp.rank_off));
     const int2* R2 = reinterpret_cast<const int2*>(R);
     const uint32_t n = (uint32_t)tp.nR;
-    const unsigned blocks = (n + 256 * SLOT_ITEMS - 1) / (256 * SLOT_ITEMS);
+    const unsigned blocks = (n + 256 * SLOT_INSERT_ITEMS - 1) / (256 * SLOT_INSERT_ITEMS);
     const unsigned few = std::min<unsigned>((n + 255) / 256, (unsigned)h->num_sms * 8);
     if (n > EJ_SLOT_DIRECT_ROWS) {
       EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES, h->stream));

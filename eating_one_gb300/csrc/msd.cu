@@ -382,11 +382,12 @@ msd_local_kernel(const ej_tuple* __restrict__ in, ej_tuple* __restrict__ tmp, co
 // own words).  Random slot updates through L2 (slot_insert_kernel) run at 40 to
 // 60 G rows/s; here they stay in shared memory and the slots leave in
 // coalesced stores.  Bound by the shared memory's compare-and-swaps (random
-// 8-byte words, a warp's longest walk of about five rounds): 2^24 rows in 193 to
-// 200 us, 84 G rows/s, where the local sort and the directory or bucket launches
-// took 230 to 250; four CTAs an SM with the runs' cursors in shared memory too
-// were level with six.  The build of a 2^24-row table in all: 446 us (432 with
-// the sort), and the probes of unique keys then take 665 us instead of 1052.
+// 8-byte words, a warp's longest walk of some rounds): 2^24 rows in 178 us, where
+// the local sort and the directory or bucket launches took 230 to 250 (200 with
+// walks that all begin with a pair's first slot; four CTAs an SM with the runs'
+// cursors in shared memory too were level with six).  The build of a 2^24-row
+// table in all: 420 us (432 with the sort), and the probes of unique keys then take
+// 665 us instead of 1052.
 constexpr uint32_t SB_PER = 12;           // rows per thread kept in registers (groups up to 3072 rows)
 constexpr uint32_t SB_SPILLED = 0xFFFFu;  // a row's slot within its group (of 4098 at most): walked past the end
 constexpr uint32_t SB_NONE = 0xFFFEu;     // no row
@@ -398,7 +399,7 @@ __device__ __forceinline__ uint32_t sb_claim(unsigned long long* slot, uint32_t 
                                              uint32_t end, uint32_t* rank) {
   const uint32_t y = hv << 1 | 1u;
   *rank = 0u;
-  for (uint32_t s = 2u * (ej_home_pair(hv, npairs) - p0); s < end; s++) {
+  for (uint32_t s = 2u * (ej_home_pair(hv, npairs) - p0) + (hv & 1u); s < end; s = ej_next_slot(s, hv, 0xFFFFFFFFu)) {
     const unsigned long long old = atomicCAS(slot + s, 0ull, (unsigned long long)y << 32 | 1u);
     if (old == 0ull) return s;
     if ((uint32_t)(old >> 32) == y) {
@@ -540,7 +541,7 @@ spill_insert_kernel(const uint2* __restrict__ spill, const uint32_t* __restrict_
       }
       if (q >= npairs) q -= npairs;
     }
-    const uint32_t at[1] = {2u * (q < npairs ? q : q - npairs)};
+    const uint32_t at[1] = {q < npairs ? q : q - npairs};
     EjSlotMark m[1];
     ej_slot_insert<1, true>(slot, npairs, key, hv, ok, m, at);
     if (ok[0]) {
