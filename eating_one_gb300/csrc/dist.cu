@@ -33,8 +33,9 @@
 // (a warp instruction takes 16 cycles, however few lanes are active), so the
 // candidates that pass the screen are collected and tested by full warps: at
 // once, most steps of a probe warp would take the double path for one or two
-// lanes.  Two of an S point's cells may share a bucket, which is then looked
-// at once: every R point lies in one bucket, so no pair comes twice.
+// lanes.  Two of an S point's cells may share a bucket (when its reach spans
+// three cells somewhere), which is then looked at once: every R point lies in one
+// bucket, so no pair comes twice.
 //
 // Launches: cells (histogram with the points' ranks in their buckets), scan,
 // placement, probe.  A probe warp takes 32 S points: each lane finds its point's
@@ -46,10 +47,11 @@
 // per-thread counters.
 // Both calls of a join (count, then rows): 2^19 x 2^19 2-D points far apart by
 // all pairs 37.7 ms, by the grid with a lane per S point and the predicate in
-// the step 0.356 ms, here 0.249 (the
-// probe 87 -> 49 us); 100 003 x 150 001 points of a 3-D box with
-// about three matches each 77.7, 1.04 and 0.242 ms (the probe
-// 430 -> 55 us).
+// the step 0.356 ms, here 0.237 (the probe 87 -> 46 us; 50 when the buckets of a
+// point's cells were unrelated and had to be compared); 100 003 x 150 001 points
+// of a 3-D box with about three matches each 77.7, 1.04 and 0.221 ms (the probe
+// 430 -> 53 us).  Bound by the chain of dependent loads and shuffles per S point
+// (half of the warps resident, the issue slots 30% busy).
 #include <float.h>
 #include <math.h>
 
@@ -114,19 +116,27 @@ __device__ __forceinline__ double dist_clamp(double x) {
   return (b & 0x7FFFFFFFFFFFFFFFull) == 0x7FF0000000000000ull ? __longlong_as_double((long long)(b - 1)) : x;
 }
 
-// the bucket of a cell: top `bits` bits of a multiplicative hash of its numbers
+// the bucket of a cell: the cells of a block of two per dimension are neighbours,
+// told by their numbers' lowest bits, and a multiplicative hash places the block.
+// So the 2^D cells of a point whose reach spans two per dimension never share a
+// bucket, and most of them lie next to each other.
 template <int D>
 __device__ __forceinline__ uint32_t dist_bucket(const long long (&c)[D], uint32_t bits) {
-  unsigned long long x = (unsigned long long)c[0] * 0x9E3779B97F4A7C15ull;
+  unsigned long long x = (unsigned long long)(c[0] >> 1) * 0x9E3779B97F4A7C15ull;
+  uint32_t low = (uint32_t)c[0] & 1u;
 #pragma unroll
   for (int i = 1; i < D; i++) {
     x ^= x >> 32;
-    x = (x + (unsigned long long)c[i]) * 0xD1342543DE82EF95ull;
+    x = (x + (unsigned long long)(c[i] >> 1)) * 0xD1342543DE82EF95ull;
+    low |= ((uint32_t)c[i] & 1u) << i;
   }
   x ^= x >> 32;
   x *= 0x9E3779B97F4A7C15ull;
-  return (uint32_t)(x >> (64u - bits));
+  return (uint32_t)(x >> (64u - (bits - D))) << D | low;
 }
+
+// a / n; cells span one or two per dimension nearly always
+__device__ __forceinline__ uint32_t dist_div(uint32_t a, uint32_t n) { return n <= 2u ? a >> (n - 1u) : a / n; }
 
 // the reference's predicate, operation by operation
 template <int D>
@@ -327,16 +337,16 @@ dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S
         const uint32_t k = first + g;
         uint32_t p = 0, end = 0, b = 0xFFFFFFFFu;
         if (k < cells) {
-          const uint32_t k1 = k / n0;
+          const uint32_t k1 = dist_div(k, n0);
           long long c[D];
           c[0] = c0[0] + (k - k1 * n0);
-          const uint32_t k2 = k1 / n1;
+          const uint32_t k2 = dist_div(k1, n1);
           c[1] = c0[1] + (k1 - k2 * n1);
           if (D == 3) c[D - 1] = c0[D - 1] + k2;
           b = dist_bucket<D>(c, bits);
-          // the point's earlier cells in this bucket: in this round of G
-          // cells (below), and in the rounds before, which only points whose
-          // reach spans three cells or more somewhere have
+          // the point's earlier cells in this bucket, which only points whose
+          // reach spans three cells or more somewhere can have: in this round of
+          // G cells (below), and in the rounds before
           for (uint32_t e = 0; e < first; e++) {
             const uint32_t e1 = e / n0, e2 = e1 / n1;
             long long f[D];
@@ -346,7 +356,9 @@ dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S
             if (dist_bucket<D>(f, bits) == b) b = 0xFFFFFFFFu;
           }
         }
-        const unsigned same = __match_any_sync(EJ_FULL_MASK, b) & group & ej_lanemask_lt();
+        unsigned same = 0;
+        if (__any_sync(EJ_FULL_MASK, n0 > 2u || n1 > 2u || n2 > 2u))
+          same = __match_any_sync(EJ_FULL_MASK, b) & group & ej_lanemask_lt();
         if (b != 0xFFFFFFFFu && same == 0) {
           p = __ldg(start + b);
           end = __ldg(start + b + 1);
