@@ -484,18 +484,16 @@ def config_lines(eng, peaks: dict, steps: int, distance: bool) -> list[dict]:
     lines.append({"config": "C1 hash join R=2^20 unique x S=2^22 (count, then write)", "ms": round(ms, 4),
                   "rows": n, "tuples_per_s": (R.shape[0] + S.shape[0]) / (ms / 1000),
                   "roofline": hbm(24 * (R.shape[0] + S.shape[0]) + 16 * n, ms)})
-    # C2: block nested loop, all 2^36 pairs
+    # C2: block nested loop, 2^36 pairs (found by hashed blocks of R)
     w = workload("c2")
     R, S = eng.generate(w["R"]), eng.generate(w["S"])
     n = eng.count("bnl", R, S)
     out = torch.empty((n, 4), dtype=torch.int32, device="cuda")
     ms = timed(lambda: eng.join("bnl", R, S, out=out), max(3, steps // 4))
     pairs = R.shape[0] * S.shape[0]
-    issue = props.multi_processor_count * 128 * 2.07e9  # one INT32 lane-instruction per clock per lane
     lines.append({"config": "C2 BNLJ R=2^16 x S=2^20, keys uniform in [0, 2^16)", "ms": round(ms, 4), "rows": n,
                   "pair_compares_per_s": pairs / (ms / 1000),
-                  "roofline": {"bound": "int32 issue", "peak_lane_ops_per_s": issue,
-                               "frac_at_one_op_per_compare": round(pairs / (ms / 1000) / issue, 4)},
+                  "roofline": hbm(8 * (R.shape[0] + S.shape[0]) + 16 * n, ms),
                   "reference_gpu_log": "2^20 x 2^16 in 1.483 s (nestLoopJoin, sm_35)"})
     del out
     # C4: index joins, outer join, star join
@@ -532,12 +530,11 @@ def config_lines(eng, peaks: dict, steps: int, distance: bool) -> list[dict]:
     del out, t
     if not distance:
         return lines
-    # distance joins: all 2^38 pairs of 2^19 x 2^19 reference-shaped points, radius 1
+    # distance joins: the 2^38 pairs of 2^19 x 2^19 reference-shaped points, radius 1 (found by a grid)
     from eating_one_gb300.native import point_result_dtype
     from eating_one_gb300.workloads import distance_workload
     from oracle import oracle as O
 
-    fp32 = props.multi_processor_count * 128 * 2.07e9  # one FP32 lane-instruction per clock per lane
     for name in ("d2", "d3"):
         dims, Rp, Sp = distance_workload(name)
         dR, dS = eng.points_to_device(Rp), eng.points_to_device(Sp)
@@ -553,8 +550,7 @@ def config_lines(eng, peaks: dict, steps: int, distance: bool) -> list[dict]:
         cpu_s = time.perf_counter() - t0
         lines.append({"config": "%dD distance join R=2^19 x S=2^19 points, radius 1, 10%% copies" % dims,
                       "ms": round(ms, 4), "rows": n, "pairs_per_s": pairs / (ms / 1000),
-                      "roofline": {"bound": "fp32 issue", "peak_lane_ops_per_s": fp32,
-                                   "frac_at_two_ops_per_pair": round(2 * pairs / (ms / 1000) / fp32, 4)},
+                      "roofline": hbm((8 + 8 * dims) * (len(Rp) + len(Sp)) + out.nbytes, ms),
                       "cpu_baseline": {"pairs_per_s": len(Rp) * len(s_sample) / cpu_s, "cores": threads,
                                        "kind": "port", "sample": "R=2^19 x the first 1024 S points"},
                       "reference_cpu_log": "2-D 2^19 x 2^19 in 3718 s (complex_block/2d_cpu/nohup.out)"})
