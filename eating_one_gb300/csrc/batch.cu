@@ -271,6 +271,7 @@ static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, uns
       continue;
     }
     b.view.npairs = (uint32_t)nR + 1u;  // at most half full
+    b.view.run_words = (uint32_t)ej_slot_run_words(nR);
     pairs += b.view.npairs;
     run_words += (ej_slot_run_bytes(nR) / sizeof(int32_t) + 3) & ~uint64_t(3);
     for (uint64_t r = 0; r < nR; r += BX_RTILE) tiles.push_back({i, (uint32_t)r});

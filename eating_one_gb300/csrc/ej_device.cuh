@@ -53,13 +53,18 @@ __device__ __forceinline__ void ej_clear_words(unsigned long long* p, uint64_t n
   if (i < n) p[i] = 0ull;
 }
 
-// Record the first device error (later errors keep the first one).  Kernels that
+// Record the first device error (later errors keep the first one, but a wait that
+// gave up replaces a short capacity, which is no error of the device).  Kernels that
 // reserve rows with an atomic add report the capacity from the one range that
 // crosses it: an atomic on this word by every warp past it made the calls that
 // only count slower (the star join of 2^25 facts, sized by a first call, 1689 us
 // instead of 1401; the outer join of 2^25 probes 1242 instead of 1136).
 __device__ __forceinline__ void ej_set_status(ej_dev_status* st, unsigned int code, unsigned int info) {
-  if (st && atomicCAS(&st->code, 0u, code) == 0u) st->info = info;
+  if (!st) return;
+  const unsigned int old = atomicCAS(&st->code, 0u, code);
+  if (old == 0u || (code == EJ_ERR_TIMEOUT && old == EJ_ERR_CAPACITY &&
+                    atomicCAS(&st->code, (unsigned int)EJ_ERR_CAPACITY, code) == EJ_ERR_CAPACITY))
+    st->info = info;
 }
 
 // Lanes of the warp whose BITS-bit digit equals this lane's, restricted to

@@ -248,6 +248,7 @@ struct ej_table_view {
   uint32_t dir_packed = 0;             // entries {hash, start << 5 | run length} (tables under 2^27 rows)
   const uint4* pair = nullptr;       // (hash, slot tables) [npairs] pairs of slots
   uint32_t npairs = 0;
+  uint32_t run_words = 0;            // words of rkey (slot tables)
   const void* vbuckets = nullptr;    // (sorted) device EjValueBuckets {vmin, vmax, vshift} of `bucket`
   uint64_t nR = 0;
   uint32_t hb = 1;

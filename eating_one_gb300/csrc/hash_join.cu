@@ -605,9 +605,10 @@ bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {
   return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table != EJ_TABLE_FORMAT_DIRECTORY;
 }
 
-size_t ej_slot_run_bytes(uint64_t nR) {
-  return ej_table_col_bytes(nR + nR / 31 + 1 + (nR > EJ_SLOT_DIRECT_ROWS ? 4ull * EJ_MSD_GROUPS : 0));
+uint64_t ej_slot_run_words(uint64_t nR) {
+  return nR + nR / 31 + 1 + (nR > EJ_SLOT_DIRECT_ROWS ? 4ull * EJ_MSD_GROUPS : 0);
 }
+size_t ej_slot_run_bytes(uint64_t nR) { return ej_table_col_bytes(ej_slot_run_words(nR)); }
 
 size_t ej_table_aux_bytes(const ej_table_plan_t& tp) {
   if (tp.slots) return EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4) + ej_slot_run_bytes(tp.nR);
@@ -725,6 +726,7 @@ ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple
     view->rkey = runs;
     view->pair = reinterpret_cast<const uint4*>(slot);
     view->npairs = tp.npairs;
+    view->run_words = (uint32_t)ej_slot_run_words(tp.nR);
     return EJ_OK;
   }
   // LSD passes over the 32-bit key (hash32(val), or the order-preserving image

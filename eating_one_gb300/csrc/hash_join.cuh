@@ -86,8 +86,9 @@ struct ej_table_knobs {
   int table = EJ_TABLE_FORMAT_PLANNER;
 };
 ej_table_knobs ej_tuned_table_knobs(const ej_handle* h, uint64_t nR);
-// bytes of a slot table's runs: every row, a count for each of 31 rows and more,
-// and the alignment of the bucket groups' parts
+// words (and bytes) of a slot table's runs: every row, a count for each of 31
+// rows and more, and the alignment of the bucket groups' parts
+uint64_t ej_slot_run_words(uint64_t nR);
 size_t ej_slot_run_bytes(uint64_t nR);
 // whether a hash table of nR rows is a slot table
 bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k);

@@ -54,12 +54,20 @@ struct MsdSegments {
 
 __global__ void __launch_bounds__(256) msd_segments_kernel(const uint32_t* __restrict__ offs1, uint32_t ntiles1,
                                                            uint64_t n, MsdSegments* __restrict__ seg) {
-  __shared__ uint32_t tmp[256 / 32 + 1];
+  __shared__ uint32_t tmp[256 / 32 + 1], first[256];
   const uint32_t d = threadIdx.x;
-  // clamped so that offsets left too small by a timed-out scan still give
-  // ordered segments inside [0, n)
-  const uint32_t s = min(offs1[(uint64_t)d * ntiles1], (uint32_t)n);
-  const uint32_t e = max(s, d < 255 ? min(offs1[(uint64_t)(d + 1) * ntiles1], (uint32_t)n) : (uint32_t)n);
+  // clamped and made monotone, so that offsets left too small by a timed-out scan
+  // still give ordered segments inside [0, n), of no more tiles than planned
+  first[d] = min(offs1[(uint64_t)d * ntiles1], (uint32_t)n);
+  for (uint32_t step = 1; step < 256; step <<= 1) {
+    __syncthreads();
+    const uint32_t before = d >= step ? first[d - step] : 0u;
+    __syncthreads();
+    first[d] = max(first[d], before);
+  }
+  __syncthreads();
+  const uint32_t s = first[d];
+  const uint32_t e = d < 255 ? first[d + 1] : (uint32_t)n;
   const uint32_t tiles = (e - s + EJ_RX_TILE - 1) / EJ_RX_TILE;
   uint32_t total;
   const uint32_t base = ej_block_exclusive_sum<256, uint32_t>(tiles, tmp, &total);
@@ -394,12 +402,17 @@ constexpr uint32_t SB_NONE = 0xFFFEu;     // no row
 constexpr int SB_BLOCKS = 6;  // CTAs per SM
 
 // row of hash hv into the group's array (pairs p0 ..., `end` slots): its slot, and
-// its rank among its key's rows
+// its rank among its key's rows.  No slot for a row of another group: there is
+// none unless a scan of the passes gave up waiting and left wrong bounds, which
+// may then overlap; taking only its own rows, each once, a group stays within
+// its run words, and the spilled rows within their list.
 __device__ __forceinline__ uint32_t sb_claim(unsigned long long* slot, uint32_t hv, uint32_t npairs, uint32_t p0,
                                              uint32_t end, uint32_t* rank) {
   const uint32_t y = hv << 1 | 1u;
   *rank = 0u;
-  for (uint32_t s = 2u * (ej_home_pair(hv, npairs) - p0) + (hv & 1u); s < end; s = ej_next_slot(s, hv, 0xFFFFFFFFu)) {
+  const uint32_t home = 2u * (ej_home_pair(hv, npairs) - p0);
+  if (home >= end) return SB_NONE;
+  for (uint32_t s = home + (hv & 1u); s < end; s = ej_next_slot(s, hv, 0xFFFFFFFFu)) {
     const unsigned long long old = atomicCAS(slot + s, 0ull, (unsigned long long)y << 32 | 1u);
     if (old == 0ull) return s;
     if ((uint32_t)(old >> 32) == y) {
@@ -432,7 +445,8 @@ __device__ __forceinline__ void sb_place(unsigned long long* slot, uint32_t s, u
 __global__ void __launch_bounds__(LS_THREADS, SB_BLOCKS)
 msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ bstart, uint32_t g, uint32_t npairs,
                  uint32_t pp, uint4* __restrict__ pair, int32_t* __restrict__ rkey, uint32_t* __restrict__ gcursor,
-                 uint2* __restrict__ spill, uint32_t* __restrict__ nspill, uint32_t* __restrict__ ranks) {
+                 uint2* __restrict__ spill, uint32_t* __restrict__ nspill, uint32_t* __restrict__ ranks,
+                 const ej_dev_status* __restrict__ st) {
   extern __shared__ __align__(16) unsigned char sb_smem_raw[];
   unsigned long long* slot = reinterpret_cast<unsigned long long*>(sb_smem_raw);
   __shared__ uint32_t s_runs;
@@ -440,7 +454,10 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
   // bounds clamped to [0, n) and ordered (they are, unless a scan timed out)
   const uint32_t n = bstart[MSD_BUCKETS];
   const uint32_t lo = min(bstart[blockIdx.x << g], n);
-  const uint32_t m = max(min(bstart[(blockIdx.x + 1u) << g], n), lo) - lo;
+  uint32_t m = max(min(bstart[(blockIdx.x + 1u) << g], n), lo) - lo;
+  // a scan of the passes gave up waiting: the call reports it, and the bounds and
+  // rows are not to be relied on, so the table stays empty
+  if (st->code == EJ_ERR_TIMEOUT) m = 0u;
   // the group's words begin at a multiple of four, so that runs of four rows
   // throughout (one 16-byte load each) stay aligned
   const uint32_t words0 = ((lo + lo / 31u) & ~3u) + 4u * blockIdx.x;
@@ -643,7 +660,7 @@ ej_status ej_msd_slots(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, e
   EJ_CUDA(h, cudaFuncSetAttribute(msd_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   uint2* spill = reinterpret_cast<uint2*>(tmp_a);
   msd_slots_kernel<<<groups, LS_THREADS, smem, h->stream>>>(tmp_b, bstart, g, npairs, pp, pair, rkey, gcursor, spill,
-                                                           nspill, mark);
+                                                           nspill, mark, h->d_status);
   EJ_TRY(ej_check_launch(h, "msd_slots_kernel"));
   // the spilled rows' marks (mark held large groups' ranks before); their ranks
   // in tmp_b, whose rows are in the table now

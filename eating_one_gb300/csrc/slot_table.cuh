@@ -51,9 +51,10 @@ struct EjSlotTable {
   const uint4* pair;    // [npairs]
   const int32_t* rkey;  // runs of the keys with several rows
   uint32_t npairs;
+  uint32_t run_words;   // words of rkey
 };
 
-__device__ __forceinline__ EjSlotTable ej_slots_of(const ej_table_view& t) { return {t.pair, t.rkey, t.npairs}; }
+__device__ __forceinline__ EjSlotTable ej_slots_of(const ej_table_view& t) { return {t.pair, t.rkey, t.npairs, t.run_words}; }
 
 __device__ __forceinline__ uint32_t ej_home_pair(uint32_t hash, uint32_t npairs) { return __umulhi(hash, npairs); }
 
@@ -176,6 +177,13 @@ __device__ __forceinline__ void ej_slot_reserve(uint2* __restrict__ slot, const 
 
 __device__ __forceinline__ bool ej_pair_full(const uint4& q) { return (q.x | q.y) != 0u && (q.z | q.w) != 0u; }
 
+// Rows of the run of 31 rows and more that begins at rkey[lo].  Never past the
+// array, also when a scan of the build's passes gave up waiting (the call then
+// reports it) and bucket groups wrote over each other's runs.
+__device__ __forceinline__ uint32_t ej_run_length(const int32_t* rkey, uint32_t lo, uint32_t run_words) {
+  return min((uint32_t)__ldg(rkey + lo - 1), run_words - lo);
+}
+
 // The matches of N probe values (ok[j] false: none): c[j] rows, the first at
 // rkey[lo[j]], or lo[j] = INLINE_RUN and c[j] = 1: the row with key key[j].
 template <int N>
@@ -221,7 +229,7 @@ __device__ __forceinline__ void ej_slot_find(const EjSlotTable& t, const int32_t
   if (longest == 31u) {
 #pragma unroll
     for (int j = 0; j < N; j++)
-      if (c[j] == 31u) c[j] = (uint32_t)__ldg(t.rkey + lo[j] - 1);
+      if (c[j] == 31u) c[j] = ej_run_length(t.rkey, lo[j], t.run_words);
   }
 }
 
@@ -366,7 +374,7 @@ __device__ __forceinline__ void ej_slot_write(const ej_tuple* __restrict__ P, co
   if (__any_sync(EJ_FULL_MASK, escape)) {  // runs of 31 rows and more: their lengths precede them
 #pragma unroll
     for (int j = 0; j < PR_ITEMS; j++)
-      if (p.cnt[j] == EJ_PACKED_ESCAPE) p.cnt[j] = (uint32_t)__ldg(t.rkey + p.lo[j] - 1);
+      if (p.cnt[j] == EJ_PACKED_ESCAPE) p.cnt[j] = ej_run_length(t.rkey, p.lo[j], t.run_words);
   }
   ej_slot_emit(p, key, t, off, out, cap, stage);
 }
