@@ -468,6 +468,11 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
   // 1. every row's slot, claimed or counted in; rows past the group's end listed
   int32_t key[SB_PER];
   uint32_t at[SB_PER];  // slot | rank << 16
+#pragma unroll
+  for (uint32_t q = 0; q < SB_PER; q++) {  // (a group may have no rows)
+    key[q] = 0;
+    at[q] = SB_NONE;
+  }
   const bool big = m > SB_PER * LS_THREADS;
   for (uint32_t j0 = 0; j0 < m; j0 += SB_PER * LS_THREADS) {
 #pragma unroll

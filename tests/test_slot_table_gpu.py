@@ -8,6 +8,8 @@ import numpy as np
 import pytest
 import torch
 
+from eating_one_gb300 import native
+from eating_one_gb300.engine import JoinError
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -97,3 +99,42 @@ def test_build_sizes(engine):
         assert rows.shape[0] == hit == engine.count("hash", R, S)
         assert bool((R[rows[:, 0].long(), 1] == rows[:, 1]).all()) and bool((rows[:, 1] == rows[:, 3]).all())
         assert bool((S[rows[:, 2].long(), 1] == rows[:, 3]).all()) and rows[:, 2].unique().numel() == hit
+
+
+@pytest.mark.parametrize("keys", [1, 50, 3000])
+def test_groups_without_rows(engine, keys):
+    """More than 2^21 rows of few keys: most bucket groups of the large build are empty, others
+    far larger than shared memory."""
+    rng = np.random.default_rng(keys)
+    n = (1 << 21) + 1000
+    R = _rel(rng.integers(0, keys, n) * 7919, 0, rng)
+    S = _rel(np.concatenate([np.arange(20) * 7919 % (7919 * keys), rng.integers(0, 1 << 30, 70000)]), 1 << 23, rng)
+    Rd, Sd = torch.from_numpy(R).cuda(), torch.from_numpy(S).cuda()
+    got = engine.join("left_outer", Rd, Sd)
+    assert np.array_equal(O.canon(got.cpu().numpy()), O.canon(O.left_outer_join(R, S)))
+    want = O.canon(O.hash_join(R, S))
+    assert np.array_equal(O.canon(engine.hash_join(Rd, Sd).cpu().numpy()), want)
+    out = torch.empty((len(want), 4), dtype=torch.int32, device="cuda")
+    assert np.array_equal(O.canon(engine.hash_join(Rd, Sd, out=out).cpu().numpy()), want)
+
+
+def test_build_survives_a_scan_that_gave_up(engine):
+    """With no time to wait, scans of the large build's passes give up: the joins report it or
+    are right, and the same handle is right afterwards."""
+    rng = np.random.default_rng(17)
+    rv = np.concatenate([rng.integers(0, 1 << 20, (1 << 21) + 77), np.repeat(5, 300)])
+    R, S = _rel(rv, 0, rng), _rel(rng.integers(0, 1 << 21, 100001), 1 << 23, rng)
+    Rd, Sd = torch.from_numpy(R).cuda(), torch.from_numpy(S).cuda()
+    want = O.canon(O.hash_join(R, S))
+    out = torch.empty((len(want), 4), dtype=torch.int32, device="cuda")
+    engine.set_option("wait_limit_ns", 0)
+    try:
+        for _ in range(3):
+            try:
+                got = engine.hash_join(Rd, Sd, out=out)
+                assert np.array_equal(O.canon(got.cpu().numpy()), want)
+            except JoinError as e:
+                assert e.status == native.EJ_ERR_TIMEOUT, e
+    finally:
+        engine.set_option("wait_limit_ns", -1)
+    assert np.array_equal(O.canon(engine.hash_join(Rd, Sd, out=out).cpu().numpy()), want)
