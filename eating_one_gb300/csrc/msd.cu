@@ -397,26 +397,27 @@ msd_local_kernel(const ej_tuple* __restrict__ in, ej_tuple* __restrict__ tmp, co
 // table in all: 420 us (432 with the sort), and the probes of unique keys then take
 // 665 us instead of 1052.
 constexpr uint32_t SB_PER = 12;           // rows per thread kept in registers (groups up to 3072 rows)
+constexpr uint32_t SB_BIG = 8;            // rows per thread and step of larger groups
 constexpr uint32_t SB_SPILLED = 0xFFFFu;  // a row's slot within its group (of 4098 at most): walked past the end
 constexpr uint32_t SB_NONE = 0xFFFEu;     // no row
 constexpr int SB_BLOCKS = 6;  // CTAs per SM
 
-// row of hash hv into the group's array (pairs p0 ..., `end` slots): its slot, and
-// its rank among its key's rows.  No slot for a row of another group: there is
+// `rows` rows of hash hv into the group's array (pairs p0 ..., `end` slots): their
+// slot, and the first one's rank among their key's rows.  No slot for a row of another group: there is
 // none unless a scan of the passes gave up waiting and left wrong bounds, which
 // may then overlap; taking only its own rows, each once, a group stays within
 // its run words, and the spilled rows within their list.
 __device__ __forceinline__ uint32_t sb_claim(unsigned long long* slot, uint32_t hv, uint32_t npairs, uint32_t p0,
-                                             uint32_t end, uint32_t* rank) {
+                                             uint32_t end, uint32_t* rank, uint32_t rows = 1u) {
   const uint32_t y = hv << 1 | 1u;
   *rank = 0u;
   const uint32_t home = 2u * (ej_home_pair(hv, npairs) - p0);
   if (home >= end) return SB_NONE;
   for (uint32_t s = home + (hv & 1u); s < end; s = ej_next_slot(s, hv, 0xFFFFFFFFu)) {
-    const unsigned long long old = atomicCAS(slot + s, 0ull, (unsigned long long)y << 32 | 1u);
+    const unsigned long long old = atomicCAS(slot + s, 0ull, (unsigned long long)y << 32 | rows);
     if (old == 0ull) return s;
     if ((uint32_t)(old >> 32) == y) {
-      *rank = atomicAdd(reinterpret_cast<uint32_t*>(slot + s), 1u);
+      *rank = atomicAdd(reinterpret_cast<uint32_t*>(slot + s), rows);
       return s;
     }
   }
@@ -474,10 +475,36 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
     at[q] = SB_NONE;
   }
   const bool big = m > SB_PER * LS_THREADS;
-  for (uint32_t j0 = 0; j0 < m; j0 += SB_PER * LS_THREADS) {
+  // more rows than the registers hold: many of few keys, so the rows of a key in a
+  // warp go together, eight steps' loads at a time (a count of 3 M rows of one key
+  // 12.4 ms when each row claims for itself, 5.8 here, 11.0 with the sorted table;
+  // 2^24 rows of 50 keys 2.76, 1.22 and 2.91)
+  for (uint32_t j0 = 0; big && j0 < m; j0 += SB_BIG * LS_THREADS) {
+    int2 r[SB_BIG];
+#pragma unroll
+    for (uint32_t q = 0; q < SB_BIG; q++) {
+      const uint32_t j = j0 + t + q * LS_THREADS;
+      r[q] = j < m ? __ldcs(rows + j) : make_int2(0, 0);
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < SB_BIG; q++) {
+      const uint32_t j = j0 + t + q * LS_THREADS;
+      const uint32_t hv = ej_hash32((uint32_t)r[q].y);
+      const unsigned peers = __match_any_sync(EJ_FULL_MASK, hv) & __ballot_sync(EJ_FULL_MASK, j < m);
+      const int leader = peers ? __ffs(peers) - 1 : 0;
+      uint32_t s = SB_NONE, rank = 0;
+      if (j < m && (int)lane == leader) s = sb_claim(slot, hv, npairs, p0, end, &rank, __popc(peers));
+      s = __shfl_sync(EJ_FULL_MASK, s, leader);
+      rank = __shfl_sync(EJ_FULL_MASK, rank, leader) + __popc(peers & ej_lanemask_lt());
+      if (j >= m) continue;
+      if (s == SB_SPILLED) spill[atomicAdd(nspill, 1u)] = make_uint2((uint32_t)r[q].x, (uint32_t)r[q].y);
+      ranks[lo + j] = rank;
+    }
+  }
+  if (!big) {
 #pragma unroll
     for (uint32_t q = 0; q < SB_PER; q++) {  // the loads together
-      const uint32_t j = j0 + t + q * LS_THREADS;
+      const uint32_t j = t + q * LS_THREADS;
       const int2 r = j < m ? __ldcs(rows + j) : make_int2(0, 0);
       key[q] = r.x;
       at[q] = (uint32_t)r.y;
@@ -486,13 +513,13 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
     // walks advancing together took 2.5 times the instructions: 464 us at 2^24)
 #pragma unroll
     for (uint32_t q = 0; q < SB_PER; q++) {
-      const uint32_t j = j0 + t + q * LS_THREADS, val = at[q];
+      const uint32_t j = t + q * LS_THREADS, val = at[q];
       at[q] = SB_NONE;
       if (j >= m) continue;
       uint32_t rank;
       const uint32_t s = sb_claim(slot, ej_hash32(val), npairs, p0, end, &rank);
       if (s == SB_SPILLED) spill[atomicAdd(nspill, 1u)] = make_uint2((uint32_t)key[q], val);
-      if (big) ranks[lo + j] = rank; else at[q] = s | rank << 16;
+      at[q] = s | rank << 16;
     }
   }
   __syncthreads();
@@ -520,10 +547,21 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
     for (uint32_t q = 0; q < SB_PER; q++)
       if ((at[q] & 0xFFFFu) < SB_NONE) sb_place(slot, at[q] & 0xFFFFu, at[q] >> 16, key[q], rkey);
   } else {
-    for (uint32_t j = t; j < m; j += LS_THREADS) {
-      const int2 r = __ldg(rows + j);
-      const uint32_t s = sb_find(slot, ej_hash32((uint32_t)r.y), npairs, p0, end);
-      if (s != SB_SPILLED) sb_place(slot, s, ranks[lo + j], r.x, rkey);
+    for (uint32_t j0 = t; j0 < m; j0 += SB_BIG * LS_THREADS) {
+      int2 r[SB_BIG];
+      uint32_t rank[SB_BIG];
+#pragma unroll
+      for (uint32_t q = 0; q < SB_BIG; q++) {
+        const uint32_t j = j0 + q * LS_THREADS;
+        r[q] = j < m ? __ldg(rows + j) : make_int2(0, 0);
+        rank[q] = j < m ? ranks[lo + j] : 0u;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < SB_BIG; q++) {
+        if (j0 + q * LS_THREADS >= m) continue;
+        const uint32_t s = sb_find(slot, ej_hash32((uint32_t)r[q].y), npairs, p0, end);
+        if (s != SB_SPILLED) sb_place(slot, s, rank[q], r[q].x, rkey);
+      }
     }
   }
   __syncthreads();
