@@ -151,11 +151,14 @@ __device__ __forceinline__ void ej_lookback_publish(unsigned long long* status, 
 // inside their buffers.  The clock is read every 64 polls, every poll when
 // the limit is under 100 us (limit 0: give up at the first poll that finds a
 // predecessor not ready), and the wait counts from its first reading: a tile
-// whose predecessors are ready never reads it.
+// whose predecessors are ready never reads it.  mark: a word that is set too when
+// the wait gives up, for later kernels of the same call (the status word may hold
+// an earlier call's code).
 __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long long* status, uint64_t tile,
                                                                   unsigned long long aggregate,
                                                                   ej_dev_status* st, unsigned int where,
-                                                                  unsigned long long limit_ns) {
+                                                                  unsigned long long limit_ns,
+                                                                  uint32_t* mark = nullptr) {
   const unsigned int lane = threadIdx.x & 31u;
   if (tile == 0) return 0ull;
   unsigned long long exclusive = 0;
@@ -196,7 +199,10 @@ __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long 
   }
   if (lane == 0) {
     ej_st_relaxed(&status[tile], (EJ_LB_PREFIX << 62) | ((exclusive + aggregate) & EJ_LB_VALUE_MASK));
-    if (gave_up) ej_set_status(st, EJ_ERR_TIMEOUT, where);
+    if (gave_up) {
+      ej_set_status(st, EJ_ERR_TIMEOUT, where);
+      if (mark) *mark = 1u;
+    }
   }
   return exclusive;
 }
@@ -205,7 +211,7 @@ __device__ __forceinline__ unsigned long long ej_lookback_resolve(unsigned long 
 __device__ __forceinline__ unsigned long long ej_lookback_warp(unsigned long long* status, uint64_t tile,
                                                              unsigned long long aggregate,
                                                              ej_dev_status* st, unsigned int where,
-                                                             unsigned long long limit_ns) {
+                                                             unsigned long long limit_ns, uint32_t* mark = nullptr) {
   ej_lookback_publish(status, tile, aggregate);
-  return ej_lookback_resolve(status, tile, aggregate, st, where, limit_ns);
+  return ej_lookback_resolve(status, tile, aggregate, st, where, limit_ns, mark);
 }

@@ -174,10 +174,11 @@ static inline uint32_t ej_ceil_log2(uint64_t x) {
 // must hold ej_scan_scratch_bytes(n) bytes of device memory.
 size_t ej_scan_scratch_bytes(uint64_t n);
 // the scratch words of a scan of n inputs; a caller whose own kernel before the
-// scan clears them (ej_clear_words, ej_device.cuh) passes cleared = true
+// scan clears them (ej_clear_words, ej_device.cuh) passes cleared = true;
+// *gave_up (a device word) is set when a wait of the scan gives up
 inline uint64_t ej_scan_words(uint64_t n) { return ej_scan_scratch_bytes(n) / sizeof(unsigned long long); }
 ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch,
-                          bool cleared = false);
+                          bool cleared = false, uint32_t* gave_up = nullptr);
 ej_status ej_scan_u32_u64(ej_handle* h, const uint32_t* in, uint64_t n, unsigned long long* out,
                           void* scratch);
 // total: also stored there when not null
@@ -207,6 +208,7 @@ struct ej_radix_plan {
   uint32_t ntiles = 0;
   size_t hist_off = 0, offs_off = 0, scan_off = 0;  // arena offsets
   const ej_rx_tile* tiles = nullptr;                // device descriptors (segmented passes)
+  uint32_t* gave_up = nullptr;                      // device word, set when the pass's scan gave up waiting
 };
 uint32_t ej_radix_tiles(uint64_t n);
 void ej_radix_plan_add(ej_plan_bytes& p, ej_radix_plan& rp, uint64_t n);

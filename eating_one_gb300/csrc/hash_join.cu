@@ -192,6 +192,7 @@ struct SlotHeader {
   uint32_t marked;  // some row was marked: a key has several rows
   uint32_t cursor;  // words of rkey[] reserved (direct build)
   uint32_t nspill;  // rows spilled (build by bucket groups)
+  uint32_t gave_up; // a scan of the build by bucket groups gave up waiting
 };
 static_assert(sizeof(SlotHeader) <= EJ_SLOT_HEADER_BYTES, "slot table header");
 
@@ -709,7 +710,7 @@ ej_status ej_table_build(ej_handle* h, const ej_table_plan_t& tp, const ej_tuple
       EJ_TRY(ej_msd_slots(h, tp.mplan, R, reinterpret_cast<ej_tuple*>(ej_arena_at(h, tp.tmp_a_off)),
                           reinterpret_cast<ej_tuple*>(ej_arena_at(h, tp.tmp_b_off)), reinterpret_cast<uint4*>(slot),
                           tp.npairs, runs, reinterpret_cast<uint32_t*>(ej_arena_at(h, tp.gcursor_off)), mark,
-                          &hdr->nspill));
+                          &hdr->nspill, &hdr->gave_up));
     } else {
       EJ_CUDA(h, cudaMemsetAsync(aux, 0, EJ_SLOT_HEADER_BYTES + tp.npairs * sizeof(uint4), h->stream));
     }

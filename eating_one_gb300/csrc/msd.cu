@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(LS_THREADS, SB_BLOCKS)
 msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ bstart, uint32_t g, uint32_t npairs,
                  uint32_t pp, uint4* __restrict__ pair, int32_t* __restrict__ rkey, uint32_t* __restrict__ gcursor,
                  uint2* __restrict__ spill, uint32_t* __restrict__ nspill, uint32_t* __restrict__ ranks,
-                 const ej_dev_status* __restrict__ st) {
+                 const uint32_t* __restrict__ gave_up) {
   extern __shared__ __align__(16) unsigned char sb_smem_raw[];
   unsigned long long* slot = reinterpret_cast<unsigned long long*>(sb_smem_raw);
   __shared__ uint32_t s_runs;
@@ -456,9 +456,10 @@ msd_slots_kernel(const ej_tuple* __restrict__ in, const uint32_t* __restrict__ b
   const uint32_t n = bstart[MSD_BUCKETS];
   const uint32_t lo = min(bstart[blockIdx.x << g], n);
   uint32_t m = max(min(bstart[(blockIdx.x + 1u) << g], n), lo) - lo;
-  // a scan of the passes gave up waiting: the call reports it, and the bounds and
-  // rows are not to be relied on, so the table stays empty
-  if (st->code == EJ_ERR_TIMEOUT) m = 0u;
+  // a scan of this build's passes gave up waiting: the call reports it, and the
+  // bounds and rows are not to be relied on, so the table stays empty.  (Not the
+  // handle's status: it holds an earlier asynchronous call's code until it is read.)
+  if (*gave_up) m = 0u;
   // the group's words begin at a multiple of four, so that runs of four rows
   // throughout (one 16-byte load each) stay aligned
   const uint32_t words0 = ((lo + lo / 31u) & ~3u) + 4u * blockIdx.x;
@@ -670,9 +671,11 @@ uint32_t ej_msd_slot_pairs(uint64_t n) {
 
 // the two radix passes (rows in tmp_b, tmp_a free again) and the bucket bounds
 static ej_status msd_passes(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
-                            uint32_t** bounds) {
+                            uint32_t** bounds, uint32_t* gave_up = nullptr) {
   // 1. by bits 24..31
-  EJ_TRY(ej_partition_pass(h, mp.pass1, R, tmp_a, 24u, 8u, EJ_DIGIT_HASH));
+  ej_radix_plan p1 = mp.pass1;
+  p1.gave_up = gave_up;
+  EJ_TRY(ej_partition_pass(h, p1, R, tmp_a, 24u, 8u, EJ_DIGIT_HASH));
   // 2. by bits 16..23 inside every segment, tiles laid out on the device
   MsdSegments* seg = reinterpret_cast<MsdSegments*>(ej_arena_at(h, mp.seg_off));
   ej_rx_tile* desc = reinterpret_cast<ej_rx_tile*>(ej_arena_at(h, mp.desc_off));
@@ -683,6 +686,7 @@ static ej_status msd_passes(ej_handle* h, const ej_msd_plan& mp, const ej_tuple*
   EJ_TRY(ej_check_launch(h, "msd_tiles_kernel"));
   ej_radix_plan p2 = mp.pass2;
   p2.tiles = desc;
+  p2.gave_up = gave_up;
   EJ_TRY(ej_partition_pass(h, p2, tmp_a, tmp_b, 16u, 8u, EJ_DIGIT_HASH));
   // 3. bucket bounds
   uint32_t* bstart = reinterpret_cast<uint32_t*>(ej_arena_at(h, mp.bstart_off));
@@ -695,15 +699,15 @@ static ej_status msd_passes(ej_handle* h, const ej_msd_plan& mp, const ej_tuple*
 
 ej_status ej_msd_slots(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
                        uint4* pair, uint32_t npairs, int32_t* rkey, uint32_t* gcursor, uint32_t* mark,
-                       uint32_t* nspill) {
+                       uint32_t* nspill, uint32_t* gave_up) {
   uint32_t* bstart = nullptr;
-  EJ_TRY(msd_passes(h, mp, R, tmp_a, tmp_b, &bstart));
+  EJ_TRY(msd_passes(h, mp, R, tmp_a, tmp_b, &bstart, gave_up));
   const uint32_t g = msd_group_bits(mp.n), groups = MSD_BUCKETS >> g, pp = npairs / groups;
   const int smem = (int)(2u * pp * sizeof(unsigned long long));
   EJ_CUDA(h, cudaFuncSetAttribute(msd_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   uint2* spill = reinterpret_cast<uint2*>(tmp_a);
   msd_slots_kernel<<<groups, LS_THREADS, smem, h->stream>>>(tmp_b, bstart, g, npairs, pp, pair, rkey, gcursor, spill,
-                                                           nspill, mark, h->d_status);
+                                                           nspill, mark, gave_up);
   EJ_TRY(ej_check_launch(h, "msd_slots_kernel"));
   // the spilled rows' marks (mark held large groups' ranks before); their ranks
   // in tmp_b, whose rows are in the table now

@@ -22,9 +22,10 @@ ej_status ej_msd_sort(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej
                       int32_t* rkey, int32_t* rval);
 // The slot table (slot_table.cuh) of R: npairs = ej_msd_slot_pairs(n) pairs, runs
 // in rkey (ej_slot_run_bytes(n)); gcursor (EJ_MSD_GROUPS words) and mark (n words)
-// are scratch; *nspill is zero before the call
+// are scratch; *nspill and *gave_up are zero before the call.  *gave_up is set, and
+// the table empty, when a scan of the build gave up waiting
 constexpr uint32_t EJ_MSD_GROUPS = 1u << 16;
 uint32_t ej_msd_slot_pairs(uint64_t n);
 ej_status ej_msd_slots(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, ej_tuple* tmp_a, ej_tuple* tmp_b,
                        uint4* pair, uint32_t npairs, int32_t* rkey, uint32_t* gcursor, uint32_t* mark,
-                       uint32_t* nspill);
+                       uint32_t* nspill, uint32_t* gave_up);

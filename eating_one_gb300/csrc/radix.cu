@@ -244,7 +244,7 @@ static ej_status radix_pass_kind(ej_handle* h, const ej_radix_plan& rp, const ej
       in, rp.n, rp.tiles, hist, rp.ntiles, shift, mask,
       reinterpret_cast<unsigned long long*>(ej_arena_at(h, rp.scan_off)), ej_scan_words(cells));
   EJ_TRY(ej_check_launch(h, "rx_hist_kernel"));
-  EJ_TRY(ej_scan_u32_u32(h, hist, cells, offs, ej_arena_at(h, rp.scan_off), /*cleared=*/true));
+  EJ_TRY(ej_scan_u32_u32(h, hist, cells, offs, ej_arena_at(h, rp.scan_off), /*cleared=*/true, rp.gave_up));
   EJ_CUDA(h, cudaFuncSetAttribute(rx_scatter_kernel<KIND, SOA, STABLE, SRC>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RxScatterSmem)));
   rx_scatter_kernel<KIND, SOA, STABLE, SRC><<<rp.ntiles, RX_THREADS, sizeof(RxScatterSmem), h->stream>>>(

@@ -19,7 +19,8 @@ constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 template <typename In, typename Out>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_kernel(const In* __restrict__ in, uint64_t n, Out* __restrict__ out, unsigned long long* status,
-            unsigned int* tile_ctr, uint64_t ntiles, ej_dev_status* st, unsigned long long wait_ns, Out* total) {
+            unsigned int* tile_ctr, uint64_t ntiles, ej_dev_status* st, unsigned long long wait_ns, Out* total,
+            uint32_t* gave_up) {
   __shared__ Out sbuf[SCAN_TILE + SCAN_TILE / 32];
   __shared__ Out warp_tmp[SCAN_THREADS / 32 + 1];
   __shared__ unsigned int s_tile;
@@ -51,7 +52,7 @@ scan_kernel(const In* __restrict__ in, uint64_t n, Out* __restrict__ out, unsign
 
   if (threadIdx.x < 32) {
     const unsigned long long ex =
-        ej_lookback_warp(status, tile, (unsigned long long)aggregate, st, /*where=*/1u, wait_ns);
+        ej_lookback_warp(status, tile, (unsigned long long)aggregate, st, /*where=*/1u, wait_ns, gave_up);
     if (threadIdx.x == 0) s_prefix = (Out)ex;
   }
   __syncthreads();
@@ -78,7 +79,7 @@ scan_kernel(const In* __restrict__ in, uint64_t n, Out* __restrict__ out, unsign
 
 template <typename In, typename Out>
 ej_status launch_scan(ej_handle* h, const In* in, uint64_t n, Out* out, void* scratch, bool cleared = false,
-                      Out* total = nullptr) {
+                      Out* total = nullptr, uint32_t* gave_up = nullptr) {
   if (n == 0) {
     EJ_CUDA(h, cudaMemsetAsync(out, 0, sizeof(Out), h->stream));
     if (total) EJ_CUDA(h, cudaMemsetAsync(total, 0, sizeof(Out), h->stream));
@@ -90,7 +91,7 @@ ej_status launch_scan(ej_handle* h, const In* in, uint64_t n, Out* out, void* sc
   unsigned int* ctr = reinterpret_cast<unsigned int*>(status + ntiles);
   if (!cleared) EJ_CUDA(h, cudaMemsetAsync(scratch, 0, ntiles * sizeof(unsigned long long) + 16, h->stream));
   scan_kernel<In, Out><<<(unsigned)ntiles, SCAN_THREADS, 0, h->stream>>>(in, n, out, status, ctr, ntiles,
-                                                                         h->d_status, h->wait_limit_ns, total);
+                                                                         h->d_status, h->wait_limit_ns, total, gave_up);
   return ej_check_launch(h, "scan_kernel");
 }
 
@@ -101,8 +102,9 @@ size_t ej_scan_scratch_bytes(uint64_t n) {
   return (size_t)(ntiles * sizeof(unsigned long long) + 16);
 }
 
-ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch, bool cleared) {
-  return launch_scan<uint32_t, uint32_t>(h, in, n, out, scratch, cleared);
+ej_status ej_scan_u32_u32(ej_handle* h, const uint32_t* in, uint64_t n, uint32_t* out, void* scratch, bool cleared,
+                          uint32_t* gave_up) {
+  return launch_scan<uint32_t, uint32_t>(h, in, n, out, scratch, cleared, nullptr, gave_up);
 }
 
 ej_status ej_scan_u32_u64(ej_handle* h, const uint32_t* in, uint64_t n, unsigned long long* out,
@@ -190,7 +192,7 @@ extern "C" ej_status ej_exclusive_scan_u32_noalloc(const uint32_t* in, uint64_t 
   }
   unsigned int* ctr = reinterpret_cast<unsigned int*>(d.scratch + ntiles);
   scan_kernel<uint32_t, unsigned long long><<<(unsigned)ntiles, SCAN_THREADS, 0, s>>>(
-      in, n, o, d.scratch, ctr, ntiles, d.status, EJ_DEFAULT_WAIT_LIMIT_NS, nullptr);
+      in, n, o, d.scratch, ctr, ntiles, d.status, EJ_DEFAULT_WAIT_LIMIT_NS, nullptr, nullptr);
   if (cudaGetLastError() != cudaSuccess) return EJ_ERR_CUDA;
   ej_dev_status host_status;
   if (cudaMemcpyAsync(&host_status, d.status, sizeof(host_status), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
