@@ -55,6 +55,7 @@ struct Lane {
   cudaStream_t stream = nullptr;
   unsigned long long* d_counts = nullptr;
   unsigned long long* h_counts = nullptr;
+  ej_dev_status* h_status = nullptr;  // the handle's device status after the batch
   // EJ_SERVE_CHECKSUM: the batch's requests and their outputs' checksums
   ej_join_desc* d_desc = nullptr;
   ej_join_desc* h_desc = nullptr;
@@ -77,6 +78,12 @@ void CUDART_CB lane_done(void* arg) {
   Lane* L = static_cast<Lane*>(arg);
   Server* S = L->srv;
   const uint64_t now = ej_now_ns();
+  // a wait of one of the batch's kernels gave up: whose rows it concerns is not
+  // known, so no request of the batch is reported as done (a short capacity is
+  // told from each request's count)
+  ej_status st = L->launch_status;
+  if (st == EJ_OK && L->h_status->code != 0 && L->h_status->code != EJ_ERR_CAPACITY)
+    st = (ej_status)L->h_status->code;
   {
     std::lock_guard<std::mutex> lock(S->mu);
     for (size_t i = 0; i < L->batch.size(); i++) {
@@ -84,8 +91,7 @@ void CUDART_CB lane_done(void* arg) {
       ej_completion c;
       c.tag = r.tag;
       c.count = L->h_counts[i];
-      c.status = L->launch_status != EJ_OK ? L->launch_status
-                 : (c.count > r.join.out_cap ? EJ_ERR_CAPACITY : EJ_OK);
+      c.status = st != EJ_OK ? st : (c.count > r.join.out_cap ? EJ_ERR_CAPACITY : EJ_OK);
       c.batch_joins = (uint32_t)L->batch.size();
       c.arrival_ns = r.arrival_ns;
       c.launch_ns = L->launch_ns;
@@ -104,8 +110,11 @@ void CUDART_CB lane_done(void* arg) {
 ej_status lane_launch(Lane* L, int mode) {
   ej_handle* h = L->h;
   const uint32_t n = (uint32_t)L->batch.size();
-  ej_status st = EJ_OK;
-  if (mode == EJ_SERVE_BATCHED) {
+  // the status word is the batch's own: cleared before its first kernel (whatever
+  // an earlier batch left), read back behind its last
+  ej_status st = cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), L->stream) == cudaSuccess ? EJ_OK : EJ_ERR_CUDA;
+  if (st != EJ_OK) {
+  } else if (mode == EJ_SERVE_BATCHED) {
     std::vector<ej_join_desc> d(n);
     for (uint32_t i = 0; i < n; i++) d[i] = L->batch[i].join;
     st = ej_batch_hash_join_async(h, d.data(), n, reinterpret_cast<uint64_t*>(L->d_counts));
@@ -128,6 +137,9 @@ ej_status lane_launch(Lane* L, int mode) {
       st = EJ_ERR_CUDA;
   }
   if (st == EJ_OK && cudaMemcpyAsync(L->h_counts, L->d_counts, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                     L->stream) != cudaSuccess)
+    st = EJ_ERR_CUDA;
+  if (st == EJ_OK && cudaMemcpyAsync(L->h_status, h->d_status, sizeof(ej_dev_status), cudaMemcpyDeviceToHost,
                                      L->stream) != cudaSuccess)
     st = EJ_ERR_CUDA;
   L->launch_status = st;
@@ -189,6 +201,7 @@ void server_free(Server* S) {
     if (L->stream) cudaStreamDestroy(L->stream);
     cudaFree(L->d_counts);
     cudaFreeHost(L->h_counts);
+    cudaFreeHost(L->h_status);
     cudaFree(L->d_desc);
     cudaFreeHost(L->h_desc);
     cudaFree(L->d_sums);
@@ -229,6 +242,7 @@ extern "C" ej_status ej_server_create(const ej_server_config* cfg, ej_server** o
     if (cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking) != cudaSuccess ||
         ej_dev_alloc(&L->d_counts, per_lane * sizeof(unsigned long long)) != cudaSuccess ||
         ej_host_alloc(&L->h_counts, per_lane * sizeof(unsigned long long)) != cudaSuccess ||
+        ej_host_alloc(&L->h_status, sizeof(ej_dev_status)) != cudaSuccess ||
         ((S->cfg.flags & EJ_SERVE_CHECKSUM) &&
          (ej_dev_alloc(&L->d_desc, per_lane * sizeof(ej_join_desc)) != cudaSuccess ||
           ej_host_alloc(&L->h_desc, per_lane * sizeof(ej_join_desc)) != cudaSuccess ||
@@ -245,6 +259,15 @@ extern "C" ej_status ej_server_create(const ej_server_config* cfg, ej_server** o
   ej_server* srv = new ej_server();
   srv->s = S;
   *out = srv;
+  return EJ_OK;
+}
+
+extern "C" ej_status ej_server_set_option(ej_server* srv, ej_option opt, int64_t value) {
+  if (!srv) return EJ_ERR_INVALID;
+  Server* S = srv->s;
+  std::lock_guard<std::mutex> lock(S->mu);
+  if (S->completed != S->submitted) return EJ_ERR_BUSY;  // the lanes' handles may be in use
+  for (Lane* L : S->lanes) EJ_TRY(ej_set_option(L->h, opt, value));
   return EJ_OK;
 }
 

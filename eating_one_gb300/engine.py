@@ -16,6 +16,11 @@ from . import native
 from .native import GenSpec
 
 
+# ej_option (include/ej.h)
+OPTIONS = {"partition_bits": 0, "bucket_bits_delta": 1, "wait_limit_ns": 2, "count_reuse": 3, "build": 4, "table": 5,
+           "probe_warps": 6}
+
+
 class JoinError(RuntimeError):
     def __init__(self, status: int, message: str):
         super().__init__("%s: %s" % (native.load().ej_status_name(status).decode(), message))
@@ -106,9 +111,7 @@ class Engine:
         self.lib.ej_set_stream(self.h, torch.cuda.current_stream(self.device).cuda_stream)
 
     def set_option(self, name: str, value: int) -> None:
-        opt = {"partition_bits": 0, "bucket_bits_delta": 1, "wait_limit_ns": 2, "count_reuse": 3, "build": 4,
-               "table": 5, "probe_warps": 6}[name]
-        self._check(self.lib.ej_set_option(self.h, opt, value))
+        self._check(self.lib.ej_set_option(self.h, OPTIONS[name], value))
 
     def set_timing(self, enable: bool) -> None:
         self._check(self.lib.ej_set_timing(self.h, 1 if enable else 0))

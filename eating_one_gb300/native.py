@@ -152,6 +152,7 @@ _SIGS = {
     "ej_batch_hash_join": [_vp, _vp, C.c_uint32, _pu64],
     "ej_batch_hash_join_async": [_vp, _vp, C.c_uint32, _vp],
     "ej_server_create": [C.POINTER(ServerConfig), C.POINTER(C.c_void_p)],
+    "ej_server_set_option": [_vp, _i32, C.c_int64],
     "ej_server_submit": [_vp, C.POINTER(JoinDesc), _u64, _u64],
     "ej_server_poll": [_vp, C.POINTER(Completion), C.c_uint32, C.POINTER(C.c_uint32), C.c_uint32],
     "ej_server_drain": [_vp],

@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import native
-from .engine import Engine, JoinError
+from .engine import OPTIONS, Engine, JoinError
 from .workloads import EJ_GEN_PERM, EJ_GEN_UNIFORM, make_spec
 
 BATCHED, PER_JOIN = native.EJ_SERVE_BATCHED, native.EJ_SERVE_PER_JOIN
@@ -40,6 +40,12 @@ class Server:
 
     def now_ns(self) -> int:
         return int(self.lib.ej_now_ns())
+
+    def set_option(self, name: str, value: int) -> None:
+        """Engine.set_option on every lane, while no request is under way."""
+        st = self.lib.ej_server_set_option(self.h, OPTIONS[name], value)
+        if st != native.EJ_OK:
+            raise JoinError(st, "ej_server_set_option failed")
 
     def submit(self, desc: native.JoinDesc, tag: int, arrival_ns: int = 0) -> None:
         st = self.lib.ej_server_submit(self.h, C.byref(desc), tag, arrival_ns)

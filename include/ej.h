@@ -367,7 +367,8 @@ typedef struct ej_server_config {
 typedef struct ej_completion {
   uint64_t tag;          /* the submit tag */
   uint64_t count;        /* the join's result count (rows past out_cap dropped) */
-  int32_t status;        /* EJ_OK, EJ_ERR_CAPACITY or the batch's error */
+  int32_t status;        /* EJ_OK, EJ_ERR_CAPACITY or the batch's error (EJ_ERR_TIMEOUT: a
+                            device-side wait of the batch gave up, the rows are not valid) */
   uint32_t batch_joins;  /* joins in the batch that carried the request */
   uint64_t arrival_ns;   /* ej_now_ns() clock: arrival, launch, completion */
   uint64_t launch_ns;
@@ -384,6 +385,9 @@ ej_status ej_server_create(const ej_server_config* cfg, ej_server** out);
 ej_status ej_server_submit(ej_server* s, const ej_join_desc* join, uint64_t tag, uint64_t arrival_ns);
 /* Take up to max completions; waits up to wait_us microseconds for the first. */
 ej_status ej_server_poll(ej_server* s, ej_completion* out, uint32_t max, uint32_t* n, uint32_t wait_us);
+/* ej_set_option on every lane's handle.  EJ_ERR_BUSY while a submitted request has
+ * not completed (nothing is changed). */
+ej_status ej_server_set_option(ej_server* s, ej_option opt, int64_t value);
 /* Wait until every submitted request has completed (its completion can still be polled). */
 ej_status ej_server_drain(ej_server* s);
 ej_status ej_server_destroy(ej_server* s);
