@@ -324,13 +324,16 @@ ej_status ej_begin(ej_handle* h) {
 }
 
 // Synchronise, with the device status and count word in the host mirror; a
-// status that was set is cleared (before anything later on the stream).
+// status that was set is cleared before the call returns: the caller may go on
+// on another stream (ej_set_stream), which nothing orders behind this one.
 static ej_status ej_read_status(ej_handle* h) {
   EJ_CUDA(h, cudaMemcpyAsync(h->h_block, h->d_block, sizeof(ej_dev_status) + sizeof(unsigned long long),
                              cudaMemcpyDeviceToHost, h->stream));
   EJ_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (h->h_block->status.code != 0)
+  if (h->h_block->status.code != 0) {
     EJ_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), h->stream));
+    EJ_CUDA(h, cudaStreamSynchronize(h->stream));
+  }
   return EJ_OK;
 }
 

@@ -108,3 +108,24 @@ def test_server_options_wait_for_the_requests(engine):
         assert n == {engine.count("hash", Rd, Sd)}
     finally:
         srv.close()
+
+
+def test_status_is_clear_when_a_call_returns(engine):
+    """A call that found a short capacity returns with the status word cleared and nothing of its
+    own under way: the next call may use another stream, which nothing orders behind this one."""
+    rng = np.random.default_rng(13)
+    R, S = _rel(rng.integers(0, 1000, 3000)), _rel(rng.integers(0, 1000, 5000), 1 << 23)
+    Rd, Sd = torch.from_numpy(R).cuda(), torch.from_numpy(S).cuda()
+    rows = len(O.left_outer_join(R, S))
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    pending = 0
+    for _ in range(50):
+        with torch.cuda.stream(a):
+            n = engine.count("left_outer", Rd, Sd)
+            pending += not a.query()
+        assert n == rows
+        with torch.cuda.stream(b):
+            engine._sync_stream()
+            assert engine.sync_status() == native.EJ_OK
+    assert pending == 0
