@@ -704,7 +704,9 @@ ej_status ej_msd_slots(ej_handle* h, const ej_msd_plan& mp, const ej_tuple* R, e
   EJ_TRY(msd_passes(h, mp, R, tmp_a, tmp_b, &bstart, gave_up));
   const uint32_t g = msd_group_bits(mp.n), groups = MSD_BUCKETS >> g, pp = npairs / groups;
   const int smem = (int)(2u * pp * sizeof(unsigned long long));
-  EJ_CUDA(h, cudaFuncSetAttribute(msd_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // 32 KB and less (LS_ROWS rows a group or fewer): within the default limit, which
+  // is the function's, for every handle and thread, so it is left alone
+  if (smem > 48 * 1024 - 256) return ej_fail(h, EJ_ERR_INTERNAL, "bucket group of %u pairs", pp);
   uint2* spill = reinterpret_cast<uint2*>(tmp_a);
   msd_slots_kernel<<<groups, LS_THREADS, smem, h->stream>>>(tmp_b, bstart, g, npairs, pp, pair, rkey, gcursor, spill,
                                                            nspill, mark, gave_up);

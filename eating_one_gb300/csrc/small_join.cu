@@ -94,11 +94,16 @@ small_join_kernel(const int2* __restrict__ R, uint32_t nR, const int2* __restric
   }
 }
 
+// most rows of the 256-thread CTAs (see sj_run)
+constexpr uint64_t SJ_SHORT_ROWS = 4096;
+
 template <int THREADS, bool COUNT_ONLY, bool OUTER>
 ej_status sj_launch(ej_handle* h, const ej_tuple* R, uint64_t nR, const ej_tuple* S, uint64_t nS, const BtOut& out) {
   const SjLayout l = sj_layout<THREADS>(nR);
   auto k = small_join_kernel<THREADS, COUNT_ONLY, OUTER>;
-  EJ_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.bytes));
+  // the attribute is the function's, for every handle and thread: always its most
+  const SjLayout most = sj_layout<THREADS>(THREADS == 256 ? SJ_SHORT_ROWS : BT_ROWS);
+  EJ_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most.bytes));
   // as many CTAs as are resident at once (1 KB of each SM's 228 KB is taken
   // per CTA by the system), fewer when S is short
   const uint64_t per_sm = std::max<uint64_t>(1, std::min<uint64_t>(2048 / THREADS, (227u * 1024u) / (l.bytes + 1280u)));
@@ -114,8 +119,8 @@ ej_status sj_run(ej_handle* h, const ej_tuple* R, uint64_t nR, const ej_tuple* S
   // tables up to 4096 rows (56 KB) leave room for three or more CTAs of 256
   // threads, whose build barriers are cheaper and which spread a short S over
   // more SMs
-  return nR <= 4096 ? sj_launch<256, COUNT_ONLY, OUTER>(h, R, nR, S, nS, out)
-                    : sj_launch<1024, COUNT_ONLY, OUTER>(h, R, nR, S, nS, out);
+  return nR <= SJ_SHORT_ROWS ? sj_launch<256, COUNT_ONLY, OUTER>(h, R, nR, S, nS, out)
+                             : sj_launch<1024, COUNT_ONLY, OUTER>(h, R, nR, S, nS, out);
 }
 
 }  // namespace
