@@ -323,11 +323,11 @@ ej_status ej_begin(ej_handle* h) {
   return EJ_OK;
 }
 
-// Synchronise, with the device status and count word in the host mirror; a
+// Synchronise, with the device status and first two words in the host mirror; a
 // status that was set is cleared before the call returns: the caller may go on
 // on another stream (ej_set_stream), which nothing orders behind this one.
 static ej_status ej_read_status(ej_handle* h) {
-  EJ_CUDA(h, cudaMemcpyAsync(h->h_block, h->d_block, sizeof(ej_dev_status) + sizeof(unsigned long long),
+  EJ_CUDA(h, cudaMemcpyAsync(h->h_block, h->d_block, sizeof(ej_dev_status) + 2 * sizeof(unsigned long long),
                              cudaMemcpyDeviceToHost, h->stream));
   EJ_CUDA(h, cudaStreamSynchronize(h->stream));
   if (h->h_block->status.code != 0) {

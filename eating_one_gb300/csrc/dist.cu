@@ -38,7 +38,8 @@
 // bucket, so no pair comes twice.
 //
 // Launches: cells (histogram with the points' ranks in their buckets), scan,
-// placement, probe.  A probe warp takes 32 S points: each lane finds its point's
+// placement, probe, and where buckets are crowded one more for these (below); few
+// S points: one launch, no grid.  A probe warp takes 32 S points: each lane finds its point's
 // cells, then groups of 4 (2-D) or 8 (3-D) lanes share a point, a lane per cell,
 // and walk the buckets together, two candidates a step; the pairs that pass
 // the screen collect in shared memory, and full buffers are tested and become
@@ -56,6 +57,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <functional>
 
 #include "ej_device.cuh"
 #include "ej_entry.h"
@@ -65,10 +67,11 @@ namespace {
 constexpr int DJ_THREADS = 256;
 constexpr int DJ_WARPS = DJ_THREADS / 32;
 constexpr int DJ_BUF = 192;  // candidate pairs a warp collects (tested past 128; a step adds at most 64)
-// points per launch sequence: 32-bit rows in the grid's entries, and a grid of
-// at most 2 GB of scratch; larger relations go in pieces
+// points per launch sequence: 32-bit rows in the grid's entries, and at most 2.5 GB
+// of scratch for the grid, 0.25 GB for crowded buckets; larger relations go in pieces
 constexpr uint64_t DJ_RPIECE = 1ull << 26;
-constexpr uint64_t DJ_SPIECE = 1ull << 31;
+constexpr uint64_t DJ_SPIECE = 1ull << 26;
+constexpr uint64_t DJ_FEW_RPIECE = 1ull << 31;  // without a grid
 
 template <int D>
 struct Point {
@@ -76,6 +79,9 @@ struct Point {
   double val[D];
 };
 static_assert(sizeof(Point<2>) == sizeof(ej_point2) && sizeof(Point<3>) == sizeof(ej_point3), "point layouts");
+
+// the handle's words of the list of crowded buckets (DistCrowd::header), behind the row cursor
+constexpr int DJ_CROWD_WORD = 1;
 
 // the radius as the kernels use it
 struct DistRadius {
@@ -164,6 +170,18 @@ __device__ __forceinline__ float dist_screen_bound(float rho_up, float m) {
   const float e = __fadd_ru(__fmul_ru(0x1p-24f, __fadd_ru(__fmul_ru(2.0f, m), __fmul_ru(4.0f, rho_up))), 0x1p-140f);
   const float b = __fmul_ru(__fadd_ru(rho_up, __fmul_ru(1.7320509f, e)), 1.0f + 0x1p-18f);
   return __fadd_ru(__fmul_ru(__fmul_ru(b, b), 1.0f + 0x1p-18f), 0x1p-140f);
+}
+
+// an S point as the screen uses it: its coordinates as floats, and the bound
+template <int D>
+__device__ __forceinline__ float dist_screen_point(const double (&v)[D], float rho_up, float (&x)[D]) {
+  float m = 0.0f;
+#pragma unroll
+  for (int d = 0; d < D; d++) {
+    x[d] = __double2float_rn(v[d]);
+    m = fmaxf(m, __fmul_ru(fabsf(x[d]), 1.0f + 0x1p-23f));
+  }
+  return dist_screen_bound(rho_up, m);
 }
 
 template <int D>
@@ -279,11 +297,150 @@ __device__ __forceinline__ uint32_t dist_flush(uint2* buf, uint32_t n, const Poi
   return rows;
 }
 
+// ---- crowded buckets -------------------------------------------------------------
+// A bucket of DJ_CROWD rows or more (a radius that reaches many points, points in
+// few cells) would be walked by one lane per S point and cell, and few S points by
+// few warps.  Its lookups become items of a list, {first S row, owners, first grid
+// entry, end}, instead: the owners (bits) are those of the probe warp's 32 S points
+// that look at it, the entries a part of the bucket.  A kernel of its own takes the
+// items, a warp each, all lanes at work: k owners and 32 / k entries a step.
+// The list has two parts: buckets in parts, as many as fill the device when few S
+// points are concerned, and whole buckets, once the first part is full.  What finds
+// no room there either (many S points in many crowded buckets) is walked as the
+// others are, by then with most lanes at work.
+// Counts of 2^20 R and 64 to 1500 S points, a radius that reaches 0.3% of R: walked
+// 4.9 to 4.5 ms; 2^24 R and 400 S points 121 ms walked, 1.7 listed.
+constexpr uint32_t DJ_CROWD = 256;
+constexpr uint32_t DJ_ITEM_ROWS = 1024;     // least entries of a part
+constexpr uint32_t DJ_SPLIT = 1u << 18;     // items in parts
+constexpr uint64_t DJ_WHOLE = 1u << 14;     // whole buckets: 8 per 32 S points, at least these
+
+struct DistCrowd {
+  uint4* items;      // [DJ_SPLIT + whole]
+  uint32_t* header;  // items {in parts, whole}, counted on past the room; {taken}
+  uint32_t whole;
+  uint32_t parts;  // parts of a bucket at most
+};
+
+// The matches of the item's owners among its entries: candidates collect in buf
+// (held of them), full buffers are tested.  Count-only: returns the lane's matches
+// among those tested.
+template <int D, bool COUNT_ONLY>
+__device__ __forceinline__ uint32_t dist_crowd(const uint4& it, const Point<D>* __restrict__ R,
+                                               const Point<D>* __restrict__ S, const float4* __restrict__ grid,
+                                               const DistRadius& rad, typename RowOf<D>::type* __restrict__ out,
+                                               uint64_t cap, unsigned long long* cursor, uint2* buf, uint32_t& held) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t lg = 0;  // 2^lg owners a step
+  while ((1u << lg) < (uint32_t)__popc(it.y)) lg++;
+  uint32_t m = it.y;
+  for (uint32_t i = lane & ((1u << lg) - 1u); i; i--) m &= m - 1u;
+  const bool ok = m != 0u;
+  const uint32_t si = it.x + (ok ? __ffs(m) - 1u : 0u);
+  float x[D], bound;
+  {
+    double v[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) v[d] = ok ? S[si].val[d] : 0.0;
+    bound = dist_screen_point<D>(v, rad.rho_up, x);
+  }
+  uint32_t rows = 0;
+  constexpr int U = 4;
+  for (uint32_t q = it.z; q < it.w; q += U * (32u >> lg)) {
+    float4 e[U];
+    bool pass[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint32_t at = q + u * (32u >> lg) + (lane >> lg);
+      pass[u] = ok && at < it.w;
+      e[u] = pass[u] ? __ldg(grid + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    bool some = false;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const float dx = e[u].x - x[0], dy = e[u].y - x[1], dz = D == 3 ? e[u].z - x[D - 1] : 0.0f;
+      pass[u] = pass[u] && !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > bound);
+      some |= pass[u];
+    }
+    if (!__any_sync(EJ_FULL_MASK, some)) continue;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const unsigned b = __ballot_sync(EJ_FULL_MASK, pass[u]);
+      if (pass[u]) buf[held + __popc(b & ej_lanemask_lt())] = make_uint2(si, __float_as_uint(e[u].w));
+      held += __popc(b);
+      if (held > DJ_BUF - 64) {
+        const uint32_t n = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+        if (COUNT_ONLY) rows += n;
+        held = 0;
+      }
+    }
+  }
+  return rows;
+}
+
+// Lists the entries [from, end) of a crowded bucket for those of the warp's S points
+// (the first is s0) that look at it; false: no room.
+__device__ __forceinline__ bool dist_list(const DistCrowd& crowd, uint32_t s0, uint32_t owners, uint32_t from,
+                                          uint32_t end) {
+  const uint32_t lane = threadIdx.x & 31u, len = end - from;
+  const uint32_t want = min(len / DJ_ITEM_ROWS + 1u, crowd.parts);
+  const uint32_t step = (len + want - 1u) / want, parts = (len + step - 1u) / step;
+  volatile const uint32_t* listed = crowd.header;  // (looked at first, so that the counters stay small)
+  uint32_t at = DJ_SPLIT, whole = crowd.whole;
+  if (lane == 0) {
+    if (listed[0] < DJ_SPLIT) at = atomicAdd(crowd.header, parts);
+    if (at + parts > DJ_SPLIT && listed[1] < crowd.whole) whole = atomicAdd(crowd.header + 1, 1u);
+  }
+  at = __shfl_sync(EJ_FULL_MASK, at, 0);
+  whole = __shfl_sync(EJ_FULL_MASK, whole, 0);
+  const bool fits = at + parts <= DJ_SPLIT;
+  for (uint32_t j = lane; j < parts && at + j < DJ_SPLIT; j += 32) {  // (empty items at the first part's end)
+    const uint32_t q = from + j * step;
+    crowd.items[at + j] = fits ? make_uint4(s0, owners, q, min(q + step, end)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (fits) return true;
+  if (whole >= crowd.whole) return false;
+  if (lane == 0) crowd.items[DJ_SPLIT + whole] = make_uint4(s0, owners, from, end);
+  return true;
+}
+
+// the listed items, a warp each until none is left
 template <int D, bool COUNT_ONLY>
 __global__ void __launch_bounds__(DJ_THREADS)
+dist_crowd_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S, const float4* __restrict__ grid,
+                  DistCrowd crowd, DistRadius rad, typename RowOf<D>::type* __restrict__ out, uint64_t cap,
+                  unsigned long long* cursor) {
+  const uint32_t split = min(crowd.header[0], DJ_SPLIT), n = split + min(crowd.header[1], crowd.whole);
+  if (n == 0) return;
+  __shared__ uint2 bufs[DJ_WARPS][DJ_BUF];
+  __shared__ unsigned long long warp_tmp[DJ_WARPS + 1];
+  uint2* buf = bufs[threadIdx.x >> 5];
+  uint32_t held = 0;
+  unsigned long long local = 0;
+  for (;;) {
+    uint32_t i = 0;
+    if ((threadIdx.x & 31u) == 0) i = atomicAdd(crowd.header + 2, 1u);
+    i = __shfl_sync(EJ_FULL_MASK, i, 0);
+    if (i >= n) break;
+    local += dist_crowd<D, COUNT_ONLY>(__ldg(crowd.items + (i < split ? i : DJ_SPLIT + (i - split))), R, S, grid, rad, out, cap, cursor, buf, held);
+  }
+  if (held) {
+    const uint32_t rows = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+    if (COUNT_ONLY) local += rows;
+  }
+  if (COUNT_ONLY) {
+    unsigned long long total;
+    ej_block_exclusive_sum<DJ_THREADS, unsigned long long>(local, warp_tmp, &total);
+    if (threadIdx.x == 0 && total) atomicAdd(cursor, total);
+  }
+}
+
+template <int D, bool COUNT_ONLY>
+__global__ void __launch_bounds__(DJ_THREADS, 4)
 dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S, uint32_t nS,
                   const uint32_t* __restrict__ start, const float4* __restrict__ grid, uint32_t bits, DistRadius rad,
-                  typename RowOf<D>::type* __restrict__ out, uint64_t cap, unsigned long long* cursor) {
+                  DistCrowd crowd, typename RowOf<D>::type* __restrict__ out, uint64_t cap,
+                  unsigned long long* cursor) {
   constexpr int G = D == 2 ? 4 : 8;  // lanes of an S point: its cells, when no dimension has three
   __shared__ uint2 bufs[DJ_WARPS][DJ_BUF];
   __shared__ unsigned long long warp_tmp[DJ_WARPS + 1];
@@ -307,17 +464,15 @@ dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S
         l = S[si];
         ok = dist_finite<D>(l);
       }
-      float m = 0.0f;
+      double v[D];
 #pragma unroll
       for (int d = 0; d < D; d++) {
-        const double v = ok ? l.val[d] : 0.0;
-        lo[d] = dist_cell(dist_clamp(__dsub_rd(v, rad.rho)), rad.inv_w);
-        const uint32_t span = (uint32_t)(dist_cell(dist_clamp(__dadd_ru(v, rad.rho)), rad.inv_w) - lo[d]) + 1u;
+        v[d] = ok ? l.val[d] : 0.0;
+        lo[d] = dist_cell(dist_clamp(__dsub_rd(v[d], rad.rho)), rad.inv_w);
+        const uint32_t span = (uint32_t)(dist_cell(dist_clamp(__dadd_ru(v[d], rad.rho)), rad.inv_w) - lo[d]) + 1u;
         spans |= (ok ? span : 0u) << (8 * d);
-        x[d] = __double2float_rn(v);
-        m = fmaxf(m, __fmul_ru(fabsf(x[d]), 1.0f + 0x1p-23f));
       }
-      bound = dist_screen_bound(rad.rho_up, m);
+      bound = dist_screen_point<D>(v, rad.rho_up, x);
     }
     // 32 / G of the warp's S points at a time, G lanes each
     for (int t = 0; t < G; t++) {
@@ -363,7 +518,19 @@ dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S
           p = __ldg(start + b);
           end = __ldg(start + b + 1);
         }
-        while (__any_sync(EJ_FULL_MASK, p < end)) {
+        uint32_t longest = __reduce_max_sync(EJ_FULL_MASK, end - p);
+        if (longest >= DJ_CROWD) {
+          for (unsigned many = __ballot_sync(EJ_FULL_MASK, end - p >= DJ_CROWD); many;) {
+            const int leader = __ffs(many) - 1;
+            const uint32_t q = __shfl_sync(EJ_FULL_MASK, p, leader), qe = __shfl_sync(EJ_FULL_MASK, end, leader);
+            const bool here = (many >> lane & 1u) && p == q;
+            many &= ~__ballot_sync(EJ_FULL_MASK, here);
+            const uint32_t owners = __reduce_or_sync(EJ_FULL_MASK, here ? 1u << owner : 0u);
+            if (dist_list(crowd, (uint32_t)w, owners, q, qe) && here) p = end;
+          }
+          longest = __reduce_max_sync(EJ_FULL_MASK, end - p);
+        }
+        for (uint32_t k2 = 0; k2 < longest; k2 += 2) {
           bool pass[2];
           uint32_t ri[2];
 #pragma unroll
@@ -404,6 +571,82 @@ dist_probe_kernel(const Point<D>* __restrict__ R, const Point<D>* __restrict__ S
   }
 }
 
+// ---- few S points ------------------------------------------------------------------
+// Few S points are compared with every R point, which a lane brings in once: no grid.
+// The grid of 2^24 R points costs 0.98 (2-D) and 1.55 ms (3-D; random atomics and
+// stores), a compare with all of them 9.2 us per S point.
+constexpr uint32_t DJ_FEW = 160;
+template <int D>
+constexpr uint32_t dist_few_most() { return D == 2 ? 112u : DJ_FEW; }
+
+template <int D, bool COUNT_ONLY>
+__global__ void __launch_bounds__(DJ_THREADS)
+dist_few_kernel(const Point<D>* __restrict__ R, uint32_t nR, const Point<D>* __restrict__ S, uint32_t nS,
+                DistRadius rad, typename RowOf<D>::type* __restrict__ out, uint64_t cap, unsigned long long* cursor) {
+  __shared__ float4 points[DJ_FEW];  // coordinates and bound; a point that matches nothing has a negative bound
+  __shared__ uint2 bufs[DJ_WARPS][DJ_BUF];
+  __shared__ unsigned long long warp_tmp[DJ_WARPS + 1];
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t i = threadIdx.x; i < nS; i += DJ_THREADS) {
+    const Point<D> l = S[i];
+    const bool ok = dist_finite<D>(l);
+    double v[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) v[d] = ok ? l.val[d] : 0.0;
+    float x[D];
+    const float bound = dist_screen_point<D>(v, rad.rho_up, x);
+    points[i] = make_float4(x[0], x[1], D == 3 ? x[D - 1] : 0.0f, ok ? bound : -1.0f);
+  }
+  __syncthreads();
+  uint2* buf = bufs[threadIdx.x >> 5];
+  uint32_t held = 0;
+  unsigned long long local = 0;
+  constexpr int U = 2;  // R points per lane and step
+  for (uint64_t w = (((uint64_t)blockIdx.x * DJ_THREADS + threadIdx.x) & ~31ull) * U; w < nR;
+       w += (uint64_t)gridDim.x * DJ_THREADS * U) {
+    float x[U][D];
+    bool ok[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t i = w + 32u * u + lane;
+      ok[u] = i < nR;
+#pragma unroll
+      for (int d = 0; d < D; d++) x[u][d] = ok[u] ? __double2float_rn(__ldg(&R[i].val[d])) : 0.0f;
+    }
+    for (uint32_t s = 0; s < nS; s++) {
+      const float4 l = points[s];
+      bool pass[U], some = false;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const float dx = x[u][0] - l.x, dy = x[u][1] - l.y, dz = D == 3 ? x[u][D - 1] - l.z : 0.0f;
+        pass[u] = ok[u] && !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > l.w);
+        some |= pass[u];
+      }
+      if (!__any_sync(EJ_FULL_MASK, some)) continue;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const unsigned b = __ballot_sync(EJ_FULL_MASK, pass[u]);
+        if (pass[u]) buf[held + __popc(b & ej_lanemask_lt())] = make_uint2(s, (uint32_t)w + 32u * u + lane);
+        held += __popc(b);
+      }
+      if (held > DJ_BUF - 64) {
+        const uint32_t rows = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+        if (COUNT_ONLY) local += rows;
+        held = 0;
+      }
+    }
+  }
+  if (held) {
+    const uint32_t rows = dist_flush<D, COUNT_ONLY>(buf, held, R, S, rad.r2, out, cap, cursor);
+    if (COUNT_ONLY) local += rows;
+  }
+  if (COUNT_ONLY) {
+    unsigned long long total;
+    ej_block_exclusive_sum<DJ_THREADS, unsigned long long>(local, warp_tmp, &total);
+    if (threadIdx.x == 0 && total) atomicAdd(cursor, total);
+  }
+}
+
 DistRadius dist_radius(double radius) {
   DistRadius r;
   r.rho = fabs(radius);
@@ -423,27 +666,57 @@ DistRadius dist_radius(double radius) {
 uint32_t dist_bits(uint64_t n) { return std::max(8u, ej_ceil_log2(n) + 1u); }
 
 template <int D>
+ej_status dist_few(ej_handle* h, const Point<D>* R, uint64_t nR, const Point<D>* S, uint32_t nS, const DistRadius& rad,
+                   void* outv, uint64_t cap, bool count_only) {
+  ej_phase_begin(h);
+  for (int k = 1; k < EJ_PHASES; k++) ej_phase_mark(h, k);
+  for (uint64_t r0 = 0; r0 < nR; r0 += DJ_FEW_RPIECE) {
+    const uint32_t n = (uint32_t)std::min<uint64_t>(DJ_FEW_RPIECE, nR - r0);
+    const unsigned blocks =
+        (unsigned)std::min<uint64_t>(((uint64_t)n + 2 * DJ_THREADS - 1) / (2 * DJ_THREADS), (uint64_t)h->num_sms * 8);
+    if (count_only)
+      dist_few_kernel<D, true><<<blocks, DJ_THREADS, 0, h->stream>>>(R + r0, n, S, nS, rad, nullptr, 0, h->d_words);
+    else
+      dist_few_kernel<D, false><<<blocks, DJ_THREADS, 0, h->stream>>>(
+          R + r0, n, S, nS, rad, static_cast<typename RowOf<D>::type*>(outv), cap, h->d_words);
+    EJ_TRY(ej_check_launch(h, "dist_few_kernel"));
+  }
+  ej_phase_mark(h, EJ_PHASES);
+  return EJ_OK;
+}
+
+template <int D>
 ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, uint64_t nS, double radius, void* outv,
-                   uint64_t cap, bool count_only) {
+                   uint64_t cap, bool count_only, std::function<ej_status()>* crowded) {
   const Point<D>* R = static_cast<const Point<D>*>(Rv);
   const Point<D>* S = static_cast<const Point<D>*>(Sv);
-  EJ_CUDA(h, cudaMemsetAsync(h->d_words, 0, sizeof(unsigned long long), h->stream));
+  EJ_CUDA(h, cudaMemsetAsync(h->d_words, 0, (DJ_CROWD_WORD + 2) * sizeof(unsigned long long), h->stream));
   const DistRadius rad = dist_radius(radius);
   if (nR == 0 || nS == 0 || !(rad.r2 > 0.0)) return EJ_OK;
+  if (nS <= dist_few_most<D>()) return dist_few<D>(h, R, nR, S, (uint32_t)nS, rad, outv, cap, count_only);
   const uint64_t piece = std::min(nR, DJ_RPIECE);
   const uint64_t nb = 1ull << dist_bits(piece);
+  // crowded buckets: few S points take all of the list's parts
+  DistCrowd crowd;
+  const uint64_t probes = std::min(nS, DJ_SPIECE);
+  crowd.whole = (uint32_t)std::max(DJ_WHOLE, (probes + 31) / 32 * 8);
+  crowd.parts = (uint32_t)std::max<uint64_t>(16, DJ_SPLIT / (probes << D));
   ej_plan_bytes p;
-  const size_t coff = p.add(nb * sizeof(uint32_t)), soff = p.add((nb + 1) * sizeof(uint32_t)),
-               scan_off = p.add(ej_scan_scratch_bytes(nb)), poff = p.add(piece * sizeof(uint2)),
-               goff = p.add(piece * sizeof(float4));
+  const size_t ioff = p.add((DJ_SPLIT + crowd.whole) * sizeof(uint4)), coff = p.add(nb * sizeof(uint32_t)),
+               soff = p.add((nb + 1) * sizeof(uint32_t)), scan_off = p.add(ej_scan_scratch_bytes(nb)),
+               poff = p.add(piece * sizeof(uint2)), goff = p.add(piece * sizeof(float4));
   EJ_TRY(ej_arena_reserve(h, p.bytes));
+  crowd.items = reinterpret_cast<uint4*>(ej_arena_at(h, ioff));
+  crowd.header = reinterpret_cast<uint32_t*>(h->d_words + DJ_CROWD_WORD);
   uint32_t* count = reinterpret_cast<uint32_t*>(ej_arena_at(h, coff));
   uint32_t* start = reinterpret_cast<uint32_t*>(ej_arena_at(h, soff));
   uint2* place = reinterpret_cast<uint2*>(ej_arena_at(h, poff));
   float4* grid = reinterpret_cast<float4*>(ej_arena_at(h, goff));
   using Row = typename RowOf<D>::type;
+  const unsigned cblocks = (unsigned)h->num_sms * 4;
   // the first piece's grid is the build phase; the probe (and any further pieces) the write phase
   ej_phase_begin(h);
+  const bool pieces = nR > DJ_RPIECE || nS > DJ_SPIECE;
   for (uint64_t r0 = 0; r0 < nR; r0 += DJ_RPIECE) {
     const uint32_t n = (uint32_t)std::min<uint64_t>(DJ_RPIECE, nR - r0);
     const uint32_t bits = dist_bits(n);
@@ -458,15 +731,31 @@ ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, ui
       for (int k = 1; k < EJ_PHASES; k++) ej_phase_mark(h, k);
     for (uint64_t s0 = 0; s0 < nS; s0 += DJ_SPIECE) {
       const uint32_t ns = (uint32_t)std::min<uint64_t>(DJ_SPIECE, nS - s0);
+      if (pieces) EJ_CUDA(h, cudaMemsetAsync(crowd.header, 0, 2 * sizeof(unsigned long long), h->stream));
       const unsigned sblocks =
           (unsigned)std::min<uint64_t>(((uint64_t)ns + DJ_THREADS - 1) / DJ_THREADS, (uint64_t)h->num_sms * 8);
       if (count_only)
         dist_probe_kernel<D, true><<<sblocks, DJ_THREADS, 0, h->stream>>>(R + r0, S + s0, ns, start, grid, bits, rad,
-                                                                          nullptr, 0, h->d_words);
+                                                                          crowd, nullptr, 0, h->d_words);
       else
-        dist_probe_kernel<D, false><<<sblocks, DJ_THREADS, 0, h->stream>>>(R + r0, S + s0, ns, start, grid, bits, rad,
-                                                                           static_cast<Row*>(outv), cap, h->d_words);
+        dist_probe_kernel<D, false><<<sblocks, DJ_THREADS, 0, h->stream>>>(
+            R + r0, S + s0, ns, start, grid, bits, rad, crowd, static_cast<Row*>(outv), cap, h->d_words);
       EJ_TRY(ej_check_launch(h, "dist_probe_kernel"));
+      const auto rest = [=]() -> ej_status {
+        if (count_only)
+          dist_crowd_kernel<D, true><<<cblocks, DJ_THREADS, 0, h->stream>>>(R + r0, S + s0, grid, crowd, rad, nullptr,
+                                                                            0, h->d_words);
+        else
+          dist_crowd_kernel<D, false><<<cblocks, DJ_THREADS, 0, h->stream>>>(
+              R + r0, S + s0, grid, crowd, rad, static_cast<Row*>(outv), cap, h->d_words);
+        return ej_check_launch(h, "dist_crowd_kernel");
+      };
+      // one piece: the caller launches it if its read-back finds items (a launch that
+      // finds none costs 5 us, of a call of 110); phase timing wants it in place
+      if (pieces || h->timing)
+        EJ_TRY(rest());
+      else
+        *crowded = rest;
     }
   }
   ej_phase_mark(h, EJ_PHASES);
@@ -483,10 +772,15 @@ ej_status dist_entry(ej_handle* h, uint32_t dims, const void* R, uint64_t nR, co
     return ej_fail(h, EJ_ERR_INVALID, "out is NULL with capacity %llu", (unsigned long long)cap);
   if (((uintptr_t)R | (uintptr_t)S | (uintptr_t)out) % 8)
     return ej_fail(h, EJ_ERR_INVALID, "point and row arrays must be 8-byte aligned");
-  EJ_TRY(dims == 2 ? dist_run<2>(h, R, nR, S, nS, radius, out, cap, count_only)
-                   : dist_run<3>(h, R, nR, S, nS, radius, out, cap, count_only));
+  std::function<ej_status()> crowded;
+  EJ_TRY(dims == 2 ? dist_run<2>(h, R, nR, S, nS, radius, out, cap, count_only, &crowded)
+                   : dist_run<3>(h, R, nR, S, nS, radius, out, cap, count_only, &crowded));
   uint64_t count = 0;
   EJ_TRY(ej_finish(h, &count));
+  if (crowded && h->h_words[DJ_CROWD_WORD] != 0) {
+    EJ_TRY(crowded());
+    EJ_TRY(ej_finish(h, &count));
+  }
   *out_count = count;
   return count_only ? EJ_OK : ej_capacity_result(h, count, cap);
 }
