@@ -71,6 +71,7 @@ constexpr int DJ_BUF = 192;  // candidate pairs a warp collects (tested past 128
 // of scratch for the grid, 0.25 GB for crowded buckets; larger relations go in pieces
 constexpr uint64_t DJ_RPIECE = 1ull << 26;
 constexpr uint64_t DJ_SPIECE = 1ull << 26;
+constexpr uint64_t DJ_LEAST_PIECE = 1ull << 16;  // R pieces get no smaller when memory is short
 constexpr uint64_t DJ_FEW_RPIECE = 1ull << 31;  // without a grid
 
 template <int D>
@@ -694,18 +695,28 @@ ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, ui
   const DistRadius rad = dist_radius(radius);
   if (nR == 0 || nS == 0 || !(rad.r2 > 0.0)) return EJ_OK;
   if (nS <= dist_few_most<D>()) return dist_few<D>(h, R, nR, S, (uint32_t)nS, rad, outv, cap, count_only);
-  const uint64_t piece = std::min(nR, DJ_RPIECE);
-  const uint64_t nb = 1ull << dist_bits(piece);
   // crowded buckets: few S points take all of the list's parts
   DistCrowd crowd;
   const uint64_t probes = std::min(nS, DJ_SPIECE);
   crowd.whole = (uint32_t)std::max(DJ_WHOLE, (probes + 31) / 32 * 8);
   crowd.parts = (uint32_t)std::max<uint64_t>(16, DJ_SPLIT / (probes << D));
-  ej_plan_bytes p;
-  const size_t ioff = p.add((DJ_SPLIT + crowd.whole) * sizeof(uint4)), coff = p.add(nb * sizeof(uint32_t)),
-               soff = p.add((nb + 1) * sizeof(uint32_t)), scan_off = p.add(ej_scan_scratch_bytes(nb)),
-               poff = p.add(piece * sizeof(uint2)), goff = p.add(piece * sizeof(float4));
-  EJ_TRY(ej_arena_reserve(h, p.bytes));
+  // R in pieces, smaller ones when memory is short
+  uint64_t piece = std::min(nR, DJ_RPIECE);
+  size_t ioff, coff, soff, scan_off, poff, goff;
+  for (;; piece = (piece + 3) / 4) {
+    const uint64_t nb = 1ull << dist_bits(piece);
+    ej_plan_bytes p;
+    ioff = p.add((DJ_SPLIT + crowd.whole) * sizeof(uint4));
+    coff = p.add(nb * sizeof(uint32_t));
+    soff = p.add((nb + 1) * sizeof(uint32_t));
+    scan_off = p.add(ej_scan_scratch_bytes(nb));
+    poff = p.add(piece * sizeof(uint2));
+    goff = p.add(piece * sizeof(float4));
+    const ej_status st = ej_arena_reserve(h, p.bytes);
+    if (st == EJ_OK) break;
+    if (st != EJ_ERR_NOMEM || piece <= DJ_LEAST_PIECE) return st;
+  }
+  h->last_error.clear();
   crowd.items = reinterpret_cast<uint4*>(ej_arena_at(h, ioff));
   crowd.header = reinterpret_cast<uint32_t*>(h->d_words + DJ_CROWD_WORD);
   uint32_t* count = reinterpret_cast<uint32_t*>(ej_arena_at(h, coff));
@@ -716,9 +727,9 @@ ej_status dist_run(ej_handle* h, const void* Rv, uint64_t nR, const void* Sv, ui
   const unsigned cblocks = (unsigned)h->num_sms * 4;
   // the first piece's grid is the build phase; the probe (and any further pieces) the write phase
   ej_phase_begin(h);
-  const bool pieces = nR > DJ_RPIECE || nS > DJ_SPIECE;
-  for (uint64_t r0 = 0; r0 < nR; r0 += DJ_RPIECE) {
-    const uint32_t n = (uint32_t)std::min<uint64_t>(DJ_RPIECE, nR - r0);
+  const bool pieces = nR > piece || nS > DJ_SPIECE;
+  for (uint64_t r0 = 0; r0 < nR; r0 += piece) {
+    const uint32_t n = (uint32_t)std::min<uint64_t>(piece, nR - r0);
     const uint32_t bits = dist_bits(n);
     const unsigned rblocks = (unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, (uint64_t)h->num_sms * 8);
     EJ_CUDA(h, cudaMemsetAsync(count, 0, sizeof(uint32_t) << bits, h->stream));

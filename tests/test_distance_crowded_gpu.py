@@ -10,6 +10,7 @@ import pytest
 import torch
 
 from eating_one_gb300 import native
+from eating_one_gb300.engine import Engine, JoinError
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -101,3 +102,25 @@ def test_crowd_on_either_side(engine, dims, radius, s):
     m, u = timed(few, many)
     assert n == m > 0
     assert t < 20 * u, (t, u)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+def test_memory_is_short(dims):
+    """R goes in smaller pieces when the scratch for all of it cannot be had (spread points and a
+    crowd), the call fails only when none can."""
+    rng = np.random.default_rng(7)
+    rv = np.concatenate([rng.random((300000, dims)) * 300.0, rng.random((2000, dims)) * 0.5])
+    sv = np.concatenate([rng.random((1000, dims)) * 300.0, rng.random((20, dims)) * 0.5])
+    lib = native.load()
+    with Engine(0) as e:
+        try:
+            lib.ej_inject_alloc_failures(2)
+            assert _check(e, dims, rv, sv, 1.0) > 20 * 2000
+            e.trim()
+            lib.ej_inject_alloc_failures(20)
+            with pytest.raises(JoinError) as x:
+                _check(e, dims, rv, sv, 1.0)
+            assert x.value.status == native.EJ_ERR_NOMEM
+        finally:
+            lib.ej_inject_alloc_failures(0)
+        _check(e, dims, rv, sv, 1.0)
