@@ -154,7 +154,8 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
     }
   }
   const BtTable table = {sm.rval, sm.rkey, sm.count, sm.start, sm.scan_tmp, lg};
-  bt_build<BN_THREADS>(table, reinterpret_cast<const int2*>(R + rbase), (uint32_t)min((uint64_t)r_block, nR - rbase));
+  const bool deep = bt_build<BN_THREADS>(table, reinterpret_cast<const int2*>(R + rbase),
+                                         (uint32_t)min((uint64_t)r_block, nR - rbase));
 
   BtBuffer found = {sm.st.buf[threadIdx.x >> 5], 0u};
   const BtOut rows = {out, cap, cursor, nullptr};
@@ -185,7 +186,8 @@ bnl_kernel(const ej_tuple* __restrict__ R, uint64_t nR, uint32_t r_block, uint32
       ok[j] = w0 + (uint32_t)j * 32u + lane < n;
       s[j] = ok[j] ? tile[j * 32 + lane] : make_int2(0, 0);
     }
-    local += bt_probe<COUNT_ONLY, false, false>(table, s, ok, 0u, nullptr, found, rows);
+    local += deep ? bt_probe<true, COUNT_ONLY, false, false>(table, s, ok, 0u, nullptr, found, rows)
+                  : bt_probe<false, COUNT_ONLY, false, false>(table, s, ok, 0u, nullptr, found, rows);
     __syncthreads();  // everyone is done with `buf` before it is refilled
   }
   if (!COUNT_ONLY && found.held) bt_flush<false>(table, found, nullptr, rows);
