@@ -603,7 +603,7 @@ uint32_t ej_table_bucket_bits(uint64_t nR, int delta) {
 constexpr uint64_t SLOT_QUARTER_ROWS = 1ull << 20;
 
 bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {
-  return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table != EJ_TABLE_FORMAT_DIRECTORY;
+  return nR <= EJ_SLOT_MAX_ROWS && k.build == EJ_BUILD_PLANNER && k.delta == 0 && k.table == EJ_TABLE_FORMAT_PLANNER;
 }
 
 uint64_t ej_slot_run_words(uint64_t nR) {

@@ -11,7 +11,7 @@
 
 // Hash tables of at most EJ_SLOT_MAX_ROWS rows are slot tables
 // (slot_table.cuh) unless the handle's options or tuning table choose a sort, a
-// load factor or a key directory.  At 2^25 rows and four probes a row the join
+// load factor or a table format.  At 2^25 rows and four probes a row the join
 // takes 2.71 ms against the sorted tables' 3.48 (unique keys), 3.74 / 4.04 (three
 // rows a key) and 5.07 / 5.02 (eight).  At 2^26 rows unique keys would still gain,
 // but four rows a key, counted and then written, took 7.46 ms against 7.37.

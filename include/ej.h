@@ -125,8 +125,7 @@ typedef enum ej_option {
                                       in place); -1 (default) lets the planner choose */
   EJ_OPT_BUCKET_BITS_DELTA = 1,    /* hash-table buckets = 2^(ceil(log2|R|) - 2 + delta),
                                       delta in -3..3 (a hash table given one is hash-sorted);
-                                      when neither this option nor the tuning table sets it: 0
-                                      for single tables, 1 for the tables of a batch */
+                                      0 leaves it to the tuning table, and then to the planner */
   EJ_OPT_WAIT_LIMIT_NS = 2,        /* bound of every device-side wait of this handle's kernels
                                       (look-back scans, the nested loop's copy waits), in ns,
                                       0..10^10; -1 restores the default of 10^9 (1 s).  A wait
@@ -139,14 +138,15 @@ typedef enum ej_option {
                                       same relations; 0: the count keeps nothing (and writes no
                                       run descriptors) */
   EJ_OPT_BUILD = 4,                /* radix passes of a hash table's build: EJ_BUILD_* (0: planner) */
-  EJ_OPT_TABLE = 5,                /* how probes find a hash table's runs: EJ_TABLE_FORMAT_* (0: planner) */
+  EJ_OPT_TABLE = 5,                /* how probes find a hash table's runs: EJ_TABLE_FORMAT_* (0: planner;
+                                      a hash table given a format is hash-sorted) */
   EJ_OPT_PROBE_WARPS = 6           /* block shape of the probe kernels: 4 or 8 warps of 32
                                       threads per block (0: planner, 8) */
 } ej_option;
 
 /* Values of EJ_OPT_BUILD and ej_tune_entry.build.  The planner gives hash tables
  * of at most 2^25 rows no sort (open addressing, one slot per key) unless
- * a load factor or a key directory is chosen for them, and then takes MSD from
+ * a load factor or a table format is chosen for them, and then takes MSD from
  * 2^20 rows on, else LSD; larger ones MSD; sorted indexes sort by LSD
  * passes (their key is the value, whose top bits need not spread, so MSD does
  * not apply to them; EJ_BUILD_ONESWEEP applies to both kinds). */
@@ -164,7 +164,7 @@ enum {
  * planner gives those of at least 2^22 rows a key directory when their runs
  * average two rows or more (or they are probed by 16 rows per table row or
  * more), the others bucket bounds; tables of at most 2^25 rows are not sorted
- * (see above) unless EJ_OPT_BUILD or a load factor asks for it. */
+ * (see above) unless EJ_OPT_BUILD, EJ_OPT_TABLE or a load factor asks for it. */
 enum {
   EJ_TABLE_FORMAT_PLANNER = 0,
   EJ_TABLE_FORMAT_BUCKETS = 1,  /* bucket bounds: one 8-byte load, then a scan of the bucket */
