@@ -15,8 +15,8 @@
 //               of the others (each warp finds its runs, reserves its rows
 //               with one atomic add on its join's count and writes them, as
 //               the one-pass probe of single joins does).
-// Joins of more than 2^26 R rows, past a slot's 27-bit run starts, run as single
-// joins after the batch's launches, on the same stream.
+// Joins of more than 2^22 R rows (EJ_BATCH_MAX_ROWS) run as single joins after the
+// batch's launches, on the same stream.
 // Every join's rows are the rows it gives alone; their order within the join
 // is not specified (warps reserve their ranges in the order they arrive).
 #include <string.h>
@@ -32,7 +32,15 @@ namespace {
 
 constexpr int BX_ITEMS = 4;                              // R rows per thread and tile (the insert: one, 4 blocks a tile)
 constexpr uint32_t BX_RTILE = 256 * BX_ITEMS;            // R rows per build tile
-constexpr uint64_t BX_MAX_R = 1ull << 26;                // larger joins run as single joins
+// Larger joins run as single joins: their tables are claimed by bucket groups in
+// shared memory and S is partitioned, where the batch claims slots and probes all
+// over memory.  Four joins in a batch, |S| = 4 |R|, unique keys and two rows a key,
+// in ms, as here, all in the batch's tables, and by radix passes as before these:
+// 2^23 rows 3.14, 3.32, 4.00 and 3.36, 6.26, 4.42; 2^24 5.80, 7.90, 10.3 and 6.28, 14.0,
+// 10.8; one of 2^25.5 2.05, 3.50, 3.93 and 2.81, 6.65, 3.89.  From 2^21 rows on it
+// is a matter of the keys: four of 2^22 1.70 as single joins, 1.43 in the batch (radix 1.82), with two
+// rows a key 1.79 and 2.70 (2.00); the served requests' keys are unique.
+constexpr uint64_t BX_MAX_R = EJ_BATCH_MAX_ROWS;
 
 // {runs' cursor of the join's table, ...}: cleared with the slots
 struct BatchTableHeader {

@@ -163,6 +163,9 @@ void ej_phase_mark(ej_handle* h, int k);
     if (s_ != EJ_OK) return s_;      \
   } while (0)
 
+// joins of a batch with more R rows run as single joins (batch.cu)
+constexpr uint64_t EJ_BATCH_MAX_ROWS = 1ull << 22;
+
 static inline uint32_t ej_ceil_log2(uint64_t x) {
   uint32_t b = 0;
   while ((uint64_t(1) << b) < x) b++;

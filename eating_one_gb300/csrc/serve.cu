@@ -70,7 +70,7 @@ struct Lane {
 
 // device scratch a request adds to a batch (see batch.cu / hash_join.cu layouts)
 uint64_t footprint(const ej_join_desc& j, int mode) {
-  const uint64_t per_r = mode == EJ_SERVE_BATCHED && j.nR <= (1ull << 26) ? 34 : 50;
+  const uint64_t per_r = mode == EJ_SERVE_BATCHED && j.nR <= EJ_BATCH_MAX_ROWS ? 34 : 50;
   return per_r * j.nR + 9 * j.nS + (1u << 20);
 }
 
