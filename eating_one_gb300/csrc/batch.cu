@@ -278,7 +278,8 @@ static ej_status batch_run(ej_handle* h, const ej_join_desc* jd, uint32_t n, uns
       if (nS) small_tasks.push_back({i, BX_SMALL_TASK});
       continue;
     }
-    b.view.npairs = (uint32_t)nR + 1u;  // at most half full
+    // at most half full; a bucket-bits delta above a batch's default, 1, makes it emptier
+    b.view.npairs = ((uint32_t)nR << std::max(0, ej_tuned_bucket_delta(h, nR, 1) - 1)) + 1u;
     b.view.run_words = (uint32_t)ej_slot_run_words(nR);
     pairs += b.view.npairs;
     run_words += (ej_slot_run_bytes(nR) / sizeof(int32_t) + 3) & ~uint64_t(3);

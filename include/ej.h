@@ -125,7 +125,9 @@ typedef enum ej_option {
                                       in place); -1 (default) lets the planner choose */
   EJ_OPT_BUCKET_BITS_DELTA = 1,    /* hash-table buckets = 2^(ceil(log2|R|) - 2 + delta),
                                       delta in -3..3 (a hash table given one is hash-sorted);
-                                      0 leaves it to the tuning table, and then to the planner */
+                                      0 leaves it to the tuning table, and then to the planner.
+                                      The tables of a batch, open addressing at half load, take
+                                      2 as a quarter and 3 as an eighth */
   EJ_OPT_WAIT_LIMIT_NS = 2,        /* bound of every device-side wait of this handle's kernels
                                       (look-back scans, the nested loop's copy waits), in ns,
                                       0..10^10; -1 restores the default of 10^9 (1 s).  A wait

@@ -37,3 +37,21 @@ def test_bucket_bounds(n, as_option):
             for algo in ("hash", "hash_index"):
                 assert np.array_equal(O.canon(e.join(algo, Rd, Sd).cpu().numpy()), want), algo
     assert launches[1] != launches[0]
+
+
+@pytest.mark.parametrize("delta", [-3, 1, 2, 3])
+def test_load_factor_of_a_batch(delta):
+    """A bucket-bits delta of 2 or 3 makes a batch's tables emptier: more scratch, the same rows."""
+    rng = np.random.default_rng(delta + 9)
+    host = [(_rel(rng.integers(0, n, n)), _rel(rng.integers(-9, n, 20011), 1 << 23)) for n in (2049, 60000, 300000)]
+    pairs = [(torch.from_numpy(R).cuda(), torch.from_numpy(S).cuda()) for R, S in host]
+    want = [O.canon(O.hash_join(R, S)) for R, S in host]
+    outs = [torch.empty((len(w), 4), dtype=torch.int32, device="cuda") for w in want]
+    scratch = []
+    for d in (0, delta):
+        with Engine(0, tuned=False) as e:
+            e.set_option("bucket_bits_delta", d)
+            for g, w in zip(e.batch_hash_join(pairs, outs), want):
+                assert np.array_equal(O.canon(g.cpu().numpy()), w)
+            scratch.append(e.scratch_bytes())
+    assert (scratch[1] > scratch[0]) == (delta > 1)
