@@ -195,7 +195,7 @@ ej_status ej_scan_u64_u64(ej_handle* h, const unsigned long long* in, uint64_t n
 // the signed val (EJ_DIGIT_VALUE, for sorting).
 enum { EJ_DIGIT_HASH = 0, EJ_DIGIT_VALUE = 1 };
 constexpr uint32_t EJ_RX_TILE = 4096;  // rows per radix tile
-// A tile of a segmented pass (batched joins): rows [start, start + n) of one
+// A tile of a segmented pass (msd.cu): rows [start, start + n) of one
 // segment (n <= EJ_RX_TILE); the histogram cell of digit d is cell0 + d * stride,
 // with cells laid out segment by segment (cell0 = segment base + tile index
 // in the segment, stride = tiles of the segment), so one scan over all cells
@@ -203,7 +203,6 @@ constexpr uint32_t EJ_RX_TILE = 4096;  // rows per radix tile
 struct ej_rx_tile {
   unsigned long long start;
   uint32_t n, cell0, stride, pad;
-  const ej_tuple* src;  // the tile's first input row (ej_partition_pass_src; other passes: input + start)
 };
 
 struct ej_radix_plan {
@@ -225,10 +224,6 @@ ej_status ej_partition_pass(ej_handle* h, const ej_radix_plan& rp, const ej_tupl
                             uint32_t shift, uint32_t bits, int digit_kind = EJ_DIGIT_HASH);
 ej_status ej_radix_pass_soa(ej_handle* h, const ej_radix_plan& rp, const ej_tuple* in, int32_t* out_keys,
                             int32_t* out_vals, uint32_t shift, uint32_t bits, int digit_kind);
-// the unordered pass by hash digits over tiles whose descriptors carry their
-// source rows (src), which may lie in separate arrays
-ej_status ej_partition_pass_src(ej_handle* h, const ej_radix_plan& rp, ej_tuple* out, uint32_t shift,
-                                uint32_t bits);
 
 // ---- probe targets (hash_join.cu) -----------------------------------------
 // R is stored as two arrays, rkey[] and rval[], in one order:
@@ -247,7 +242,7 @@ struct ej_table_view {
   int kind = EJ_TABLE_HASH;
   const int32_t* rkey = nullptr;     // [nR + pad] row ids in table order
   const int32_t* rval = nullptr;     // [nR + pad] join keys in table order
-  const uint2* bucket = nullptr;     // [2^hb] (hash, batched tables): row bounds of each bucket
+  const uint2* bucket = nullptr;     // [2^hb] (sorted tables without a directory): row bounds of each bucket
   const uint2* dir = nullptr;        // (hash, single tables) key directory {hash, run start [, length]}
   const uint32_t* dir_bits = nullptr;  // device word: the directory has 2^bits home slots
   uint32_t dir_packed = 0;             // entries {hash, start << 5 | run length} (tables under 2^27 rows)
@@ -257,7 +252,6 @@ struct ej_table_view {
   const void* vbuckets = nullptr;    // (sorted) device EjValueBuckets {vmin, vmax, vshift} of `bucket`
   uint64_t nR = 0;
   uint32_t hb = 1;
-  uint32_t voff = 0;  // rval - voff is 16-byte aligned (tables of a batch share one array)
   // known on the host to have runs of about one row (an index whose build
   // chose bucket bounds for its short runs): probes load run keys in 8-byte chunks
   uint32_t short_runs = 0;

@@ -92,7 +92,6 @@ __global__ void __launch_bounds__(256) msd_tiles_kernel(const MsdSegments* __res
   if (i >= max_tiles) return;
   const uint32_t used = tb[256];
   ej_rx_tile t;
-  t.src = nullptr;
   t.pad = 0;
   if (i < used) {
     uint32_t lo = 0, hi = 256;  // the segment d with tb[d] <= i < tb[d + 1]

@@ -190,14 +190,7 @@ __device__ __forceinline__ void ej_find_runs_bucket(const ej_table_view& t, cons
       s1[j] = bb.y;
     }
   }
-  // vector loads address the aligned base rval - voff; positions are shifted
-  // by voff while scanning and shifted back when recorded
-  const int4* rv4 = reinterpret_cast<const int4*>(t.rval - t.voff);
-#pragma unroll
-  for (int j = 0; j < N; j++) {
-    s0[j] += t.voff;
-    s1[j] += t.voff;
-  }
+  const int4* rv4 = reinterpret_cast<const int4*>(t.rval);
   int4 qa[N], qb[N];
 #pragma unroll
   for (int j = 0; j < N; j++) {
@@ -234,7 +227,7 @@ __device__ __forceinline__ void ej_find_runs_bucket(const ej_table_view& t, cons
       else if (!c[j] && to >= 8u) lower |= 1u << j;
     }
   }
-  const int32_t* rv = t.rval - t.voff;
+  const int32_t* rv = t.rval;
   // 4 more values per round (one 16-byte load per probe and round): hash
   // tables until the run or the bucket ends (a long run there is a key with
   // many rows in a small table); sorted tables, whose value buckets can be
@@ -296,8 +289,6 @@ __device__ __forceinline__ void ej_find_runs_bucket(const ej_table_view& t, cons
     for (int j = 0; j < N; j++)
       if (found & (1u << j)) c[j] = sl[j] - lo[j];
   }
-#pragma unroll
-  for (int j = 0; j < N; j++) lo[j] -= t.voff;
 }
 
 // The key directory's slots of N probe hashes (dir.cuh): every probe loads

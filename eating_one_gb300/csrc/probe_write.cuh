@@ -92,14 +92,14 @@ __device__ __forceinline__ unsigned long long ej_group_rows(uint32_t c, uint32_t
   return __shfl_sync(EJ_FULL_MASK, incl, 31);
 }
 
-// keys of the first PW_PREFETCH rows of every run (rkey - voff is 16-byte
+// keys of the first PW_PREFETCH rows of every run (rkey is 16-byte
 // aligned and the column is padded, so every load stays inside it), in one
 // of two schemes fixed at compile time (the L1 data path pays for the bytes
 // it delivers; both schemes in one kernel cost more than either saves):
 //   EJ_KEYS_WINDOW  the aligned 8-key window holding the first four keys, one
 //                   or two 16-byte loads (single tables: C3's runs of four);
 //   EJ_KEYS_CHUNKS  the aligned 8-byte chunks holding them, one to three
-//                   loads (batched tables, whose runs are mostly of one or
+//                   loads (indexes whose build found runs of mostly one or
 //                   two rows).
 enum { EJ_KEYS_WINDOW = 0, EJ_KEYS_CHUNKS = 1 };
 // INL (inline tables): rows found in slots (INLINE_RUN) have their key in key[].
@@ -109,8 +109,8 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
                                                   const int32_t (&key)[PR_ITEMS] = {}) {
   static_assert(PW_PREFETCH == 4, "the window holds 4 keys past any offset");
   constexpr bool chunks = KEYS == EJ_KEYS_CHUNKS;
-  const int4* rk4 = reinterpret_cast<const int4*>(t.rkey - t.voff);
-  const int2* rk2 = reinterpret_cast<const int2*>(t.rkey - t.voff);
+  const int4* rk4 = reinterpret_cast<const int4*>(t.rkey);
+  const int2* rk2 = reinterpret_cast<const int2*>(t.rkey);
   int4 qa[PR_ITEMS], qb[PR_ITEMS];
   uint32_t o[PR_ITEMS];
 #pragma unroll
@@ -118,7 +118,7 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
     qa[j] = qb[j] = make_int4(EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY);
     o[j] = 0;
     if (w.lo[j] < (INL ? INLINE_RUN : NULL_RUN) && w.cnt[j]) {
-      const uint32_t p = w.lo[j] + t.voff;
+      const uint32_t p = w.lo[j];
       if (chunks) {  // keys p .. p + min(cnt, 4) - 1 from the 8-byte chunks holding them
         const uint32_t last = (p + min(w.cnt[j], (uint32_t)PW_PREFETCH) - 1u) / 2u;
         o[j] = p & 1u;
