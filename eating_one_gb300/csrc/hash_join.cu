@@ -8,7 +8,7 @@
 // compares per block, and the write pass repeats all of them.
 //
 // Here:
-//   build  Hash tables of up to 2^25 rows by open addressing, one slot per
+//   build  Hash tables of up to 7 2^23 rows by open addressing, one slot per
 //          key (slot_table.cuh; above 2^21 rows by bucket groups, msd.cu; hash
 //          and outer joins of up to 16384 build rows run whole in shared
 //          memory instead, small_join.cu).  Larger ones, and those for which
@@ -597,9 +597,13 @@ uint32_t ej_table_bucket_bits(uint64_t nR, int delta) {
 
 
 // Slot tables up to this many rows are at most a quarter full, larger ones half.
-// 2^20 rows, one join of 2^22 probes: a quarter 151 us, half 171 (the inserts walk
-// longer); but two 2^20-row dimension tables probed by 2^26 facts 1.60 ms at a
-// quarter, 1.35 at half (32 MB less in L2), so probe-heavy callers take half.
+// A quarter against half, |S| from half to 16 |R|: below 2^20 rows faster for any keys
+// (unique 0.74 to 0.85, two and four rows a key 0.95 to 1.02; one join of 2^20 rows
+// and 2^22 probes 120 us, 147); above it unique keys still gain (2^20.25 0.83, 2^21
+// 0.87) but four rows a key lose (1.02 to 1.05, 2^20.5 1.04 to 1.10, 2^21 1.07), whose
+// emptier array spreads their gathers.  Two 2^20-row dimension tables probed by
+// 2^26 facts 1.60 ms at a quarter, 1.35 at half (32 MB less in L2), so probe-heavy
+// callers take half.
 constexpr uint64_t SLOT_QUARTER_ROWS = 1ull << 20;
 
 bool ej_table_is_slots(uint64_t nR, const ej_table_knobs& k) {

@@ -11,11 +11,13 @@
 
 // Hash tables of at most EJ_SLOT_MAX_ROWS rows are slot tables
 // (slot_table.cuh) unless the handle's options or tuning table choose a sort, a
-// load factor or a table format.  At 2^25 rows and four probes a row the join
-// takes 2.71 ms against the sorted tables' 3.48 (unique keys), 3.74 / 4.04 (three
-// rows a key) and 5.07 / 5.02 (eight).  At 2^26 rows unique keys would still gain,
-// but four rows a key, counted and then written, took 7.46 ms against 7.37.
-constexpr uint64_t EJ_SLOT_MAX_ROWS = 1ull << 25;
+// load factor or a table format.  The line: at 2^25 to 2^25.75 rows slot tables are
+// the faster ones for one to eight rows a key, half to four probes a row, uniform
+// and Zipf-skewed S, counted first or not (0.63 to 0.98 of the sorted tables' time;
+// 2^25.75 rows, four probes a row, 4.34 against 5.60 ms for unique keys, 5.91 / 6.05
+// for four rows a key).  At 2^26 unique keys still gain (5.21 / 6.77), but four rows a
+// key, probed by a skewed S, counted and then written, take 7.36 ms against 7.24.
+constexpr uint64_t EJ_SLOT_MAX_ROWS = 7ull << 23;
 // Up to EJ_SLOT_DIRECT_ROWS the slots are claimed through L2, above it group by
 // group in shared memory after two radix passes (msd.cu).  Claims through L2 are
 // quick for unique keys (3 M rows: the join with 12 M probes 275 us against 322

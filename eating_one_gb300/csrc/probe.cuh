@@ -2,7 +2,7 @@
 //
 // A table stores R as rkey[]/rval[] in one order (ej_table_view).  In both
 // kinds the matches of a value v form one contiguous run [lo, lo + c):
-//   EJ_TABLE_HASH    rows sorted by hash32(val) (tables of more than 2^25 rows,
+//   EJ_TABLE_HASH    rows sorted by hash32(val) (tables of more than 7 2^23 rows,
 //                    and those for which a sort, a load factor or a directory
 //                    was chosen; the others are slot tables, slot_table.cuh).
 //                    Tables of 2^22 rows or more whose runs average two rows

@@ -147,7 +147,7 @@ typedef enum ej_option {
 } ej_option;
 
 /* Values of EJ_OPT_BUILD and ej_tune_entry.build.  The planner gives hash tables
- * of at most 2^25 rows no sort (open addressing, one slot per key) unless
+ * of at most 7 * 2^23 rows no sort (open addressing, one slot per key) unless
  * a load factor or a table format is chosen for them, and then takes MSD from
  * 2^20 rows on, else LSD; larger ones MSD; sorted indexes sort by LSD
  * passes (their key is the value, whose top bits need not spread, so MSD does
@@ -165,7 +165,7 @@ enum {
 /* Values of EJ_OPT_TABLE and ej_tune_entry.table, for hash-sorted tables.  The
  * planner gives those of at least 2^22 rows a key directory when their runs
  * average two rows or more (or they are probed by 16 rows per table row or
- * more), the others bucket bounds; tables of at most 2^25 rows are not sorted
+ * more), the others bucket bounds; tables of at most 7 * 2^23 rows are not sorted
  * (see above) unless EJ_OPT_BUILD, EJ_OPT_TABLE or a load factor asks for it. */
 enum {
   EJ_TABLE_FORMAT_PLANNER = 0,

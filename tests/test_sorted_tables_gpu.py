@@ -1,4 +1,4 @@
-"""Hash-sorted tables below the sizes at which the planner takes them (2^25 rows), so
+"""Hash-sorted tables below the sizes at which the planner takes them (7 * 2^23 rows), so
 that the sort, the key directory and the bucket bounds are tested where they can go
 wrong: bucket groups too large for shared memory, long runs, the directory's choice
 by the length of the runs, probes that take its general path."""
