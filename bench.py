@@ -492,7 +492,7 @@ def config_lines(eng, peaks: dict, steps: int, distance: bool) -> list[dict]:
     ms = timed(lambda: eng.join("bnl", R, S, out=out), max(3, steps // 4))
     pairs = R.shape[0] * S.shape[0]
     lines.append({"config": "C2 BNLJ R=2^16 x S=2^20, keys uniform in [0, 2^16)", "ms": round(ms, 4), "rows": n,
-                  "pair_compares_per_s": pairs / (ms / 1000),
+                  "input_pairs_per_s": pairs / (ms / 1000),  # |R| |S| over the time; few are compared
                   "roofline": hbm(8 * (R.shape[0] + S.shape[0]) + 16 * n, ms),
                   "reference_gpu_log": "2^20 x 2^16 in 1.483 s (nestLoopJoin, sm_35)"})
     del out
@@ -549,7 +549,8 @@ def config_lines(eng, peaks: dict, steps: int, distance: bool) -> list[dict]:
         O.distance_join(dims, Rp, s_sample, 1.0, threads=threads)
         cpu_s = time.perf_counter() - t0
         lines.append({"config": "%dD distance join R=2^19 x S=2^19 points, radius 1, 10%% copies" % dims,
-                      "ms": round(ms, 4), "rows": n, "pairs_per_s": pairs / (ms / 1000),
+                      "ms": round(ms, 4), "rows": n,
+                      "input_pairs_per_s": pairs / (ms / 1000),  # |R| |S| over the time; few are compared
                       "roofline": hbm((8 + 8 * dims) * (len(Rp) + len(Sp)) + out.nbytes, ms),
                       "cpu_baseline": {"pairs_per_s": len(Rp) * len(s_sample) / cpu_s, "cores": threads,
                                        "kind": "port", "sample": "R=2^19 x the first 1024 S points"},

@@ -223,8 +223,8 @@ __device__ __forceinline__ void batch_small_join(const BatchJoin& j, int4* smem,
 
 // The probe of a batch as one launch over a task list, one task per block,
 // handed out in list order by the block scheduler: a whole small join (table
-// built and probed in shared memory) or one 1024-probe tile of a larger join
-// (table from the segmented passes).  The small joins come first, so that no
+// built and probed in shared memory) or BX_TASK_TILES 1024-probe tiles of a join
+// with a slot table.  The small joins come first, so that no
 // large task waits behind them at the end.  (A resident grid pulling tasks
 // from an atomic counter measured slower.)  32 served requests of 13.3 M
 // R rows in all: four segmented radix passes, bucket bounds and this kernel over

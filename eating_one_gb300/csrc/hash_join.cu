@@ -873,9 +873,9 @@ uint32_t ej_probe_partition_bits(const ej_handle* h, uint64_t nR, uint64_t nS) {
   const double table = slots ? 16.0 * (double)nR : (double)ej_table_bytes(nR, k.delta);
   const double l2 = (double)(h->l2_bytes ? h->l2_bytes : (size_t)126 << 20);
   // what the probes touch stays in L2: a sorted table of a quarter of it; half
-  // full slots, one 16-byte pair a probe, up to 0.6 (4.5 M unique keys and 18 M
-  // probes 435 us against 504 partitioned, 6 M 562 / 618, but 6 M rows of four a
-  // key 828 / 759)
+  // full slots, one 16-byte pair a probe, of half of it (at 0.6 unique keys would
+  // still gain, 4.5 M and 18 M probes 435 us against 504 partitioned, 6 M 562 / 618,
+  // but 6 M rows of four a key lose, 828 / 759)
   if (table <= l2 * (slots ? 0.5 : 0.25)) return 0;
   // one partition's table region should be several MB so that the partitions
   // in flight share L2 with the streaming probe and output traffic (C3's
@@ -1005,8 +1005,8 @@ ej_status ej_hash_join_run(ej_handle* h, const ej_tuple* R, uint64_t nR, const e
   ej_table_plan_t tp;
   ej_table_plan(p, tp, nR, /*own_storage=*/false, EJ_TABLE_HASH, ej_tuned_table_knobs(h, nR), nS);
   ej_probe_layout L;
-  // the build-side-only join keeps its rows in probe order (the batched joins
-  // give the same rows in the same order); the others take the one-pass probe
+  // the build-side-only join keeps its rows in probe order; the others take the
+  // one-pass probe
   ej_probe_layout_add(p, L, nS, pb, mode == 2, /*two_pass=*/mode == 1 || keep, ej_tuned_probe_warps(h, nR));
   EJ_TRY(ej_arena_reserve(h, p.bytes));
   ej_phase_begin(h);

@@ -322,10 +322,11 @@ typedef struct ej_join_desc {
 } ej_join_desc;
 
 /* Many hash joins as one pipeline: a fixed sequence of launches builds every
- * join's table (segmented radix passes) and probes every join (one work queue
- * of (join, tile) tasks), instead of one pipeline per join.  The reference runs
- * one join per process (joins/hashJoin_gpu/main_street/hj.cc:171-1269).  Each
- * join's rows are bitwise those of ej_single_hash_join on the same inputs.
+ * join's table (open addressing) and probes every join (one list of (join, tiles)
+ * tasks), instead of one pipeline per join; joins of more than 2^22 R rows follow
+ * as single joins.  The reference runs one join per process
+ * (joins/hashJoin_gpu/main_street/hj.cc:171-1269).  Each join's rows are bitwise
+ * those of ej_single_hash_join on the same inputs, in no particular order.
  * counts[i] (host) receives join i's total; EJ_ERR_CAPACITY when any join has
  * more results than its out_cap (its rows past out_cap are dropped). */
 ej_status ej_batch_hash_join(ej_handle* h, const ej_join_desc* joins, uint32_t njoins, uint64_t* counts);

@@ -47,6 +47,18 @@ def test_one_crowded_cell(engine, dims, n, s):
 
 
 @pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("radius", [1.0, 1e19, 1e200, 0.0])
+def test_few_points_with_odd_values(engine, dims, radius):
+    """Values that never match, or only at radii whose floats overflow, on both sides of few S points."""
+    rng = np.random.default_rng(8)
+    odd = np.array([1e300, -1e300, 1e18, 3.5e38, 1e19, np.inf, -np.inf, np.nan, 5e-324, -0.0, 0.0, 1e150])
+    rv, sv = rng.random((3000, dims)) * 2.0, rng.random((100, dims)) * 2.0
+    rv[::7] = rng.choice(odd, size=rv[::7].shape)
+    sv[::3] = rng.choice(odd, size=sv[::3].shape)
+    _check(engine, dims, rv, sv, radius)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
 def test_crowded_cells_of_many_points(engine, dims):
     """S points over several crowded cells, different ones in a warp."""
     rng = np.random.default_rng(dims)
