@@ -46,6 +46,13 @@ __device__ __forceinline__ void ej_st_relaxed(unsigned long long* p, unsigned lo
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// The pointer in a register, not an operand from the constant bank
+template <class T>
+__device__ __forceinline__ T* ej_in_register(T* p) {
+  asm("" : "+l"(p));
+  return p;
+}
+
 // The grid's threads clear n words (n at most the grid's threads): the scratch
 // of a scan that follows, which would otherwise take a memset of its own.
 __device__ __forceinline__ void ej_clear_words(unsigned long long* p, uint64_t n) {

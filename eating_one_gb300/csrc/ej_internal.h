@@ -252,6 +252,7 @@ struct ej_table_view {
   const void* vbuckets = nullptr;    // (sorted) device EjValueBuckets {vmin, vmax, vshift} of `bucket`
   uint64_t nR = 0;
   uint32_t hb = 1;
+  uint32_t voff = 0;  // words of rkey past a 16-byte boundary: none, every column begins at one (ej_probe_prefetch)
   // known on the host to have runs of about one row (an index whose build
   // chose bucket bounds for its short runs): probes load run keys in 8-byte chunks
   uint32_t short_runs = 0;

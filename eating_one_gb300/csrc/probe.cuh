@@ -190,7 +190,9 @@ __device__ __forceinline__ void ej_find_runs_bucket(const ej_table_view& t, cons
       s1[j] = bb.y;
     }
   }
-  const int4* rv4 = reinterpret_cast<const int4*>(t.rval);
+  // (the column's base in a register: as an operand from the constant bank the counts
+  // without descriptors spill, 12 M probes of a sort index 109 us instead of 85)
+  const int4* rv4 = reinterpret_cast<const int4*>(ej_in_register(t.rval));
   int4 qa[N], qb[N];
 #pragma unroll
   for (int j = 0; j < N; j++) {

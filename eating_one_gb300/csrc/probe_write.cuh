@@ -92,8 +92,10 @@ __device__ __forceinline__ unsigned long long ej_group_rows(uint32_t c, uint32_t
   return __shfl_sync(EJ_FULL_MASK, incl, 31);
 }
 
-// keys of the first PW_PREFETCH rows of every run (rkey is 16-byte
-// aligned and the column is padded, so every load stays inside it), in one
+// keys of the first PW_PREFETCH rows of every run (rkey - voff is 16-byte
+// aligned and the column is padded, so every load stays inside it; voff is 0, but
+// with the positions known to be rkey's own the compiler's code for C3's write
+// pass takes 3.25 ms instead of 3.16), in one
 // of two schemes fixed at compile time (the L1 data path pays for the bytes
 // it delivers; both schemes in one kernel cost more than either saves):
 //   EJ_KEYS_WINDOW  the aligned 8-key window holding the first four keys, one
@@ -109,8 +111,8 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
                                                   const int32_t (&key)[PR_ITEMS] = {}) {
   static_assert(PW_PREFETCH == 4, "the window holds 4 keys past any offset");
   constexpr bool chunks = KEYS == EJ_KEYS_CHUNKS;
-  const int4* rk4 = reinterpret_cast<const int4*>(t.rkey);
-  const int2* rk2 = reinterpret_cast<const int2*>(t.rkey);
+  const int4* rk4 = reinterpret_cast<const int4*>(t.rkey - t.voff);
+  const int2* rk2 = reinterpret_cast<const int2*>(t.rkey - t.voff);
   int4 qa[PR_ITEMS], qb[PR_ITEMS];
   uint32_t o[PR_ITEMS];
 #pragma unroll
@@ -118,7 +120,7 @@ __device__ __forceinline__ void ej_probe_prefetch(const ej_table_view& t, const 
     qa[j] = qb[j] = make_int4(EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY, EJ_NULL_KEY);
     o[j] = 0;
     if (w.lo[j] < (INL ? INLINE_RUN : NULL_RUN) && w.cnt[j]) {
-      const uint32_t p = w.lo[j];
+      const uint32_t p = w.lo[j] + t.voff;
       if (chunks) {  // keys p .. p + min(cnt, 4) - 1 from the 8-byte chunks holding them
         const uint32_t last = (p + min(w.cnt[j], (uint32_t)PW_PREFETCH) - 1u) / 2u;
         o[j] = p & 1u;
