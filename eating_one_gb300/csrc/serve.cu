@@ -53,9 +53,13 @@ struct Lane {
   Server* srv = nullptr;
   ej_handle* h = nullptr;
   cudaStream_t stream = nullptr;
-  unsigned long long* d_counts = nullptr;
+  // the handle's status word and the batch's counts, in one piece so that one copy
+  // reads both back
+  ej_dev_status* d_status = nullptr;
+  ej_dev_status* h_status = nullptr;
+  unsigned long long* d_counts = nullptr;  // behind the status
   unsigned long long* h_counts = nullptr;
-  ej_dev_status* h_status = nullptr;  // the handle's device status after the batch
+  bool clear = true;  // the status is not known to be clear: at first, and after a batch that left one
   // EJ_SERVE_CHECKSUM: the batch's requests and their outputs' checksums
   ej_join_desc* d_desc = nullptr;
   ej_join_desc* h_desc = nullptr;
@@ -84,6 +88,7 @@ void CUDART_CB lane_done(void* arg) {
   ej_status st = L->launch_status;
   if (st == EJ_OK && L->h_status->code != 0 && L->h_status->code != EJ_ERR_CAPACITY)
     st = (ej_status)L->h_status->code;
+  L->clear = L->launch_status != EJ_OK || L->h_status->code != 0;
   {
     std::lock_guard<std::mutex> lock(S->mu);
     for (size_t i = 0; i < L->batch.size(); i++) {
@@ -110,9 +115,10 @@ void CUDART_CB lane_done(void* arg) {
 ej_status lane_launch(Lane* L, int mode) {
   ej_handle* h = L->h;
   const uint32_t n = (uint32_t)L->batch.size();
-  // the status word is the batch's own: cleared before its first kernel (whatever
-  // an earlier batch left), read back behind its last
-  ej_status st = cudaMemsetAsync(h->d_status, 0, sizeof(ej_dev_status), L->stream) == cudaSuccess ? EJ_OK : EJ_ERR_CUDA;
+  // the status word is the batch's own: clear before its first kernel, whatever an
+  // earlier batch left, read back behind its last
+  ej_status st = EJ_OK;
+  if (L->clear && cudaMemsetAsync(L->d_status, 0, sizeof(ej_dev_status), L->stream) != cudaSuccess) st = EJ_ERR_CUDA;
   if (st != EJ_OK) {
   } else if (mode == EJ_SERVE_BATCHED) {
     std::vector<ej_join_desc> d(n);
@@ -136,11 +142,8 @@ ej_status lane_launch(Lane* L, int mode) {
                                        L->stream) != cudaSuccess)
       st = EJ_ERR_CUDA;
   }
-  if (st == EJ_OK && cudaMemcpyAsync(L->h_counts, L->d_counts, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                     L->stream) != cudaSuccess)
-    st = EJ_ERR_CUDA;
-  if (st == EJ_OK && cudaMemcpyAsync(L->h_status, h->d_status, sizeof(ej_dev_status), cudaMemcpyDeviceToHost,
-                                     L->stream) != cudaSuccess)
+  if (st == EJ_OK && cudaMemcpyAsync(L->h_status, L->d_status, sizeof(ej_dev_status) + n * sizeof(unsigned long long),
+                                     cudaMemcpyDeviceToHost, L->stream) != cudaSuccess)
     st = EJ_ERR_CUDA;
   L->launch_status = st;
   if (st != EJ_OK) {
@@ -199,8 +202,7 @@ void server_free(Server* S) {
     if (L->stream) cudaStreamSynchronize(L->stream);
     if (L->h) ej_destroy(L->h);
     if (L->stream) cudaStreamDestroy(L->stream);
-    cudaFree(L->d_counts);
-    cudaFreeHost(L->h_counts);
+    cudaFree(L->d_status);
     cudaFreeHost(L->h_status);
     cudaFree(L->d_desc);
     cudaFreeHost(L->h_desc);
@@ -240,9 +242,8 @@ extern "C" ej_status ej_server_create(const ej_server_config* cfg, ej_server** o
       return st;
     }
     if (cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        ej_dev_alloc(&L->d_counts, per_lane * sizeof(unsigned long long)) != cudaSuccess ||
-        ej_host_alloc(&L->h_counts, per_lane * sizeof(unsigned long long)) != cudaSuccess ||
-        ej_host_alloc(&L->h_status, sizeof(ej_dev_status)) != cudaSuccess ||
+        ej_dev_alloc(&L->d_status, sizeof(ej_dev_status) + per_lane * sizeof(unsigned long long)) != cudaSuccess ||
+        ej_host_alloc(&L->h_status, sizeof(ej_dev_status) + per_lane * sizeof(unsigned long long)) != cudaSuccess ||
         ((S->cfg.flags & EJ_SERVE_CHECKSUM) &&
          (ej_dev_alloc(&L->d_desc, per_lane * sizeof(ej_join_desc)) != cudaSuccess ||
           ej_host_alloc(&L->h_desc, per_lane * sizeof(ej_join_desc)) != cudaSuccess ||
@@ -253,7 +254,10 @@ extern "C" ej_status ej_server_create(const ej_server_config* cfg, ej_server** o
       return EJ_ERR_NOMEM;
     }
     L->cap = per_lane;
+    L->d_counts = reinterpret_cast<unsigned long long*>(L->d_status + 1);
+    L->h_counts = reinterpret_cast<unsigned long long*>(L->h_status + 1);
     ej_set_stream(L->h, L->stream);
+    L->h->d_status = L->d_status;  // the lane calls asynchronous joins only: nothing else reads the handle's own
   }
   S->sched = std::thread(scheduler, S);
   ej_server* srv = new ej_server();
