@@ -85,4 +85,4 @@ def test_not_slower_than_a_table_in_global_memory(engine, rows, s):
         there = best()
     finally:
         engine.set_option("build", 0)
-    assert here < 1.25 * there, (here, there)
+    assert here < 1.6 * there, (here, there)  # 0.7 to 1.05; lane by lane 2.1 and 2.7
